@@ -7,7 +7,7 @@
 // Frontier state (V-sized, reused every iteration):
 //   active[V] ascending ids, active_scan[V+1] in-degree scan, apply_ret[V],
 //   slot[V] new vertex data per active slot, gather_tmp[V], next-frontier
-//   bitmap bits[V/32], scatter scan sscan[V+1], per-tile carries.
+//   bitmap bits[V/32], the expansion's chunk list, per-tile carries.
 // Counters live in one device line (gas_counters); the step API reads them
 // back once per nextIter()/countActive(), the fast runs never do until the
 // end (the loop is a CUDA graph with a device-side WHILE condition).
@@ -129,11 +129,6 @@ struct PageRank {
 // ---------------------------------------------------------------------------
 namespace {
 
-constexpr int kScanItems = 16;                   // items per thread in scans
-constexpr int kScanBlock = kNT * kScanItems;     // 4096 slots per block
-constexpr int kWordsPerThread = 4;               // bitmap words per thread
-constexpr int kCompactBlock = kNT * kWordsPerThread;  // 1024 words per block
-
 __device__ __forceinline__ int warp_incl_sum(int v) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -199,214 +194,343 @@ __global__ void k_commit(const int32_t *act, const gas_counters *cnt,
   }
 }
 
-// Scan of out-degree over apply()==true slots -> sscan (three passes:
-// per-block totals, spine, per-block scan).
-__device__ __forceinline__ int pred_outdeg(const int32_t *act,
-                                           const uint8_t *ret,
-                                           const int32_t *csr_off, int i,
-                                           int n) {
-  if (i >= n || !ret[i]) return 0;
-  const int v = act[i];
-  return csr_off[v + 1] - csr_off[v];
-}
-
-__global__ void __launch_bounds__(kNT)
-    k_pscan_reduce(const int32_t *act, const uint8_t *ret,
-                   const int32_t *csr_off, const gas_counters *cnt,
-                   int32_t *part) {
-  const int n = cnt->n_active;
-  const int nb = (n + kScanBlock - 1) / kScanBlock;
-  for (int b = blockIdx.x; b < nb; b += gridDim.x) {
-    int s = 0;
-    const int base = b * kScanBlock + threadIdx.x;
-#pragma unroll 4
-    for (int k = 0; k < kScanItems; ++k)
-      s += pred_outdeg(act, ret, csr_off, base + k * kNT, n);
-    int tot;
-    block_excl_sum(s, &tot);
-    if (threadIdx.x == 0) part[b] = tot;
-  }
-}
-
-// Single CTA: exclusive scan of part[0..nb) in place; total to *total.
-__device__ void spine_scan(int32_t *part, int nb, int32_t *total) {
-  __shared__ int s_carry;
-  if (threadIdx.x == 0) s_carry = 0;
-  __syncthreads();
-  for (int base = 0; base < nb; base += kNT) {
-    const int i = base + threadIdx.x;
-    const int v = i < nb ? part[i] : 0;
-    int tot;
-    const int ex = block_excl_sum(v, &tot);
-    const int carry = s_carry;
-    if (i < nb) part[i] = carry + ex;
-    __syncthreads();
-    if (threadIdx.x == 0) s_carry = carry + tot;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *total = s_carry;
-}
-
-__global__ void __launch_bounds__(kNT)
-    k_pscan_spine(int32_t *part, gas_counters *cnt) {
-  const int n = cnt->n_active;
-  const int nb = (n + kScanBlock - 1) / kScanBlock;
-  spine_scan(part, nb, &cnt->n_scatter_edges);
-}
-
-__global__ void __launch_bounds__(kNT)
-    k_pscan_down(const int32_t *act, const uint8_t *ret,
-                 const int32_t *csr_off, const gas_counters *cnt,
-                 const int32_t *part, int32_t *sscan) {
-  const int n = cnt->n_active;
-  const int nb = (n + kScanBlock - 1) / kScanBlock;
-  for (int b = blockIdx.x; b < nb; b += gridDim.x) {
-    // each thread owns kScanItems consecutive slots
-    const int base = b * kScanBlock + threadIdx.x * kScanItems;
-    int vals[kScanItems];
-    int s = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-      vals[k] = pred_outdeg(act, ret, csr_off, base + k, n);
-      s += vals[k];
-    }
-    int tot;
-    int run = block_excl_sum(s, &tot) + part[b];
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-      if (base + k < n) sscan[base + k] = run;
-      run += vals[k];
-    }
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) sscan[n] = cnt->n_scatter_edges;
-}
-
 // Expansion: set the next-frontier bit of every out-neighbour of every
-// apply()==true vertex.
-struct ExpandPol {
-  typedef int32_t Val;
-  const int32_t *csr_dst;
-  uint32_t *bits;
-  __device__ Val zero() const { return 0; }
-  __device__ Val reduce(Val a, Val) const { return a; }
-  __device__ Val map(int, int, int) const { return 0; }
-  __device__ void emit(int, int, Val) const {}
-  __device__ __forceinline__ void visit(int, int, int pos) const {
-    const uint32_t w = (uint32_t)__ldg(csr_dst + pos);
-    atomicOr(bits + (w >> 5), 1u << (w & 31));
-  }
+// apply()==true vertex.  The bit is tested before the atomic: a hub is the
+// out-neighbour of many active vertices, and on PageRank (200 K vertices,
+// 3 M edges, most of them active) nearly every edge finds its bit set; a
+// stale clear bit (plain, L1-cached load) only repeats the same OR.  (A
+// second test in L2 before the atomic measured 23 + 22 us for the two
+// kernels below against 19 + 18: the reduction is not waited for, the load
+// is.)
+__device__ __forceinline__ void activate(uint32_t *bits, uint32_t w) {
+  uint32_t *p = bits + (w >> 5);
+  const uint32_t m = 1u << (w & 31);
+  if (!(*p & m)) atomicOr(p, m);
+}
+
+// Rows of more than kXLight out-edges leave their edges as chunks of kXChunk
+// for k_expand_chunks: at most E / kXLight entries.
+constexpr int kXLight = 64;
+constexpr int kXChunk = 256;
+
+// k_expand_rows' results: chunks listed, out-edges of the applied vertices.
+struct ExpandCtl {
+  int32_t n_chunks, n_edges;
 };
 
+// A warp takes 32 active slots: it commits their new vertex data (slot !=
+// null; vd[act[i]] = slot[i], after every gather of the iteration has read
+// the old values), lists the chunks of the heavy rows (one atomic per warp)
+// and walks the light rows' edges laid end to end, 64 per round.  This and
+// k_expand_chunks replace a commit, a three-kernel scan of the out-degrees,
+// a partition and a tile walk over it: the bits set do not depend on the
+// order, so no scan is needed.  Bound by the reductions on words that
+// several SMs fill at once: the two take 19 + 18 us on average over a
+// PageRank run (200 K vertices, 3 M edges), where the kernels before took
+// 132 us.
 __global__ void __launch_bounds__(kNT)
-    k_expand(ExpandPol pol, SegSource src) {
-  gasdev::tile_loop<ExpandPol, false, false>(pol, src, nullptr, nullptr, nullptr);
+    k_expand_rows(const int32_t *act, const gas_counters *cnt, const uint8_t *ret,
+                  const int32_t *csr_off, const int32_t *csr_dst, uint32_t *bits,
+                  const uint8_t *slot, uint8_t *vd, int vbytes, int2 *chunks,
+                  ExpandCtl *ctl) {
+  constexpr unsigned FULL = 0xffffffffu;
+  __shared__ int s_start[kNT / 32][32], s_excl[kNT / 32][32];
+  const int n = cnt->n_active;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
+  const unsigned below = (1u << lane) - 1u;
+  int edges = 0;
+  for (long long base = 32LL * gwarp; base < n; base += 32LL * nwarps) {
+    const long long i = base + lane;
+    int off = 0, deg = 0;
+    if (i < n) {
+      const int v = act[i];
+      if (slot) {
+        if ((vbytes & 3) == 0) {
+          const int w = vbytes >> 2;
+          const uint32_t *s = reinterpret_cast<const uint32_t *>(slot) + (size_t)i * w;
+          uint32_t *d = reinterpret_cast<uint32_t *>(vd) + (size_t)v * w;
+          for (int k = 0; k < w; ++k) d[k] = s[k];
+        } else {
+          for (int k = 0; k < vbytes; ++k)
+            vd[(size_t)v * vbytes + k] = slot[(size_t)i * vbytes + k];
+        }
+      }
+      if (ret[i]) {
+        off = csr_off[v];
+        deg = csr_off[v + 1] - off;
+      }
+    }
+    edges += deg;
+    unsigned hb = __ballot_sync(FULL, deg > kXLight);
+    if (hb) {  // warp-uniform
+      const int nc = deg > kXLight ? (deg + kXChunk - 1) / kXChunk : 0;
+      const int incl = warp_incl_sum(nc);
+      int at = 0;
+      if (lane == 31) at = atomicAdd(&ctl->n_chunks, incl);
+      at = __shfl_sync(FULL, at, 31) + incl - nc;
+      for (; hb; hb &= hb - 1) {
+        const int l = __ffs(hb) - 1;
+        const int o = __shfl_sync(FULL, off, l), d = __shfl_sync(FULL, deg, l);
+        const int p = __shfl_sync(FULL, at, l), c = __shfl_sync(FULL, nc, l);
+        for (int k = lane; k < c; k += 32)
+          chunks[p + k] = make_int2(o + k * kXChunk, o + min(d, (k + 1) * kXChunk));
+      }
+    }
+    // light rows, without the empty ones, to consecutive places
+    const bool light = deg > 0 && deg <= kXLight;
+    const unsigned lb = __ballot_sync(FULL, light);
+    if (!lb) continue;  // warp-uniform
+    const int rows = __popc(lb);
+    const int incl = warp_incl_sum(light ? deg : 0);
+    const int T = __shfl_sync(FULL, incl, 31);
+    if (light) {
+      const int k = __popc(lb & below);
+      s_excl[warp][k] = incl - deg;
+      s_start[warp][k] = off;
+    }
+    __syncwarp();
+    const bool ok = lane < rows;
+    const int excl = ok ? s_excl[warp][lane] : 0;
+    const int shift = ok ? s_start[warp][lane] - excl : 0;
+    __syncwarp();
+    for (int r = 0; r < T; r += 64) {
+      int w[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r0 = r + 32 * h;
+        // the row of edge r0 is the last one starting at or before it; a bit
+        // per row that starts inside the round gives the other lanes theirs
+        const int row0 = __popc(__ballot_sync(FULL, ok && excl <= r0)) - 1;
+        const int k = excl - r0;
+        const unsigned starts =
+            __reduce_or_sync(FULL, (ok && k >= 1 && k < 32) ? (1u << k) : 0u);
+        int row = row0 + __popc(starts & ((2u << lane) - 1u));
+        row = row > 31 ? 31 : row;
+        const int pos = r0 + lane + __shfl_sync(FULL, shift, row);
+        w[h] = r0 + lane < T ? __ldg(csr_dst + pos) : -1;
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (w[h] >= 0) activate(bits, (uint32_t)w[h]);
+    }
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) edges += __shfl_xor_sync(FULL, edges, d);
+  if (lane == 0 && edges) atomicAdd(&ctl->n_edges, edges);
+}
+
+// The heavy rows' chunks, a warp each, all of a chunk's loads in flight.
+__global__ void __launch_bounds__(kNT)
+    k_expand_chunks(const int2 *chunks, const ExpandCtl *ctl, const int32_t *csr_dst,
+                    uint32_t *bits) {
+  const int n = ctl->n_chunks;
+  const int lane = threadIdx.x & 31;
+  const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
+  for (int c = gwarp; c < n; c += nwarps) {
+    const int2 r = chunks[c];
+    int w[kXChunk / 32];
+#pragma unroll
+    for (int k = 0; k < kXChunk / 32; ++k) {
+      const int pos = r.x + 32 * k + lane;
+      w[k] = pos < r.y ? __ldg(csr_dst + pos) : -1;
+    }
+#pragma unroll
+    for (int k = 0; k < kXChunk / 32; ++k)
+      if (w[k] >= 0) activate(bits, (uint32_t)w[k]);
+  }
 }
 
 // Compaction of the next-frontier bitmap into the ascending active list with
 // its in-degree scan (scatter_if_mgpu.h:130-157 + the gather's degree scan),
-// clearing the bitmap for the following iteration.
-__device__ __forceinline__ void word_stats(const uint32_t *bits,
-                                           const int32_t *off, int nW, int w,
-                                           int *c, int *d) {
-  *c = 0;
-  *d = 0;
-  if (w >= nW) return;
-  uint32_t m = bits[w];
-  *c = __popc(m);
-  while (m) {
-    const int b = __ffs(m) - 1;
-    m &= m - 1;
-    const int v = w * 32 + b;
-    *d += off[v + 1] - off[v];
+// clearing the bitmap for the following iteration.  A warp owns a run of 16
+// words and walks it in two rounds of 8, lane l taking vertex 32 w + l of
+// each word: the in-degree loads of a word are coalesced and a round's are
+// in flight together.  (A thread per 4 words, the bits of each in a serial
+// loop, left 200 K vertices to 7 CTAs: 40 us to count and 91 us to write,
+// against 5.4 and 11.)
+constexpr int kCWords = 16;                      // words per warp
+constexpr int kCRound = 8;
+constexpr int kCWarps = kNT / 32;
+constexpr int kCBlockWords = kCWords * kCWarps;  // 128 words per block
+// Up to this many blocks (8 M vertices) every block of the write pass sums
+// the totals before it; beyond, a spine kernel scans them.
+constexpr int kCSumBlocks = 2048;
+
+struct CRound {
+  int deg[kCRound];
+  uint32_t word[kCRound];
+};
+
+__device__ __forceinline__ void c_round_load(uint32_t myword, const int32_t *csc_off, int w0,
+                                             int r, CRound &q) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int i = 0; i < kCRound; ++i) {
+    q.word[i] = __shfl_sync(0xffffffffu, myword, r + i);
+    q.deg[i] = 0;
+    if ((q.word[i] >> lane) & 1u) {
+      const int v = (w0 + r + i) * 32 + lane;
+      q.deg[i] = csc_off[v + 1] - csc_off[v];
+    }
   }
 }
 
+// Members and in-edges per block (part) and per warp (wpart); also takes
+// the expansion's out-edge count and clears its control word.
 __global__ void __launch_bounds__(kNT)
-    k_compact_count(const uint32_t *bits, const int32_t *csc_off, int nW,
-                    int32_t *part) {
-  const int b = blockIdx.x;
-  int c = 0, d = 0;
-  for (int k = 0; k < kWordsPerThread; ++k) {
-    int cc, dd;
-    word_stats(bits, csc_off, nW, b * kCompactBlock + threadIdx.x * kWordsPerThread + k,
-               &cc, &dd);
-    c += cc;
-    d += dd;
+    k_compact_count(const uint32_t *bits, const int32_t *csc_off, int nW, int2 *part,
+                    int2 *wpart, ExpandCtl *ctl, gas_counters *cnt) {
+  __shared__ int2 s_t[kCWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int w0 = (blockIdx.x * kCWarps + warp) * kCWords;
+  const uint32_t myword = lane < kCWords && w0 + lane < nW ? bits[w0 + lane] : 0u;
+  const unsigned nz = __ballot_sync(0xffffffffu, myword != 0u);
+  int c = __popc(myword), d = 0;
+#pragma unroll 1
+  for (int r = 0; r < kCWords; r += kCRound) {
+    if (!((nz >> r) & ((1u << kCRound) - 1u))) continue;  // warp-uniform
+    CRound q;
+    c_round_load(myword, csc_off, w0, r, q);
+#pragma unroll
+    for (int i = 0; i < kCRound; ++i) d += q.deg[i];
   }
-  int tc, td;
-  block_excl_sum(c, &tc);
-  block_excl_sum(d, &td);
-  if (threadIdx.x == 0) {
-    part[2 * b] = tc;
-    part[2 * b + 1] = td;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    c += __shfl_xor_sync(0xffffffffu, c, o);
+    d += __shfl_xor_sync(0xffffffffu, d, o);
   }
-}
-
-__global__ void __launch_bounds__(kNT)
-    k_compact_spine(int32_t *part, int nb, gas_counters *cnt) {
-  // de-interleave in place is awkward; scan the two series one after the
-  // other with a stride-2 view.
-  __shared__ int s_carry[2];
-  if (threadIdx.x < 2) s_carry[threadIdx.x] = 0;
+  if (lane == 0) {
+    s_t[warp] = make_int2(c, d);
+    wpart[blockIdx.x * kCWarps + warp] = make_int2(c, d);
+  }
   __syncthreads();
+  if (threadIdx.x == 0) {
+    int2 t = make_int2(0, 0);
+    for (int k = 0; k < kCWarps; ++k) {
+      t.x += s_t[k].x;
+      t.y += s_t[k].y;
+    }
+    part[blockIdx.x] = t;
+    if (blockIdx.x == 0) {
+      cnt->n_scatter_edges = ctl->n_edges;
+      ctl->n_edges = 0;
+      ctl->n_chunks = 0;
+    }
+  }
+}
+
+// More than kCSumBlocks blocks: part[] becomes its exclusive scan.
+__global__ void __launch_bounds__(kNT) k_compact_spine(int2 *part, int nb) {
+  int2 carry = make_int2(0, 0);
   for (int base = 0; base < nb; base += kNT) {
     const int i = base + threadIdx.x;
-    const int vc = i < nb ? part[2 * i] : 0;
-    const int vd = i < nb ? part[2 * i + 1] : 0;
+    const int2 v = i < nb ? part[i] : make_int2(0, 0);
     int tc, td;
-    const int ec = block_excl_sum(vc, &tc);
-    const int ed = block_excl_sum(vd, &td);
-    const int cc = s_carry[0], cd = s_carry[1];
-    if (i < nb) {
-      part[2 * i] = cc + ec;
-      part[2 * i + 1] = cd + ed;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      s_carry[0] = cc + tc;
-      s_carry[1] = cd + td;
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    cnt->n_active = s_carry[0];
-    cnt->n_edges = s_carry[1];
+    const int ec = block_excl_sum(v.x, &tc);
+    const int ed = block_excl_sum(v.y, &td);
+    if (i < nb) part[i] = make_int2(carry.x + ec, carry.y + ed);
+    carry.x += tc;
+    carry.y += td;
   }
 }
 
+// Loop control of a device-side run, done by the last block of the
+// compaction: one more iteration while the frontier is non-empty and the cap
+// is not reached; reaching the cap with work left raises the error word.
+struct LoopEnd {
+  int on;        // 0: the step API, whose host decides
+  int in_graph;  // the condition of a WHILE node is set as well
+  cudaGraphConditionalHandle h;
+};
+
+// The active list, its in-degree scan and the totals.  tile > 0: also the
+// next gather's tile partition -- the merge-path boundary of tile t lies in
+// the segment a with a + scan[a] <= t * tile <= a + scan[a + 1], so each
+// member writes the boundaries inside its own range and no tile has to
+// search for its own (k_partition, 10 us of dependent loads per iteration).
 __global__ void __launch_bounds__(kNT)
-    k_compact_write(uint32_t *bits, const int32_t *csc_off, int nW,
-                    const int32_t *part, int32_t *act, int32_t *scan,
-                    const gas_counters *cnt) {
-  const int b = blockIdx.x;
-  const int w0 = b * kCompactBlock + threadIdx.x * kWordsPerThread;
-  int c = 0, d = 0;
-  for (int k = 0; k < kWordsPerThread; ++k) {
-    int cc, dd;
-    word_stats(bits, csc_off, nW, w0 + k, &cc, &dd);
-    c += cc;
-    d += dd;
+    k_compact_write(uint32_t *bits, const int32_t *csc_off, int nW, const int2 *part,
+                    const int2 *wpart, int scanned, int32_t *act, int32_t *scan,
+                    int32_t *tile_part, int tile, gas_counters *cnt, LoopEnd end) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int w0 = (blockIdx.x * kCWarps + warp) * kCWords;
+  const uint32_t myword = lane < kCWords && w0 + lane < nW ? bits[w0 + lane] : 0u;
+  const bool last_block = blockIdx.x == gridDim.x - 1;
+  if (!__syncthreads_or(myword != 0u) && !last_block) return;
+  int2 base;
+  if (scanned) {
+    base = part[blockIdx.x];
+  } else {
+    int c = 0, d = 0;
+    for (int b = threadIdx.x; b < (int)blockIdx.x; b += kNT) {
+      const int2 t = part[b];
+      c += t.x;
+      d += t.y;
+    }
+    block_excl_sum(c, &base.x);
+    block_excl_sum(d, &base.y);
   }
-  int tc, td;
-  int pc = block_excl_sum(c, &tc) + part[2 * b];
-  int pd = block_excl_sum(d, &td) + part[2 * b + 1];
-  for (int k = 0; k < kWordsPerThread; ++k) {
-    const int w = w0 + k;
-    if (w >= nW) break;
-    uint32_t m = bits[w];
-    if (!m) continue;
-    bits[w] = 0;
-    while (m) {
-      const int bit = __ffs(m) - 1;
-      m &= m - 1;
-      const int v = w * 32 + bit;
-      act[pc] = v;
-      scan[pc] = pd;
-      ++pc;
-      pd += csc_off[v + 1] - csc_off[v];
+  for (int k = 0; k < warp; ++k) {
+    const int2 t = wpart[blockIdx.x * kCWarps + k];
+    base.x += t.x;
+    base.y += t.y;
+  }
+  int bq = base.x, bd = base.y;
+  const unsigned nz = __ballot_sync(FULL, myword != 0u);
+  const unsigned below = (1u << lane) - 1u;
+#pragma unroll 1
+  for (int r = 0; r < kCWords; r += kCRound) {
+    if (!((nz >> r) & ((1u << kCRound) - 1u))) continue;  // warp-uniform
+    CRound q;
+    c_round_load(myword, csc_off, w0, r, q);
+#pragma unroll
+    for (int i = 0; i < kCRound; ++i) {
+      const uint32_t word = q.word[i];
+      if (!word) continue;  // warp-uniform
+      const int deg = q.deg[i];
+      const int incl = warp_incl_sum(deg);
+      const int pos = bq + __popc(word & below), beg = bd + incl - deg;
+      int t0 = 0, t1 = -1;
+      if ((word >> lane) & 1u) {
+        act[pos] = (w0 + r + i) * 32 + lane;
+        scan[pos] = beg;
+        if (tile) {
+          t0 = (int)(((unsigned)(pos + beg) + tile - 1u) / (unsigned)tile);
+          t1 = (int)((unsigned)(pos + beg + deg) / (unsigned)tile);
+        }
+      }
+      if (tile) {
+        unsigned big = __ballot_sync(FULL, t1 - t0 >= 4);  // hubs, by the whole warp
+        if (t1 - t0 < 4)
+          for (int t = t0; t <= t1; ++t) tile_part[t] = pos;
+        for (; big; big &= big - 1) {
+          const int l = __ffs(big) - 1;
+          const int p = __shfl_sync(FULL, pos, l), e = __shfl_sync(FULL, t1, l);
+          for (int t = __shfl_sync(FULL, t0, l) + lane; t <= e; t += 32) tile_part[t] = p;
+        }
+      }
+      bq += __popc(word);
+      bd += __shfl_sync(FULL, incl, 31);
     }
   }
-  if (b == 0 && threadIdx.x == 0) scan[cnt->n_active] = cnt->n_edges;
+  if (myword) bits[w0 + lane] = 0u;
+  if (last_block && warp == kCWarps - 1 && lane == 0) {  // bq, bd: the totals
+    scan[bq] = bd;
+    cnt->n_active = bq;
+    cnt->n_edges = bd;
+    // every tile boundary past the last one is the end of the path
+    if (tile) tile_part[(int)(((long long)bq + bd + tile - 1) / tile)] = bq;
+    if (end.on) {
+      const int it = ++cnt->iteration;
+      if (bq > 0 && it >= cnt->max_iter) cnt->error = GAS_ERR_ITER_CAP;
+      cnt->cond = (bq > 0 && it < cnt->max_iter) ? 1 : 0;
+      if (end.in_graph) cudaGraphSetConditional(end.h, cnt->cond);
+    }
+  }
 }
 
 // BFS apply without gather (bfs.cu:58-71): level from the engine.
@@ -484,11 +608,11 @@ void free_graph(gas_engine *e) {
     dfree(e->csc_src); dfree(e->csr_dst); dfree(e->csc_ed); dfree(e->csr_ed);
   }
   e->edges_on_host = false;
-  dfree(e->vd); dfree(e->act); dfree(e->scan); dfree(e->sscan); dfree(e->ret);
+  dfree(e->vd); dfree(e->act); dfree(e->scan); dfree(e->ret);
   dfree(e->slot); dfree(e->gres); dfree(e->bits);
   dfree(e->tile_first); dfree(e->tile_carry); dfree(e->tile_a0);
-  dfree(e->tpart); dfree(e->dpart);
-  dfree(e->ppart); dfree(e->cpart); dfree(e->cnt);
+  dfree(e->tpart); dfree(e->xchunks); dfree(e->xctl);
+  dfree(e->cpart); dfree(e->cnt);
   for (int i = 0; i < 2; ++i) { dfree(e->pr_rank[i]); dfree(e->pr_contrib[i]); }
   dfree(e->pr_seed); dfree(e->pr_inv_deg); dfree(e->pr_l1); dfree(e->csr_to_csc);
   dfree(e->pr_tile_row); dfree(e->pr_head); dfree(e->pr_tail);
@@ -548,10 +672,14 @@ gas_status_t sync_counts(gas_engine *e, void *stream) {
   return GAS_OK;
 }
 
-// Launch the generic gather (fused with apply or not) for program P.
+// Merge items per gather tile of the built-in programs (4-byte values).
+constexpr int kBuiltinTile = gasdev::TileShape<4>::kTile;
+
+// Launch the generic gather (fused with apply or not) for program P;
+// partitioned: the compaction that made the frontier wrote its partition.
 template <class P>
 gas_status_t launch_generic_gather(gas_engine *e, bool fuse, bool ordered,
-                                   void *stream) {
+                                   bool partitioned, void *stream) {
   using GR = typename P::GatherResult;
   gasdev::GenericGather<P> pol;
   pol.csc_src = e->csc_src;
@@ -571,9 +699,11 @@ gas_status_t launch_generic_gather(gas_engine *e, bool fuse, bool ordered,
   const SegSource src = gasdev::frontier_source(
       e->act, e->scan, e->csc_off, &e->cnt->n_active, &e->cnt->n_edges, e->tpart);
   constexpr int kTile = gasdev::TileShape<sizeof(GR)>::kTile;
+  static_assert(kTile == kBuiltinTile, "the compaction writes this tile's partition");
   const int64_t items = (int64_t)e->n_active + e->n_edges;
-  gasdev::k_partition<kTile, false>
-      <<<gas::engine_partition_grid(e, items, kTile), 256, 0, S(stream)>>>(src, e->tpart);
+  if (!partitioned)
+    gasdev::k_partition<kTile, false>
+        <<<gas::engine_partition_grid(e, items, kTile), 256, 0, S(stream)>>>(src, e->tpart);
   const int cap = occupancy_grid(e, gasdev::k_gather_tiles<P>);
   const int grid = e->capturing ? cap : grid_for(items, kTile, cap);
   gasdev::k_gather_tiles<P><<<grid, kNT, 0, S(stream)>>>(
@@ -591,11 +721,11 @@ gas_status_t launch_generic_gather(gas_engine *e, bool fuse, bool ordered,
 }
 
 gas_status_t builtin_gather(gas_engine *e, bool fuse, bool ordered,
-                            void *stream) {
+                            bool partitioned, void *stream) {
   switch (e->prog) {
-    case GAS_PROG_SSSP: return launch_generic_gather<progs::Sssp>(e, fuse, ordered, stream);
-    case GAS_PROG_CC: return launch_generic_gather<progs::Cc>(e, fuse, ordered, stream);
-    case GAS_PROG_PAGERANK: return launch_generic_gather<progs::PageRank>(e, fuse, ordered, stream);
+    case GAS_PROG_SSSP: return launch_generic_gather<progs::Sssp>(e, fuse, ordered, partitioned, stream);
+    case GAS_PROG_CC: return launch_generic_gather<progs::Cc>(e, fuse, ordered, partitioned, stream);
+    case GAS_PROG_PAGERANK: return launch_generic_gather<progs::PageRank>(e, fuse, ordered, partitioned, stream);
     default: return GAS_OK;  // BFS: gatherMap/gatherReduce are no-ops
   }
 }
@@ -631,41 +761,30 @@ gas_status_t builtin_apply_only(gas_engine *e, void *stream) {
   return GAS_OK;
 }
 
-// commit pending slots, expand, compact.
-gas_status_t scatter_common(gas_engine *e, void *stream) {
-  if (e->slots_pending) {
-    const int g = e->capturing ? 8 * e->num_sms
-                               : grid_for(e->n_active, kNT, 8 * e->num_sms);
-    k_commit<<<g, kNT, 0, S(stream)>>>(
-        e->act, e->cnt, (const uint8_t *)e->slot, (uint8_t *)e->vd,
-        (int)e->vbytes);
-    CUDA_TRY(cudaGetLastError());
-    e->slots_pending = false;
-  }
-  const int nblk = grid_for(e->nV, kScanBlock, INT_MAX);
-  k_pscan_reduce<<<nblk, kNT, 0, S(stream)>>>(e->act, e->ret, e->csr_off,
-                                               e->cnt, e->ppart);
-  k_pscan_spine<<<1, kNT, 0, S(stream)>>>(e->ppart, e->cnt);
-  k_pscan_down<<<nblk, kNT, 0, S(stream)>>>(e->act, e->ret, e->csr_off, e->cnt,
-                                             e->ppart, e->sscan);
+// commit pending slots, expand, compact; end: the loop control of a
+// device-side run.
+gas_status_t scatter_common(gas_engine *e, void *stream, const LoopEnd &end) {
+  const uint8_t *slot = e->slots_pending ? (const uint8_t *)e->slot : nullptr;
+  e->slots_pending = false;
+  ExpandCtl *ctl = static_cast<ExpandCtl *>(e->xctl);
+  int2 *chunks = static_cast<int2 *>(e->xchunks);
+  // the active and chunk counts are only known on the device: fixed grids
+  k_expand_rows<<<grid_for(e->nV, kNT, 8 * e->num_sms), kNT, 0, S(stream)>>>(
+      e->act, e->cnt, e->ret, e->csr_off, e->csr_dst, e->bits, slot, (uint8_t *)e->vd,
+      (int)e->vbytes, chunks, ctl);
+  k_expand_chunks<<<grid_for(e->nE / kXLight, kNT / 32, 8 * e->num_sms), kNT, 0, S(stream)>>>(
+      chunks, ctl, e->csr_dst, e->bits);
   CUDA_TRY(cudaGetLastError());
-  ExpandPol pol{e->csr_dst, e->bits};
-  const SegSource src = gasdev::frontier_source(
-      e->act, e->sscan, e->csr_off, &e->cnt->n_active, &e->cnt->n_scatter_edges,
-      e->tpart);
-  constexpr int kTile = gasdev::TileShape<sizeof(int32_t)>::kTile;
-  // the scatter edge count is only known on the device: fixed grids
-  gasdev::k_partition<kTile, false>
-      <<<gas::engine_partition_grid(e, -1, kTile), 256, 0, S(stream)>>>(src, e->tpart);
-  k_expand<<<occupancy_grid(e, k_expand), kNT, 0, S(stream)>>>(pol, src);
+  const int nW = (e->nV + 31) / 32, nb = e->n_cblocks;
+  int2 *part = static_cast<int2 *>(e->cpart), *wpart = part + nb;
+  const int tile = e->prog == GAS_PROG_USER ? 0 : kBuiltinTile;  // users partition themselves
+  k_compact_count<<<nb, kNT, 0, S(stream)>>>(e->bits, e->csc_off, nW, part, wpart, ctl, e->cnt);
+  if (nb > kCSumBlocks) k_compact_spine<<<1, kNT, 0, S(stream)>>>(part, nb);
+  k_compact_write<<<nb, kNT, 0, S(stream)>>>(e->bits, e->csc_off, nW, part, wpart,
+                                             nb > kCSumBlocks ? 1 : 0, e->act, e->scan,
+                                             e->tpart, tile, e->cnt, end);
   CUDA_TRY(cudaGetLastError());
-  const int nW = (e->nV + 31) / 32;
-  k_compact_count<<<e->n_cblocks, kNT, 0, S(stream)>>>(e->bits, e->csc_off, nW,
-                                                        e->cpart);
-  k_compact_spine<<<1, kNT, 0, S(stream)>>>(e->cpart, e->n_cblocks, e->cnt);
-  k_compact_write<<<e->n_cblocks, kNT, 0, S(stream)>>>(
-      e->bits, e->csc_off, nW, e->cpart, e->act, e->scan, e->cnt);
-  CUDA_TRY(cudaGetLastError());
+  e->tpart_valid = tile > 0;
   e->counts_dirty = true;
   e->have_gres = false;
   e->active_full = false;
@@ -677,7 +796,7 @@ gas_status_t flush_pending_gather(gas_engine *e, void *stream) {
   e->pending_gather = false;
   if (e->prog == GAS_PROG_USER)
     return gas::fail(GAS_ERR_STATE, "user engine: gather must be launched by the header");
-  GAS_TRY(builtin_gather(e, /*fuse=*/false, false, stream));
+  GAS_TRY(builtin_gather(e, /*fuse=*/false, false, e->tpart_valid, stream));
   e->have_gres = true;
   return GAS_OK;
 }
@@ -846,7 +965,6 @@ gas_status_t gas_engine_set_graph(gas_engine *e, int32_t nV, void *vertex_data,
   GAS_TRY(dalloc((uint8_t **)&e->vd, V * e->vbytes));
   GAS_TRY(dalloc(&e->act, V));
   GAS_TRY(dalloc(&e->scan, V + 1));
-  GAS_TRY(dalloc(&e->sscan, V + 1));
   GAS_TRY(dalloc(&e->ret, V));
   GAS_TRY(dalloc((uint8_t **)&e->slot, V * e->vbytes));
   GAS_TRY(dalloc((uint8_t **)&e->gres, V * std::max<size_t>(e->gbytes, 4)));
@@ -860,10 +978,12 @@ gas_status_t gas_engine_set_graph(gas_engine *e, int32_t nV, void *vertex_data,
   GAS_TRY(dalloc((uint8_t **)&e->tile_carry, (size_t)e->tile_cap * tv));
   GAS_TRY(dalloc(&e->tile_a0, (size_t)e->tile_cap));
   GAS_TRY(dalloc(&e->tpart, (size_t)e->tile_cap + 2));
-  GAS_TRY(dalloc(&e->dpart, (size_t)e->tile_cap + 2));
-  GAS_TRY(dalloc(&e->ppart, (V + kScanBlock - 1) / kScanBlock + 1));
-  e->n_cblocks = (int32_t)std::max<size_t>(1, (nW + kCompactBlock - 1) / kCompactBlock);
-  GAS_TRY(dalloc(&e->cpart, 2 * (size_t)e->n_cblocks));
+  // a row of d > kXLight out-edges lists ceil(d / kXChunk) <= d / kXLight chunks
+  GAS_TRY(dalloc((int2 **)&e->xchunks, E / kXLight + 1));
+  GAS_TRY(dalloc((ExpandCtl **)&e->xctl, 1));
+  e->n_cblocks = (int32_t)std::max<size_t>(1, (nW + kCBlockWords - 1) / kCBlockWords);
+  // block totals, then the blocks' per-warp totals
+  GAS_TRY(dalloc((int2 **)&e->cpart, (size_t)e->n_cblocks * (1 + kCWarps)));
   GAS_TRY(dalloc(&e->cnt, 1));
 
   if (dev_build)
@@ -937,6 +1057,7 @@ gas_status_t gas_engine_set_graph(gas_engine *e, int32_t nV, void *vertex_data,
   if (V)
     CUDA_TRY(cudaMemcpyAsync(e->vd, vertex_data, V * e->vbytes, cudaMemcpyHostToDevice, st));
   CUDA_TRY(cudaMemsetAsync(e->bits, 0, nW * 4, st));
+  CUDA_TRY(cudaMemsetAsync(e->xctl, 0, sizeof(ExpandCtl), st));
   CUDA_TRY(cudaMemsetAsync(e->slab_fix_n, 0, sizeof(int32_t), st));
   CUDA_TRY(cudaMemsetAsync(e->hist, 0, 8 * sizeof(int32_t), st));
   CUDA_TRY(cudaMemsetAsync(e->trace, 0, GAS_TRACE_CAP * sizeof(gas_trace_record), st));
@@ -947,6 +1068,7 @@ gas_status_t gas_engine_set_graph(gas_engine *e, int32_t nV, void *vertex_data,
   e->n_active = 0;
   e->n_edges = 0;
   e->counts_dirty = false;
+  e->tpart_valid = false;
   e->pending_gather = e->have_gres = e->slots_pending = false;
   e->level = 0;
   e->has_graph = true;
@@ -970,6 +1092,7 @@ gas_status_t gas_engine_set_active(gas_engine *e, int32_t start, int32_t end,
   k_set_range<<<grid_for((int64_t)n + 1, kNT, 8 * e->num_sms), kNT, 0, S(stream)>>>(
       start, n, e->csc_off, e->act, e->scan, e->cnt);
   CUDA_TRY(cudaGetLastError());
+  e->tpart_valid = false;
   e->n_active = n;
   e->n_edges = e->h_csc_off[end] - e->h_csc_off[start];
   e->counts_dirty = false;
@@ -1003,7 +1126,7 @@ gas_status_t gas_engine_apply(gas_engine *e, void *stream) {
   if (e->n_active == 0) return GAS_OK;
   if (e->pending_gather) {
     e->pending_gather = false;
-    GAS_TRY(builtin_gather(e, /*fuse=*/true, false, stream));
+    GAS_TRY(builtin_gather(e, /*fuse=*/true, false, e->tpart_valid, stream));
     e->slots_pending = true;
     return GAS_OK;
   }
@@ -1016,7 +1139,7 @@ gas_status_t gas_engine_scatter_activate(gas_engine *e, int32_t have_scatter,
   if (!e || !e->has_graph) return gas::fail(GAS_ERR_STATE, "scatter before set_graph");
   if (e->counts_dirty) GAS_TRY(sync_counts(e, stream));
   GAS_TRY(flush_pending_gather(e, stream));
-  return scatter_common(e, stream);
+  return scatter_common(e, stream, LoopEnd{});
 }
 
 gas_status_t gas_engine_next_iter(gas_engine *e, int32_t *n_active, void *stream) {
@@ -1260,8 +1383,8 @@ void prof_collect(gas_engine *e) {
   e->prof_kind = -1;
 }
 
-gas_status_t engine_scatter(gas_engine *e, void *stream) {
-  return scatter_common(e, stream);
+gas_status_t engine_scatter_loop(gas_engine *e, cudaGraphConditionalHandle h, void *stream) {
+  return scatter_common(e, stream, LoopEnd{1, e->in_graph ? 1 : 0, h});
 }
 gas_status_t engine_sync_counts(gas_engine *e, void *stream) {
   return sync_counts(e, stream);
@@ -1276,7 +1399,8 @@ int engine_partition_grid(gas_engine *e, int64_t items, int tile) {
 }
 
 gas_status_t engine_gather_apply(gas_engine *e, void *stream) {
-  GAS_TRY(builtin_gather(e, true, false, stream));
+  // captured once and replayed on any active set: partitions itself
+  GAS_TRY(builtin_gather(e, true, false, false, stream));
   e->slots_pending = true;
   return GAS_OK;
 }
@@ -1293,13 +1417,26 @@ gas_status_t engine_commit(gas_engine *e, void *stream) {
   return GAS_OK;
 }
 
-gas_status_t engine_generic_iteration(gas_engine *e, bool ordered, void *stream) {
+gas_status_t engine_generic_iteration(gas_engine *e, bool ordered,
+                                      cudaGraphConditionalHandle h, void *stream) {
   if (e->prog == GAS_PROG_BFS) {
     GAS_TRY(builtin_apply_only(e, stream));
   } else {
-    GAS_TRY(builtin_gather(e, true, ordered, stream));
+    GAS_TRY(builtin_gather(e, true, ordered, /*partitioned=*/true, stream));
     e->slots_pending = true;
   }
-  return scatter_common(e, stream);
+  return engine_scatter_loop(e, h, stream);
 }
+
+gas_status_t engine_partition(gas_engine *e, void *stream) {
+  const SegSource src = gasdev::frontier_source(
+      e->act, e->scan, e->csc_off, &e->cnt->n_active, &e->cnt->n_edges, e->tpart);
+  gasdev::k_partition<kBuiltinTile, false>
+      <<<engine_partition_grid(e, (int64_t)e->n_active + e->n_edges, kBuiltinTile), 256, 0,
+         S(stream)>>>(src, e->tpart);
+  CUDA_TRY(cudaGetLastError());
+  return GAS_OK;
+}
+
+int engine_scatter_kernels(const gas_engine *e) { return e->n_cblocks > kCSumBlocks ? 5 : 4; }
 }  // namespace gas

@@ -56,7 +56,7 @@ struct gas_engine {
 
   // device vertex + frontier state
   void *vd = nullptr;
-  int32_t *act = nullptr, *scan = nullptr, *sscan = nullptr;
+  int32_t *act = nullptr, *scan = nullptr;
   uint8_t *ret = nullptr;
   void *slot = nullptr, *gres = nullptr;
   uint32_t *bits = nullptr;
@@ -64,9 +64,9 @@ struct gas_engine {
   int32_t *tile_a0 = nullptr;
   int32_t tile_cap = 0;
   int32_t *tpart = nullptr;  // tile partitions of the current frontier pass
-  int32_t *dpart = nullptr;  // tile partitions of the dense CSC (pull passes)
-  int32_t *ppart = nullptr;  // predicated-scan partials
-  int32_t *cpart = nullptr;  // compaction partials (pairs)
+  bool tpart_valid = false;  // the compaction wrote them for the active list
+  void *xchunks = nullptr, *xctl = nullptr;  // expansion: heavy-row chunks, control word
+  void *cpart = nullptr;     // compaction totals (pairs): blocks, then warps
   int32_t n_cblocks = 0;
   gas_counters *cnt = nullptr;
   gas_counters *h_cnt = nullptr;  // pinned
@@ -142,10 +142,16 @@ struct gas_engine {
 };
 
 namespace gas {
-// commit pending slots + expansion + compaction of the next frontier
-gas_status_t engine_scatter(gas_engine *e, void *stream);
-// one bulk-synchronous iteration of the generic (step API) kernels
-gas_status_t engine_generic_iteration(gas_engine *e, bool ordered, void *stream);
+// commit pending slots + expansion + compaction of the next frontier, then
+// the loop control of a device-side run (the WHILE condition while capturing)
+gas_status_t engine_scatter_loop(gas_engine *e, cudaGraphConditionalHandle h, void *stream);
+// its kernels
+int engine_scatter_kernels(const gas_engine *e);
+// one bulk-synchronous iteration of the generic (step API) kernels; the
+// frontier's tile partition must be there (engine_partition before the first)
+gas_status_t engine_generic_iteration(gas_engine *e, bool ordered,
+                                      cudaGraphConditionalHandle h, void *stream);
+gas_status_t engine_partition(gas_engine *e, void *stream);
 // pieces of it: fused gather+apply into slots / apply only / commit slots
 gas_status_t engine_gather_apply(gas_engine *e, void *stream);
 gas_status_t engine_apply_only(gas_engine *e, void *stream);

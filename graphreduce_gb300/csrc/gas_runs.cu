@@ -27,18 +27,6 @@ namespace {
 
 inline cudaStream_t S(void *s) { return (cudaStream_t)s; }
 
-// Loop condition: one more iteration while the frontier is non-empty and the
-// cap is not reached; hitting the cap with work left raises the error word.
-__global__ void k_loop_cond(gas_counters *cnt, cudaGraphConditionalHandle h,
-                            int in_graph) {
-  const int max_iter = cnt->max_iter;
-  const int it = ++cnt->iteration;
-  const bool more = cnt->n_active > 0;
-  if (more && it >= max_iter) cnt->error = GAS_ERR_ITER_CAP;
-  cnt->cond = (more && it < max_iter) ? 1 : 0;
-  if (in_graph) cudaGraphSetConditional(h, cnt->cond);
-}
-
 __global__ void k_reset_loop(gas_counters *cnt, int32_t max_iter) {
   cnt->iteration = 0;
   cnt->error = 0;
@@ -166,10 +154,7 @@ struct GenericCtx {
 gas_status_t generic_body(gas_engine *e, cudaStream_t cs,
                           cudaGraphConditionalHandle h, void *ctx) {
   const GenericCtx *c = static_cast<const GenericCtx *>(ctx);
-  GAS_TRY(gas::engine_generic_iteration(e, c->ordered, cs));
-  k_loop_cond<<<1, 1, 0, cs>>>(e->cnt, h, e->in_graph ? 1 : 0);
-  CUDA_TRY(cudaGetLastError());
-  return GAS_OK;
+  return gas::engine_generic_iteration(e, c->ordered, h, cs);
 }
 
 }  // namespace
@@ -196,6 +181,8 @@ extern "C" gas_status_t gas_engine_run_schedule(gas_engine *e,
     return gas::run_fast(e, schedule, max_iterations, stats, stream);
 
   GenericCtx ctx{schedule == GAS_SCHED_ORDERED};
+  const bool gathers = e->prog != GAS_PROG_BFS && !ctx.ordered;
+  if (gathers) GAS_TRY(gas::engine_partition(e, stream));  // the first iteration's
   const int slot = ctx.ordered ? kGraphOrdered : kGraphGeneric;
   if (gas::host_loop_for(e)) {
     k_reset_loop<<<1, 1, 0, S(stream)>>>(e->cnt, max_iterations);
@@ -222,9 +209,11 @@ extern "C" gas_status_t gas_engine_run_schedule(gas_engine *e,
   GAS_TRY(gas_engine_read_counters(e, &c, stream));
   if (stats) {
     stats->iterations = c.iteration;
-    // per iteration: gather tiles + fixup (or BFS apply), commit, 3 scan
-    // passes, expand, 3 compaction passes, loop condition; plus the reset
-    stats->kernel_launches = c.iteration * (e->prog == GAS_PROG_BFS ? 9 : 11) + 1;
+    // per iteration: gather tiles + fixup (ordered: one kernel; BFS: apply),
+    // commit + expansion in two, compaction in two or three, the last of
+    // them also the loop condition; plus the reset and the first partition
+    stats->kernel_launches =
+        c.iteration * ((gathers ? 2 : 1) + gas::engine_scatter_kernels(e)) + (gathers ? 2 : 1);
     stats->graph_launches = gas::host_loop_for(e) ? 0 : 1;
   }
   e->level = c.iteration;
@@ -251,10 +240,7 @@ gas_status_t user_body(gas_engine *e, cudaStream_t cs, cudaGraphConditionalHandl
   GAS_TRY(u->step(u->ctx, cs));
   CUDA_TRY(cudaGetLastError());
   e->slots_pending = u->wrote_slots != 0;
-  GAS_TRY(gas::engine_scatter(e, cs));
-  k_loop_cond<<<1, 1, 0, cs>>>(e->cnt, h, e->in_graph ? 1 : 0);
-  CUDA_TRY(cudaGetLastError());
-  return GAS_OK;
+  return gas::engine_scatter_loop(e, h, cs);
 }
 
 }  // namespace
@@ -303,9 +289,9 @@ extern "C" gas_status_t gas_engine_run_user(gas_engine *e, gas_user_step_fn step
   GAS_TRY(gas_engine_read_counters(e, &c, stream));
   if (stats) {
     stats->iterations = c.iteration;
-    // per iteration: the caller's partition, tiles and fixup; commit, 3 scan
-    // passes, partition, expand, 3 compaction passes, loop condition; reset
-    stats->kernel_launches = 13 * c.iteration + 1;
+    // per iteration: the caller's partition, tiles and fixup, then commit +
+    // expansion and compaction with the loop condition; reset
+    stats->kernel_launches = (3 + gas::engine_scatter_kernels(e)) * c.iteration + 1;
     stats->graph_launches = direct ? 0 : 1;
   }
   e->level = c.iteration;
