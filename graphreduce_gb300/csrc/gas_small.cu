@@ -49,7 +49,7 @@ constexpr int kSbHeavy = 256;   // out-edges of a member walked by the grid
 using gasgrid::warp_add;
 
 struct SmallCtl {
-  gasgrid::Barrier bar;  // bar.err: 1 a barrier wait gave up
+  gasgrid::Barrier bar;
   int iterations;
   int n_push, n_pull;
   int n_heavy[2];        // heavy members listed at a level (by level parity)
@@ -64,15 +64,19 @@ __global__ void __launch_bounds__(kSbNT, 1)
                 int32_t *depth, const int32_t *__restrict__ act, int n_act, uint32_t *bits,
                 int32_t *heavy, int nW, int nV, long long nE, int forced, int max_iter,
                 SmallCtl *c, gas_counters *cnt) {
-  // a barrier wait that gave up: every CTA leaves; the error goes straight
-  // to the engine's counters (the epilogue below does not run)
-#define SB_SYNC()                                                     \
-  do {                                                                \
-    if (!gasgrid::barrier(&c->bar)) {                                 \
-      if (threadIdx.x == 0) atomicExch(&cnt->error, (int)GAS_ERR_DEVICE); \
-      return;                                                         \
-    }                                                                 \
+  // out: a control value every thread goes on with, loaded after the wait by
+  // one thread of the CTA; a barrier wait that gave up: every CTA leaves, the
+  // error goes straight to the engine's counters (the epilogue below does
+  // not run)
+#define SB_SYNC(out, load)                                                     \
+  do {                                                                         \
+    if (!gasgrid::barrier_with(&c->bar, bar, &(out), [&] { return load; })) {  \
+      if (threadIdx.x == 0) atomicExch(&cnt->error, (int)GAS_ERR_DEVICE);      \
+      return;                                                                  \
+    }                                                                          \
   } while (0)
+  unsigned int bar = c->bar.next;
+  long long fe = 0;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int nthr = gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31, gwarp = tid >> 5, nwarps = nthr >> 5;
@@ -88,14 +92,11 @@ __global__ void __launch_bounds__(kSbNT, 1)
     }
   }
   warp_add(found, &c->f_edges[0]);
-  SB_SYNC();
+  SB_SYNC(fe, __ldcg(&c->f_edges[0]));
   int it = 1;
-  // the cap stays in each CTA: marked in the barrier's error word, a CTA
-  // still leaving the previous barrier would read it as a failed wait
   bool capped = false;
   for (int k = 0;; ++k) {
     const int cur = k % 3, nxt = (k + 1) % 3, old = (k + 2) % 3;
-    const long long fe = *(volatile long long *)&c->f_edges[cur];
     if (fe == 0) break;  // A_{k+1} = N(C_k) is empty
     if (it >= max_iter) {  // every CTA stops here at the same level
       capped = true;
@@ -139,8 +140,8 @@ __global__ void __launch_bounds__(kSbNT, 1)
         }
       }
       // the heavy members: every thread of the grid over their edges
-      SB_SYNC();
-      const int nh = *(volatile int *)n_heavy;
+      int nh;
+      SB_SYNC(nh, __ldcg(n_heavy));
       for (int h = 0; h < nh; ++h) {
         const int u = __ldcg(heavy + h);
         const int b = __ldg(csr_off + u), e1 = __ldg(csr_off + u + 1);
@@ -192,20 +193,19 @@ __global__ void __launch_bounds__(kSbNT, 1)
       else
         ++c->n_push;
     }
-    SB_SYNC();
+    SB_SYNC(fe, __ldcg(&c->f_edges[nxt]));
   }
   if (kCount) warp_add(bytes, &c->bytes);
   // the next run finds the bitmaps clear (nothing reads them any more)
   for (int w = tid; w < 3 * nW; w += nthr) bits[w] = 0u;
   if (tid == 0) {
     // the engine's counters, as the fast schedule leaves them
-    // a wait that gave up in another CTA has written GAS_ERR_DEVICE already
-    const bool failed = *(volatile int *)&c->bar.err != 0;
     cnt->iteration = it;
     cnt->n_push = c->n_push;
     cnt->n_pull = c->n_pull;
-    if (!failed) cnt->error = capped ? GAS_ERR_ITER_CAP : 0;
-    if (!failed && !capped) cnt->n_active = 0;
+    cnt->error = capped ? GAS_ERR_ITER_CAP : 0;
+    if (!capped) cnt->n_active = 0;
+    c->bar.next = bar;
     // and the control word clear for the next run: its counts are read by
     // no thread after the loop (a thread still to test f_edges reads 0 and
     // leaves as well)
