@@ -31,6 +31,14 @@
 // set_graph, since their kernels capture the engine's buffers).
 // BFS runs on graphs up to this many vertices take the one-kernel path.
 constexpr int kBfsSmallMaxV = 1 << 18;
+// SSSP and CC from the full active set likewise (figures in
+// gas_small_min.cu): under AUTO up to 2^21 vertices; the kernel still halves
+// the fixed heuristic's time at 2^22, but from there on LEARNED's
+// multi-kernel push is the faster schedule and the heuristic stays what it
+// is compared with.  Under LEARNED up to 2^20: at 2^21 the multi-kernel push
+// wins on R-MAT CC (752 against 835 us).
+constexpr int kMinSmallMaxV = 1 << 21;
+constexpr int kMinSmallLearnedMaxV = 1 << 20;
 
 enum { kGraphGeneric = 0, kGraphOrdered = 1, kGraphPagerank = 2, kGraphUser = 3,
        kGraphFast0 = 4, kGraphSlots = 12 };
@@ -135,6 +143,11 @@ struct gas_engine {
   void *sb_ctl = nullptr;
   int32_t *sb_heavy = nullptr;
   bool sb_clean = false;  // the kernel left them clear for the next run
+  // small-graph SSSP and CC (gas_small_min.cu): second value buffer, the two
+  // queues, the control word
+  int32_t *sm_vals = nullptr;
+  void *sm_queue = nullptr, *sm_ctl = nullptr;
+  bool sm_clean = false;
   // what graphs[kGraphUser] was captured with (gas_engine_run_user)
   gas_user_step_fn user_step = nullptr;
   void *user_ctx = nullptr;

@@ -1137,6 +1137,8 @@ gas_status_t run_fast(gas_engine *e, gas_schedule_t schedule,
     return fail(GAS_ERR_STATE, "LEARNED schedule without a schedule model");
   if (bfs_small_eligible(e, schedule))
     return run_bfs_small(e, schedule, max_iterations, stats, stream);
+  if (min_small_eligible(e, schedule))
+    return run_min_small(e, max_iterations, stats, stream);
   GAS_TRY(ensure_fast_buffers(e));
   FastCtx ctx;
   ctx.nW = (e->nV + 31) / 32;

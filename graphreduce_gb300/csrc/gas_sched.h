@@ -33,6 +33,13 @@ bool bfs_small_eligible(const gas_engine *e, gas_schedule_t schedule);
 gas_status_t run_bfs_small(gas_engine *e, gas_schedule_t schedule, int32_t max_iterations,
                            gas_run_stats *stats, void *stream);
 
+// SSSP and CC from the full active set on a graph of at most kMinSmallMaxV
+// vertices as one cooperative kernel (gas_small_min.cu): same vertex data
+// and iteration count as run_fast.
+bool min_small_eligible(const gas_engine *e, gas_schedule_t schedule);
+gas_status_t run_min_small(gas_engine *e, int32_t max_iterations, gas_run_stats *stats,
+                           void *stream);
+
 // The loop of build_while_graph as direct launches (GAS_HOST_LOOP=1).
 gas_status_t run_host_loop(
     gas_engine *e,

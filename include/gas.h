@@ -247,6 +247,10 @@ typedef enum {
                            /* sequentially in CSC order (parity mode)      */
   GAS_SCHED_LEARNED = 5    /* push or pull per iteration from the engine's */
                            /* schedule model (gas_engine_set_schedule_model) */
+  /* SSSP and CC from the full active set: graphs of up to 2^21 (AUTO) or
+   * 2^20 (LEARNED) vertices run as one cooperative kernel that pushes in
+   * every iteration; with tracing or profiling on, and for other active
+   * sets, the per-iteration choice is made as stated. */
 } gas_schedule_t;
 
 typedef struct {
