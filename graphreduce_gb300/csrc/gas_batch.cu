@@ -29,10 +29,12 @@
 //     the L lanes of an in-edge's source are one contiguous 4L-byte read.
 //     The CSC edge range is cut into pieces of P edges (P autotuned); a group
 //     of L threads (one per lane) folds a piece in edge order with FP32
-//     two-sum compensation, finishing every row that lies inside the piece;
-//     rows cut by piece boundaries leave per-piece partials that a second
-//     pass folds in piece order.  The sums are deterministic.  The loop runs
-//     until the largest per-lane FP64 L1 residual is <= tol.
+//     two-sum compensation and stores the sum of every row that lies inside
+//     the piece; rows cut by piece boundaries leave per-piece partials that a
+//     second pass folds in a fixed order; a streaming pass turns the rows'
+//     sums into ranks, contributions and residuals.  The sums are
+//     deterministic.  The loop runs until the largest per-lane FP64 L1
+//     residual is <= tol.
 //
 // The loops are WHILE nodes of one CUDA graph (BFS, SSSP, then PPR), each
 // preceded by its prologue; a run is one cudaGraphLaunch.
@@ -70,7 +72,7 @@ struct BatchParams {
   int32_t n_sources;  // G * bfs_lanes
   int32_t sssp_max_iter;
   int32_t n_sssp_sources;  // G * sssp_lanes
-  int32_t pad;
+  int32_t n_seeds;         // G * ppr_lanes
 };
 
 __device__ __forceinline__ void set_cond(gas_counters *cnt, bool more, int it,
@@ -693,7 +695,7 @@ __global__ void __launch_bounds__(kMssSpineNT)
 // ---------------------------------------------------------------------------
 // multi-seed personalized PageRank
 // ---------------------------------------------------------------------------
-struct CVal {
+struct __align__(8) CVal {
   float s, c;
 };
 
@@ -706,185 +708,466 @@ __device__ __forceinline__ CVal two_sum_add(CVal a, CVal b) {
 }
 
 struct PprArgs {
-  const int32_t *csc_off, *csc_src, *csr_off;
-  const int32_t *first_row;  // [n_pieces] first row with an edge in the piece
-  int32_t n_pieces, P, E, L, G;
-  const int32_t *fix;        // [n_fix][3] (row, first piece, last piece):
-  int32_t n_fix;             // rows cut by pieces, then rows without
-  int32_t n_split;           // in-edges (first piece -1) from n_split on
-  CVal *head, *tail;         // [n_pieces][L] partials of cut rows
-  float *rank[2], *contrib[2];
+  const int32_t *csc_src, *csc_off, *csr_off;
+  // the rows with in-edges (vertex, end of its in-edges), and one bit per
+  // in-edge: the last of its row
+  const int32_t *ne_vid, *ne_end;
+  const uint32_t *row_bits;
+  // pieces of P edges (a multiple of kPprU): row of the first edge; and for
+  // a row that starts in the piece and goes on past it, the row and the last
+  // piece with an edge of it (-1: none)
+  const int32_t *first_row, *split_row, *split_last;
+  int32_t n_pieces, P, E, L, G, n_ne, nV;
+  CVal *head, *tail;  // [n_pieces][L] partials of cut rows
+  float *sum;         // [n_ne][L] the rows' sums of an iteration
+  float *rank, *contrib;  // [V][L]
   const uint32_t *seed_mask;
   const BatchParams *prm;
   gas_counters *cnt;
+  double *l1_part;        // [blocks][G] of k_ppr_rows
+  double *lane_resid;
+  unsigned int *ticket;   // blocks of k_ppr_rows done (left at 0)
 };
 
-struct PprLane {
-  const float *contrib, *rank_old;
-  float *rank_new, *contrib_new;
-  float d, base;
-  int l;
-  bool on;
+constexpr int kPprU = 8;      // in-edges of a step of the gather
+constexpr int kPprLong = 16;  // rows over more pieces are folded by a whole CTA
+
+// Eight CSC sources from edge e (a multiple of 8): one 32-byte load, the
+// same address in every thread of the group.
+__device__ __forceinline__ void ppr_src8(const PprArgs &a, int e, int end, int (&u)[kPprU]) {
+  const int n = end - e;  // (differences: e + 8 may not fit an int)
+  if (a.E - e >= kPprU) {
+    nc8(a.csc_src + e, u);
+  } else {
+#pragma unroll
+    for (int j = 0; j < kPprU; ++j) u[j] = j < n ? __ldg(a.csc_src + e + j) : -1;
+  }
+  if (n < kPprU) {
+#pragma unroll
+    for (int j = 0; j < kPprU; ++j)
+      if (j >= n) u[j] = -1;
+  }
+}
+
+// VL consecutive lanes of a row, one load or store.
+template <int VL>
+struct Lanes {
+  float f[VL];
 };
 
-__device__ __forceinline__ PprLane ppr_lane(const PprArgs &a) {
-  PprLane o;
-  const int p = a.cnt->iteration & 1;
-  o.contrib = a.contrib[p];
-  o.rank_old = a.rank[p];
-  o.rank_new = a.rank[p ^ 1];
-  o.contrib_new = a.contrib[p ^ 1];
-  o.d = (float)a.prm->damping;
-  o.base = (float)(1.0 - a.prm->damping);
-  o.l = threadIdx.x % a.G;
-  o.on = o.l < a.L;
+template <int VL>
+__device__ __forceinline__ Lanes<VL> ppr_ld(const float *p) {
+  Lanes<VL> o;
+  if constexpr (VL == 4) {
+    const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
+    o.f[0] = t.x; o.f[1] = t.y; o.f[2] = t.z; o.f[3] = t.w;
+  } else if constexpr (VL == 2) {
+    const float2 t = __ldg(reinterpret_cast<const float2 *>(p));
+    o.f[0] = t.x; o.f[1] = t.y;
+  } else {
+    o.f[0] = __ldg(p);
+  }
   return o;
 }
 
-__device__ __forceinline__ void ppr_finish_row(const PprArgs &a, const PprLane &t, int v,
-                                               CVal acc, double &l1) {
-  const float sum = __fadd_rn(acc.s, acc.c);
-  const float b = ((__ldg(a.seed_mask + v) >> t.l) & 1u) ? t.base : 0.f;
-  const float r = __fadd_rn(b, __fmul_rn(t.d, sum));
-  const int deg = __ldg(a.csr_off + v + 1) - __ldg(a.csr_off + v);
-  const size_t k = (size_t)v * a.L + t.l;
-  l1 += fabs((double)r - (double)t.rank_old[k]);
-  t.rank_new[k] = r;
-  t.contrib_new[k] = deg ? __fdiv_rn(r, (float)deg) : 0.f;
+template <int VL>
+__device__ __forceinline__ void ppr_st(float *p, const Lanes<VL> &v) {
+  if constexpr (VL == 4)
+    *reinterpret_cast<float4 *>(p) = make_float4(v.f[0], v.f[1], v.f[2], v.f[3]);
+  else if constexpr (VL == 2)
+    *reinterpret_cast<float2 *>(p) = make_float2(v.f[0], v.f[1]);
+  else
+    *p = v.f[0];
 }
 
-// Edge-order fold of one lane over [e, stop): groups of 8 contributions are
-// summed pairwise in FP32 (relative error <= 3 u of the group's sum, the
-// terms being non-negative), and the group sums are accumulated with two-sum
-// compensation, so the error of a row stays near 3 u of its value.
-__device__ __forceinline__ CVal ppr_fold(const PprArgs &a, const PprLane &t, int e, int stop) {
-  CVal acc{0.f, 0.f};
-  constexpr int U = 8;
-  for (; e + U <= stop; e += U) {
-    int u[U];
-    float x[U];
+template <int VL>
+__device__ __forceinline__ void ppr_contrib8(const PprArgs &a, const int (&u)[kPprU], int l,
+                                             Lanes<VL> (&x)[kPprU]) {
 #pragma unroll
-    for (int j = 0; j < U; ++j) u[j] = __ldg(a.csc_src + e + j);
+  for (int j = 0; j < kPprU; ++j) {
+    if (u[j] >= 0) {
+      x[j] = ppr_ld<VL>(a.contrib + (size_t)u[j] * a.L + l);
+    } else {
 #pragma unroll
-    for (int j = 0; j < U; ++j) x[j] = __ldg(t.contrib + (size_t)u[j] * a.L + t.l);
-    const float g = __fadd_rn(__fadd_rn(__fadd_rn(x[0], x[1]), __fadd_rn(x[2], x[3])),
-                              __fadd_rn(__fadd_rn(x[4], x[5]), __fadd_rn(x[6], x[7])));
-    acc = two_sum_add(acc, CVal{g, 0.f});
-  }
-  for (; e < stop; ++e) {
-    const int u = __ldg(a.csc_src + e);
-    acc = two_sum_add(acc, CVal{__ldg(t.contrib + (size_t)u * a.L + t.l), 0.f});
-  }
-  return acc;
-}
-
-// Per-lane block sums of l1 in a fixed order into out[lane].
-__device__ __forceinline__ void lane_block_sums(double l1, int G, double *out) {
-  __shared__ double s[kNT];
-  s[threadIdx.x] = l1;
-  __syncthreads();
-  if (threadIdx.x < G) {
-    double t = 0.0;
-    for (int j = threadIdx.x; j < kNT; j += G) t += s[j];
-    out[threadIdx.x] = t;
+      for (int q = 0; q < VL; ++q) x[j].f[q] = 0.f;
+    }
   }
 }
 
-__global__ void __launch_bounds__(kNT) k_ppr_pieces(PprArgs a, double *l1_part) {
-  const PprLane t = ppr_lane(a);
-  const int per_block = kNT / a.G;
-  const int local = threadIdx.x / a.G;
-  double l1 = 0.0;
-  if (t.on) {
-    for (int k = blockIdx.x * per_block + local; k < a.n_pieces; k += gridDim.x * per_block) {
-      int e = k * a.P;
-      const int end = min(a.E, e + a.P);
-      int r = __ldg(a.first_row + k);
-      int row_end = __ldg(a.csc_off + r + 1);
-      bool cont = __ldg(a.csc_off + r) < e;
-      for (;;) {
-        const int stop = min(row_end, end);
-        const CVal acc = ppr_fold(a, t, e, stop);
-        if (stop < row_end) {  // the piece ends inside row r
-          (cont ? a.head : a.tail)[(size_t)k * a.L + t.l] = acc;
-          break;
+// The gather: a group of G / VL threads (VL lanes each) walks a piece in
+// steps of 8 in-edges whatever the rows are, two steps' contribution rows,
+// two steps' sources and the next 32 row ends in flight; the row ends come
+// from a bit per edge.  A step inside one row is summed pairwise in FP32
+// (relative error <= 3 u of the step's sum, the terms being non-negative),
+// other steps term by term; both go into the row's sum by two-sum, so a
+// row's error stays near 3 u of its value.  Rows that end in the piece they
+// start in store their sum (by row, no dependent load); the others leave
+// partials for k_ppr_fix.  What follows a row's sum (rank, contribution,
+// residual) is k_ppr_rows', a streaming pass: done here, each row end
+// stalled the walk on four loads.
+template <int VL>
+__global__ void __launch_bounds__(kNT) k_ppr_pieces(PprArgs a) {
+  const int T = a.G / VL;
+  const int l = threadIdx.x % T * VL;
+  if (l >= a.L) return;
+  const int per_block = kNT / T;
+  for (int k = blockIdx.x * per_block + (int)threadIdx.x / T; k < a.n_pieces;
+       k += gridDim.x * per_block) {
+    const int e0 = k * a.P;
+    const int end = a.E - e0 < a.P ? a.E : e0 + a.P;
+    int r = __ldg(a.first_row + k);
+    bool cont = e0 > 0 && !((__ldg(a.row_bits + ((e0 - 1) >> 5)) >> ((e0 - 1) & 31)) & 1u);
+    uint32_t word = __ldg(a.row_bits + (e0 >> 5)), word2 = 0u;
+    if (((end - 1) >> 5) > (e0 >> 5)) word2 = __ldg(a.row_bits + (e0 >> 5) + 1);
+    int u[kPprU], u2[kPprU];
+    Lanes<VL> x[kPprU], y[kPprU];
+    ppr_src8(a, e0, end, u);
+    if (end - e0 > kPprU) ppr_src8(a, e0 + kPprU, end, u2);
+    ppr_contrib8<VL>(a, u, l, x);
+    CVal acc[VL];
+#pragma unroll
+    for (int q = 0; q < VL; ++q) acc[q] = CVal{0.f, 0.f};
+    bool open = true;  // the piece's last edge does not end its row
+    for (int e = e0;; e += kPprU) {
+      const uint32_t ends = (word >> (e & 31)) & 0xFFu;
+      const bool more = end - e > kPprU;
+      if (more) {
+#pragma unroll
+        for (int j = 0; j < kPprU; ++j) u[j] = u2[j];
+        if (end - e > 2 * kPprU) ppr_src8(a, e + 2 * kPprU, end, u2);
+        ppr_contrib8<VL>(a, u, l, y);
+        if ((e & 31) == 32 - kPprU) {
+          word = word2;
+          if (((end - 1) >> 5) > ((e + kPprU) >> 5))
+            word2 = __ldg(a.row_bits + ((e + kPprU) >> 5) + 1);
         }
-        if (cont)
-          a.head[(size_t)k * a.L + t.l] = acc;
-        else
-          ppr_finish_row(a, t, r, acc, l1);
-        if (stop == end) break;
-        do {  // next row with in-edges (one exists: stop < end <= E)
-          ++r;
-          row_end = __ldg(a.csc_off + r + 1);
-        } while (row_end == stop);
-        cont = false;
-        e = stop;
       }
+      if (!ends) {
+#pragma unroll
+        for (int q = 0; q < VL; ++q) {
+          const float g = __fadd_rn(
+              __fadd_rn(__fadd_rn(x[0].f[q], x[1].f[q]), __fadd_rn(x[2].f[q], x[3].f[q])),
+              __fadd_rn(__fadd_rn(x[4].f[q], x[5].f[q]), __fadd_rn(x[6].f[q], x[7].f[q])));
+          acc[q] = two_sum_add(acc[q], CVal{g, 0.f});
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < kPprU; ++j) {
+#pragma unroll
+          for (int q = 0; q < VL; ++q) acc[q] = two_sum_add(acc[q], CVal{x[j].f[q], 0.f});
+          if ((ends >> j) & 1u) {
+            if (cont) {
+#pragma unroll
+              for (int q = 0; q < VL; ++q) a.head[(size_t)k * a.L + l + q] = acc[q];
+            } else {
+              Lanes<VL> o;
+#pragma unroll
+              for (int q = 0; q < VL; ++q) o.f[q] = __fadd_rn(acc[q].s, acc[q].c);
+              ppr_st<VL>(a.sum + (size_t)r * a.L + l, o);
+            }
+            cont = false;
+            ++r;
+#pragma unroll
+            for (int q = 0; q < VL; ++q) acc[q] = CVal{0.f, 0.f};
+          }
+        }
+      }
+      if (!more) {
+        open = !((ends >> (end - 1 - e)) & 1u);
+        break;
+      }
+#pragma unroll
+      for (int j = 0; j < kPprU; ++j) x[j] = y[j];
+    }
+    if (open) {
+      CVal *to = (cont ? a.head : a.tail) + (size_t)k * a.L + l;
+#pragma unroll
+      for (int q = 0; q < VL; ++q) to[q] = acc[q];
     }
   }
-  lane_block_sums(l1, a.G, l1_part + (size_t)blockIdx.x * a.G);
 }
 
-// Rows cut by piece boundaries (partials folded in piece order), and in the
-// first iteration the rows without in-edges (first piece -1): their rank is
-// (1-d) [seed] from then on, so it is written into both buffers once and
-// those rows are skipped afterwards.
-__global__ void __launch_bounds__(kNT) k_ppr_fix(PprArgs a, double *l1_part) {
-  const PprLane t = ppr_lane(a);
-  const int per_block = kNT / a.G;
-  const int local = threadIdx.x / a.G;
-  const bool first = a.cnt->iteration == 0;
-  const int limit = first ? a.n_fix : a.n_split;
-  double l1 = 0.0;
-  if (t.on) {
-    for (int i = blockIdx.x * per_block + local; i < limit; i += gridDim.x * per_block) {
-      const int v = a.fix[3 * i], ps = a.fix[3 * i + 1], pe = a.fix[3 * i + 2];
-      CVal acc{0.f, 0.f};
-      if (ps >= 0) {
-        acc = a.tail[(size_t)ps * a.L + t.l];
-        for (int k = ps + 1; k <= pe; ++k) acc = two_sum_add(acc, a.head[(size_t)k * a.L + t.l]);
-      }
-      ppr_finish_row(a, t, v, acc, l1);
-      if (ps < 0) {  // first iteration only: the other buffer too (the
-                     // pieces of this iteration have read it already)
-        const size_t k = (size_t)v * a.L + t.l;
-        a.rank[0][k] = t.rank_new[k];
-        a.contrib[0][k] = t.contrib_new[k];
+// VL lanes' partials, 16 bytes at a time.
+template <int VL>
+struct Partials {
+  CVal p[VL];
+};
+
+template <int VL>
+__device__ __forceinline__ Partials<VL> ppr_partials(const CVal *p) {
+  Partials<VL> o;
+  if constexpr (VL >= 2) {
+#pragma unroll
+    for (int q = 0; q < VL; q += 2) {
+      const float4 t = *reinterpret_cast<const float4 *>(p + q);
+      o.p[q] = CVal{t.x, t.y};
+      o.p[q + 1] = CVal{t.z, t.w};
+    }
+  } else {
+    o.p[0] = *p;
+  }
+  return o;
+}
+
+// Rows cut by piece boundaries, their partials folded in a fixed order: a
+// group per row, or the whole CTA (every group a strided share, then the
+// groups' sums) for rows over more than kPprLong pieces -- one group folding
+// a hub's 1,200 partials one after the other took 90 us.  Nearly every piece
+// cuts a row and nearly every cut row ends in the next piece, so its two
+// partials are loaded with the row's number, not after it.
+template <int VL>
+__global__ void __launch_bounds__(kNT) k_ppr_fix(PprArgs a) {
+  __shared__ Partials<VL> s_part[kNT];
+  __shared__ int s_last[kNT];
+  const int T = a.G / VL;
+  const int l = threadIdx.x % T * VL, g = threadIdx.x / T, groups = kNT / T;
+  const bool on = l < a.L;
+  for (int k0 = blockIdx.x * groups; k0 < a.n_pieces; k0 += gridDim.x * groups) {
+    const int k = k0 + g;
+    int r = -1, last = -1;
+    Partials<VL> acc, next;
+    if (k < a.n_pieces) {
+      r = __ldg(a.split_row + k);
+      last = __ldg(a.split_last + k);
+      if (on) {
+        acc = ppr_partials<VL>(a.tail + (size_t)k * a.L + l);
+        next = ppr_partials<VL>(a.head + (size_t)min(k + 1, a.n_pieces - 1) * a.L + l);
       }
     }
+    const bool lng = r >= 0 && last - k > kPprLong;
+    if (r >= 0 && !lng && on) {
+      for (int q = k + 1;; ++q) {
+#pragma unroll
+        for (int i = 0; i < VL; ++i) acc.p[i] = two_sum_add(acc.p[i], next.p[i]);
+        if (q == last) break;
+        next = ppr_partials<VL>(a.head + (size_t)(q + 1) * a.L + l);
+      }
+      Lanes<VL> o;
+#pragma unroll
+      for (int i = 0; i < VL; ++i) o.f[i] = __fadd_rn(acc.p[i].s, acc.p[i].c);
+      ppr_st<VL>(a.sum + (size_t)r * a.L + l, o);
+    }
+    if (!__syncthreads_or(lng)) continue;  // CTA-uniform
+    if (l == 0) s_last[g] = lng ? last : -1;
+    __syncthreads();
+    for (int h = 0; h < groups; ++h) {
+      const int hl = s_last[h];
+      if (hl < 0) continue;  // CTA-uniform
+      const int kh = k0 + h;
+#pragma unroll
+      for (int i = 0; i < VL; ++i) acc.p[i] = CVal{0.f, 0.f};
+      if (on)
+#pragma unroll 4
+        for (int q = kh + 1 + g; q <= hl; q += groups) {
+          next = ppr_partials<VL>(a.head + (size_t)q * a.L + l);
+#pragma unroll
+          for (int i = 0; i < VL; ++i) acc.p[i] = two_sum_add(acc.p[i], next.p[i]);
+        }
+      s_part[threadIdx.x] = acc;
+      __syncthreads();
+      for (int w = groups >> 1; w > 0; w >>= 1) {
+        if (g < w) {
+#pragma unroll
+          for (int i = 0; i < VL; ++i)
+            s_part[threadIdx.x].p[i] =
+                two_sum_add(s_part[threadIdx.x].p[i], s_part[threadIdx.x + w * T].p[i]);
+        }
+        __syncthreads();
+      }
+      if (g == 0 && on) {
+        const Partials<VL> t = ppr_partials<VL>(a.tail + (size_t)kh * a.L + l);
+        Lanes<VL> o;
+#pragma unroll
+        for (int i = 0; i < VL; ++i) {
+          const CVal c = two_sum_add(t.p[i], s_part[threadIdx.x].p[i]);
+          o.f[i] = __fadd_rn(c.s, c.c);
+        }
+        ppr_st<VL>(a.sum + (size_t)__ldg(a.split_row + kh) * a.L + l, o);
+      }
+      __syncthreads();
+    }
   }
-  lane_block_sums(l1, a.G, l1_part + (size_t)blockIdx.x * a.G);
 }
 
-// Per-lane residuals (fixed-order sums over the blocks); the loop goes on
-// while the largest is above tol.
+// A row's inputs, loaded before any is used; then its new rank and
+// contribution from its sum, and its L1 step.
+template <int VL>
+struct PprRow {
+  int v, deg;
+  uint32_t seed;
+  Lanes<VL> sum, old;
+};
+
+template <int VL>
+__device__ __forceinline__ void ppr_row_load(const PprArgs &a, int l, PprRow<VL> &w) {
+  w.seed = __ldg(a.seed_mask + w.v);
+  w.deg = __ldg(a.csr_off + w.v + 1) - __ldg(a.csr_off + w.v);
+  const float *o = a.rank + (size_t)w.v * a.L + l;
+  if constexpr (VL == 4) {
+    const float4 t = *reinterpret_cast<const float4 *>(o);
+    w.old.f[0] = t.x; w.old.f[1] = t.y; w.old.f[2] = t.z; w.old.f[3] = t.w;
+  } else {
+#pragma unroll
+    for (int q = 0; q < VL; ++q) w.old.f[q] = o[q];
+  }
+}
+
+// The L1 step is kept without FP64 (two conversions and two additions per
+// rank took three quarters of this kernel's time at GB300's FP64 rate):
+// new - old = s + c exactly (two-sum), and |new - old| joins the thread's
+// sum by two-sum, so its error is of second order in 2^-24.
+template <int VL>
+__device__ __forceinline__ void ppr_row_finish(const PprArgs &a, int l, const PprRow<VL> &w,
+                                               float d, float base, CVal (&l1)[VL]) {
+  Lanes<VL> rank, contrib;
+#pragma unroll
+  for (int q = 0; q < VL; ++q) {
+    const float b = ((w.seed >> (l + q)) & 1u) ? base : 0.f;
+    const float r = __fadd_rn(b, __fmul_rn(d, w.sum.f[q]));
+    const CVal step = two_sum_add(CVal{r, 0.f}, CVal{-w.old.f[q], 0.f});
+    l1[q] = two_sum_add(l1[q], step.s < 0.f ? CVal{-step.s, -step.c} : step);
+    rank.f[q] = r;
+    contrib.f[q] = w.deg ? __fdiv_rn(r, (float)w.deg) : 0.f;
+  }
+  ppr_st<VL>(a.rank + (size_t)w.v * a.L + l, rank);
+  ppr_st<VL>(a.contrib + (size_t)w.v * a.L + l, contrib);
+}
+
+// Ranks, contributions and residual of every row with in-edges; in the first
+// iteration also of those without (their rank is (1-d) [seed] from then on,
+// so they are skipped afterwards).  Bound by memory: four arrays of [V][L]
+// floats streamed, two rows per group in flight.  The last block done adds
+// the blocks' residuals up, in a fixed order, and sets the loop condition:
+// on while the largest lane's is above tol.
+template <int VL>
 __global__ void __launch_bounds__(kNT)
-    k_ppr_finish(const double *l1_part, int nblocks, int G, int L, const BatchParams *prm,
-                 gas_counters *cnt, double *lane_resid, cudaGraphConditionalHandle h,
-                 int in_graph) {
-  __shared__ double s[kNT];
-  const int l = threadIdx.x % G, j = threadIdx.x / G, nj = kNT / G;
+    k_ppr_rows(PprArgs a, cudaGraphConditionalHandle h, int in_graph) {
+  const int T = a.G / VL;
+  const int l = threadIdx.x % T * VL, grp = threadIdx.x / T, per_block = kNT / T;
+  const float d = (float)a.prm->damping, base = (float)(1.0 - a.prm->damping);
+  const bool first = a.cnt->iteration == 0;
+  CVal l1[VL];
+#pragma unroll
+  for (int q = 0; q < VL; ++q) l1[q] = CVal{0.f, 0.f};
+  if (l < a.L) {
+    const int stride = gridDim.x * per_block;
+    int i = blockIdx.x * per_block + grp;
+    for (; i < a.n_ne - stride; i += 2 * stride) {  // (n_ne + stride may not fit an int)
+      PprRow<VL> w[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        w[k].v = __ldg(a.ne_vid + i + k * stride);
+        w[k].sum = ppr_ld<VL>(a.sum + (size_t)(i + k * stride) * a.L + l);
+      }
+#pragma unroll
+      for (int k = 0; k < 2; ++k) ppr_row_load<VL>(a, l, w[k]);
+#pragma unroll
+      for (int k = 0; k < 2; ++k) ppr_row_finish<VL>(a, l, w[k], d, base, l1);
+    }
+    if (i < a.n_ne) {
+      PprRow<VL> w;
+      w.v = __ldg(a.ne_vid + i);
+      w.sum = ppr_ld<VL>(a.sum + (size_t)i * a.L + l);
+      ppr_row_load<VL>(a, l, w);
+      ppr_row_finish<VL>(a, l, w, d, base, l1);
+    }
+    if (first)
+      for (int v = blockIdx.x * per_block + grp; v < a.nV; v += stride)
+        if (__ldg(a.csc_off + v) == __ldg(a.csc_off + v + 1)) {
+          PprRow<VL> w;
+          w.v = v;
+#pragma unroll
+          for (int q = 0; q < VL; ++q) w.sum.f[q] = 0.f;
+          ppr_row_load<VL>(a, l, w);
+          ppr_row_finish<VL>(a, l, w, d, base, l1);
+        }
+  }
+  // per-lane block sums in a fixed order
+  __shared__ double s[kNT * VL];
+#pragma unroll
+  for (int q = 0; q < VL; ++q) s[grp * a.G + l + q] = (double)l1[q].s + (double)l1[q].c;
+  __syncthreads();
+  if (threadIdx.x < a.G) {
+    double t = 0.0;
+    for (int j = threadIdx.x; j < kNT * VL; j += a.G) t += s[j];
+    a.l1_part[(size_t)blockIdx.x * a.G + threadIdx.x] = t;
+  }
+  const int g = threadIdx.x / a.G, groups = kNT / a.G;
+  __shared__ bool s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
   double v = 0.0;
-  for (int b = j; b < nblocks; b += nj) v += l1_part[(size_t)b * G + l];
+#pragma unroll 8
+  for (int b = g; b < (int)gridDim.x; b += groups)
+    v += __ldcg(a.l1_part + (size_t)b * a.G + threadIdx.x % a.G);
   s[threadIdx.x] = v;
   __syncthreads();
   double t = 0.0;
-  if (threadIdx.x < G)
-    for (int q = 0; q < nj; ++q) t += s[q * G + threadIdx.x];
+  if (threadIdx.x < a.G)
+    for (int q = 0; q < groups; ++q) t += s[q * a.G + threadIdx.x];
   __syncthreads();
-  if (threadIdx.x < G) s[threadIdx.x] = t;
+  if (threadIdx.x < a.G) s[threadIdx.x] = t;
   __syncthreads();
   if (threadIdx.x == 0) {
     double mx = 0.0;
-    for (int q = 0; q < L; ++q) {
-      lane_resid[1 + q] = s[q];
+    for (int q = 0; q < a.L; ++q) {
+      a.lane_resid[1 + q] = s[q];
       mx = s[q] > mx ? s[q] : mx;
     }
-    lane_resid[0] = mx;
-    const int it = ++cnt->iteration;
-    set_cond(cnt, !(mx <= prm->tol), it, h, in_graph);
+    a.lane_resid[0] = mx;
+    *a.ticket = 0u;
+    const int it = ++a.cnt->iteration;
+    set_cond(a.cnt, !(mx <= a.prm->tol), it, h, in_graph);
   }
+}
+
+// The plan, once per piece size: a bit at every row's last in-edge ...
+__global__ void k_ppr_row_bits(const int32_t *ne_end, int n_ne, uint32_t *bits) {
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n_ne; r += gridDim.x * blockDim.x) {
+    const int e = ne_end[r] - 1;
+    atomicOr(bits + (e >> 5), 1u << (e & 31));
+  }
+}
+
+// The row of in-edge e: the first whose end is past it.
+__device__ __forceinline__ int ppr_row_of(const int32_t *ne_end, int n_ne, int e) {
+  int lo = 0, hi = n_ne;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (ne_end[mid] <= e)
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  return lo;
+}
+
+// ... and the pieces' first rows and the rows they cut.
+__global__ void k_ppr_plan(const int32_t *ne_end, int n_ne, int n_pieces, int P, int E,
+                           int32_t *first_row, int32_t *split_row, int32_t *split_last) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n_pieces;
+       k += gridDim.x * blockDim.x) {
+    const int e0 = k * P;
+    const int end = E - e0 < P ? E : e0 + P;
+    first_row[k] = ppr_row_of(ne_end, n_ne, e0);
+    const int r = ppr_row_of(ne_end, n_ne, end - 1);
+    const int row_start = r > 0 ? ne_end[r - 1] : 0, row_end = ne_end[r];
+    const bool cut = row_start >= e0 && row_end > end;
+    split_row[k] = cut ? r : -1;
+    split_last[k] = cut ? (row_end - 1) / P : -1;
+  }
+}
+
+// Each (graph, lane) seed's bit.
+__global__ void k_ppr_seed(const int32_t *seeds, const BatchParams *prm, int L,
+                           uint32_t *seed_mask) {
+  const int n = prm->n_seeds;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    if (seeds[i] >= 0) atomicOr(seed_mask + seeds[i], 1u << (i % L));
 }
 
 // r0 = e_seed per lane; contributions accordingly.
@@ -895,9 +1178,13 @@ __global__ void k_ppr_init(const uint32_t *seed_mask, const int32_t *csr_off, in
        k += (size_t)gridDim.x * blockDim.x) {
     const int v = (int)(k / L), l = (int)(k % L);
     const float r = ((seed_mask[v] >> l) & 1u) ? 1.f : 0.f;
-    const int deg = csr_off[v + 1] - csr_off[v];
+    float c = 0.f;
+    if (r != 0.f) {
+      const int deg = csr_off[v + 1] - csr_off[v];
+      c = deg ? __fdiv_rn(r, (float)deg) : 0.f;
+    }
     rank[k] = r;
-    contrib[k] = deg ? __fdiv_rn(r, (float)deg) : 0.f;
+    contrib[k] = c;
   }
 }
 
@@ -938,12 +1225,14 @@ struct gas_batch {
   cudaEvent_t pev[2] = {nullptr, nullptr};
   gas_kernel_profile prof{};
   // PPR
-  int32_t *first_row = nullptr, *fix = nullptr;
+  int32_t *first_row = nullptr, *split_row = nullptr, *split_last = nullptr;
   CVal *head = nullptr, *tail = nullptr;
-  float *rank[2] = {nullptr, nullptr}, *contrib[2] = {nullptr, nullptr};
-  uint32_t *seed_mask = nullptr;
+  float *rank = nullptr, *contrib = nullptr, *sum = nullptr;
+  uint32_t *seed_mask = nullptr, *row_bits = nullptr;
+  int32_t *seeds = nullptr;
   double *l1 = nullptr;
-  int32_t n_pieces = 0, n_fix = 0, n_split = 0, piece_edges = 0, ppr_lanes = 0, l1_cap = 0;
+  unsigned int *ticket = nullptr;
+  int32_t n_pieces = 0, piece_edges = 0, ppr_lanes = 0, l1_cap = 0, seeds_cap = 0;
   int32_t tuned_piece = 0;
   // cached graph
   cudaGraphExec_t graph = nullptr;
@@ -969,15 +1258,23 @@ void free_state(gas_batch *b) {
   bfree(b->vn); bfree(b->next); bfree(b->tbits); bfree(b->depth);
   bfree(b->q_mask); bfree(b->q_end); bfree(b->q_delta);
   bfree(b->part); bfree(b->qpart); bfree(b->srcs);
-  bfree(b->first_row); bfree(b->fix); bfree(b->head); bfree(b->tail);
-  bfree(b->seed_mask); bfree(b->l1);
+  bfree(b->first_row); bfree(b->split_row); bfree(b->split_last);
+  bfree(b->head); bfree(b->tail); bfree(b->row_bits);
+  bfree(b->seed_mask); bfree(b->seeds); bfree(b->l1); bfree(b->ticket);
   bfree(b->dist); bfree(b->q_vals); bfree(b->sssp_srcs); bfree(b->lane_rounds);
   bfree(b->lanes_active);
   b->dist_ls = b->sssp_srcs_cap = 0;
-  for (int i = 0; i < 2; ++i) { bfree(b->rank[i]); bfree(b->contrib[i]); }
-  b->n_pieces = b->n_fix = b->n_split = b->piece_edges = b->ppr_lanes = b->depth_lanes = 0;
-  b->srcs_cap = b->l1_cap = 0;
+  bfree(b->rank); bfree(b->contrib); bfree(b->sum);
+  b->n_pieces = b->piece_edges = b->ppr_lanes = b->depth_lanes = 0;
+  b->srcs_cap = b->l1_cap = b->seeds_cap = 0;
 }
+
+// Lanes per thread of the PPR kernels (four: 16-byte loads).  A walk of 8
+// pieces per warp beats one of 2 although their row ends diverge: 16 graphs,
+// 16 lanes 16.9 ms per run with 4 lanes a thread, 17.8 with 2, 22.7 with 1;
+// 4 lanes 2.53 / 2.75 / 2.92.  Two lanes go one to a thread (2.25 ms against
+// 2.49).
+int ppr_vl(int L) { return L % 4 == 0 ? 4 : L % 2 == 0 && L > 2 ? 2 : 1; }
 
 int lane_group(int L) {
   int g = 1;
@@ -1059,68 +1356,74 @@ gas_status_t ensure_bfs(gas_batch *b, int lanes, int n_sources) {
   return GAS_OK;
 }
 
-// Pieces of P edges over the CSC, their first rows, and the rows the second
-// pass finishes (cut rows and rows without in-edges).
-gas_status_t ensure_ppr(gas_batch *b, int lanes, int P, int grid_pieces, int grid_fix) {
+// Ranks, contributions and row sums of the lanes; pieces of P edges over the
+// CSC (P rounded up to whole steps of the gather), their first rows and the
+// rows they cut.
+gas_status_t ensure_ppr(gas_batch *b, int lanes, int P, int n_seeds, int grid_rows,
+                        cudaStream_t s) {
   gas_engine *e = b->eng;
-  const size_t nV = std::max(1, e->nV);
+  const size_t nV = std::max(1, e->nV), n_ne = std::max(1, e->n_ne);
+  const size_t nE = std::max(1, e->nE);
   if (b->ppr_lanes != lanes) {
     drop_graph(b);
-    for (int i = 0; i < 2; ++i) { bfree(b->rank[i]); bfree(b->contrib[i]); }
-    for (int i = 0; i < 2; ++i) {
-      CUDA_TRY(cudaMalloc(&b->rank[i], nV * lanes * 4));
-      CUDA_TRY(cudaMalloc(&b->contrib[i], nV * lanes * 4));
-    }
+    bfree(b->rank);
+    bfree(b->contrib);
+    bfree(b->sum);
+    b->ppr_lanes = 0;
+    CUDA_TRY(cudaMalloc(&b->rank, nV * lanes * 4));
+    CUDA_TRY(cudaMalloc(&b->contrib, nV * lanes * 4));
+    CUDA_TRY(cudaMalloc(&b->sum, n_ne * lanes * 4));
     b->ppr_lanes = lanes;
     b->piece_edges = 0;  // head/tail are sized by lanes
   }
   if (!b->seed_mask) CUDA_TRY(cudaMalloc(&b->seed_mask, nV * 4));
+  if (!b->ticket) {
+    CUDA_TRY(cudaMalloc(&b->ticket, 4));
+    CUDA_TRY(cudaMemsetAsync(b->ticket, 0, 4, s));
+  }
+  if (b->seeds_cap < n_seeds) {
+    drop_graph(b);
+    bfree(b->seeds);
+    b->seeds_cap = 0;
+    CUDA_TRY(cudaMalloc(&b->seeds, (size_t)n_seeds * 4));
+    b->seeds_cap = n_seeds;
+  }
   const int G = lane_group(lanes);
-  const int need_l1 = (grid_pieces + grid_fix) * G;
+  const int need_l1 = grid_rows * G;
   if (b->l1_cap < need_l1) {
     drop_graph(b);
     bfree(b->l1);
+    b->l1_cap = 0;
     CUDA_TRY(cudaMalloc(&b->l1, (size_t)need_l1 * sizeof(double)));
     b->l1_cap = need_l1;
   }
+  if (!b->row_bits) {
+    const size_t words = (nE + 31) / 32;
+    CUDA_TRY(cudaMalloc(&b->row_bits, words * 4));
+    CUDA_TRY(cudaMemsetAsync(b->row_bits, 0, words * 4, s));
+    k_ppr_row_bits<<<8 * e->num_sms, 256, 0, s>>>(e->ne_end, e->n_ne, b->row_bits);
+    CUDA_TRY(cudaGetLastError());
+  }
   if (b->piece_edges == P) return GAS_OK;
   drop_graph(b);
-  const std::vector<int32_t> &off = e->h_csc_off;
-  const int32_t E = e->nE, V = e->nV;
-  const int32_t n_pieces = (int32_t)(((int64_t)E + P - 1) / P);
-  std::vector<int32_t> first((size_t)std::max(1, n_pieces));
-  for (int32_t k = 0, r = 0; k < n_pieces; ++k) {
-    const int64_t e0 = (int64_t)k * P;
-    while (off[r + 1] <= e0) ++r;  // first row with csc_off[r+1] > e0
-    first[k] = r;
-  }
-  std::vector<int32_t> fix, zero;
-  for (int32_t v = 0; v < V; ++v) {
-    const int32_t lo = off[v], hi = off[v + 1];
-    if (lo == hi) {
-      zero.insert(zero.end(), {v, -1, -1});
-    } else {
-      const int32_t ps = lo / P, pe = (hi - 1) / P;
-      if (ps != pe) fix.insert(fix.end(), {v, ps, pe});
-    }
-  }
-  const int32_t n_split = (int32_t)(fix.size() / 3);
-  fix.insert(fix.end(), zero.begin(), zero.end());
+  b->piece_edges = 0;
+  const int Pu = (P + kPprU - 1) / kPprU * kPprU;
+  const int32_t n_pieces = (int32_t)(((int64_t)e->nE + Pu - 1) / Pu);
+  const size_t np = std::max(1, n_pieces);
   bfree(b->first_row);
-  bfree(b->fix);
+  bfree(b->split_row);
+  bfree(b->split_last);
   bfree(b->head);
   bfree(b->tail);
-  CUDA_TRY(cudaMalloc(&b->first_row, first.size() * 4));
-  CUDA_TRY(cudaMalloc(&b->fix, std::max<size_t>(1, fix.size()) * 4));
-  const size_t hp = std::max<size_t>(1, (size_t)n_pieces * lanes) * sizeof(CVal);
-  CUDA_TRY(cudaMalloc(&b->head, hp));
-  CUDA_TRY(cudaMalloc(&b->tail, hp));
-  CUDA_TRY(cudaMemcpy(b->first_row, first.data(), first.size() * 4, cudaMemcpyHostToDevice));
-  if (!fix.empty())
-    CUDA_TRY(cudaMemcpy(b->fix, fix.data(), fix.size() * 4, cudaMemcpyHostToDevice));
+  for (int32_t **p : {&b->first_row, &b->split_row, &b->split_last})
+    CUDA_TRY(cudaMalloc(p, np * 4));
+  CUDA_TRY(cudaMalloc(&b->head, np * lanes * sizeof(CVal)));
+  CUDA_TRY(cudaMalloc(&b->tail, np * lanes * sizeof(CVal)));
+  k_ppr_plan<<<8 * e->num_sms, 256, 0, s>>>(e->ne_end, e->n_ne, n_pieces, Pu, e->nE,
+                                           b->first_row, b->split_row, b->split_last);
+  CUDA_TRY(cudaGetLastError());
+  CUDA_TRY(cudaStreamSynchronize(s));  // the plan outlives this call and its stream
   b->n_pieces = n_pieces;
-  b->n_fix = (int32_t)(fix.size() / 3);
-  b->n_split = n_split;
   b->piece_edges = P;
   return GAS_OK;
 }
@@ -1128,31 +1431,37 @@ gas_status_t ensure_ppr(gas_batch *b, int lanes, int P, int grid_pieces, int gri
 struct RunCtx {
   gas_batch *b;
   int bfs_lanes, ppr_lanes, sssp_lanes;
-  int slab_grid, grid_pieces, grid_fix, sssp_grid;
+  int slab_grid, grid_pieces, grid_fix, grid_rows, sssp_grid;
   PprArgs ppr;
 };
 
 PprArgs ppr_args(gas_batch *b, int lanes) {
   gas_engine *e = b->eng;
   PprArgs a;
-  a.csc_off = e->csc_off;
   a.csc_src = e->csc_src;
+  a.csc_off = e->csc_off;
   a.csr_off = e->csr_off;
+  a.ne_vid = e->ne_vid;
+  a.ne_end = e->ne_end;
+  a.row_bits = b->row_bits;
   a.first_row = b->first_row;
+  a.split_row = b->split_row;
+  a.split_last = b->split_last;
   a.n_pieces = b->n_pieces;
-  a.P = b->piece_edges;
+  a.P = (b->piece_edges + kPprU - 1) / kPprU * kPprU;
   a.E = e->nE;
   a.L = lanes;
   a.G = lane_group(lanes);
-  a.fix = b->fix;
-  a.n_fix = b->n_fix;
-  a.n_split = b->n_split;
+  a.n_ne = e->n_ne;
+  a.nV = e->nV;
   a.head = b->head;
   a.tail = b->tail;
-  for (int i = 0; i < 2; ++i) {
-    a.rank[i] = b->rank[i];
-    a.contrib[i] = b->contrib[i];
-  }
+  a.sum = b->sum;
+  a.rank = b->rank;
+  a.contrib = b->contrib;
+  a.l1_part = b->l1;
+  a.lane_resid = b->resid;
+  a.ticket = b->ticket;
   a.seed_mask = b->seed_mask;
   a.prm = b->prm;
   a.cnt = b->cnt + 1;
@@ -1311,22 +1620,30 @@ gas_status_t ppr_prologue(RunCtx *c, cudaStream_t s, cudaGraphConditionalHandle 
   gas_batch *b = c->b;
   gas_engine *e = b->eng;
   k_b_reset<<<1, 1, 0, s>>>(b->cnt + 1, b->prm, 1, nullptr);
+  CUDA_TRY(cudaMemsetAsync(b->seed_mask, 0, (size_t)std::max(1, e->nV) * 4, s));
+  k_ppr_seed<<<2 * e->num_sms, 256, 0, s>>>(b->seeds, b->prm, c->ppr_lanes, b->seed_mask);
   k_ppr_init<<<8 * e->num_sms, 256, 0, s>>>(b->seed_mask, e->csr_off, e->nV, c->ppr_lanes,
-                                           b->rank[0], b->contrib[0]);
+                                           b->rank, b->contrib);
   k_ppr_precond<<<1, 1, 0, s>>>(b->cnt + 1, h, ig);
   CUDA_TRY(cudaGetLastError());
   return GAS_OK;
 }
 
-gas_status_t ppr_body(RunCtx *c, cudaStream_t s, cudaGraphConditionalHandle h, int ig) {
-  gas_batch *b = c->b;
-  const int G = c->ppr.G;
-  k_ppr_pieces<<<c->grid_pieces, kNT, 0, s>>>(c->ppr, b->l1);
-  k_ppr_fix<<<c->grid_fix, kNT, 0, s>>>(c->ppr, b->l1 + (size_t)c->grid_pieces * G);
-  k_ppr_finish<<<1, kNT, 0, s>>>(b->l1, c->grid_pieces + c->grid_fix, G, c->ppr_lanes,
-                                 b->prm, b->cnt + 1, b->resid, h, ig);
+template <int VL>
+gas_status_t ppr_step(RunCtx *c, cudaStream_t s, cudaGraphConditionalHandle h, int ig) {
+  k_ppr_pieces<VL><<<c->grid_pieces, kNT, 0, s>>>(c->ppr);
+  k_ppr_fix<VL><<<c->grid_fix, kNT, 0, s>>>(c->ppr);
+  k_ppr_rows<VL><<<c->grid_rows, kNT, 0, s>>>(c->ppr, h, ig);
   CUDA_TRY(cudaGetLastError());
   return GAS_OK;
+}
+
+gas_status_t ppr_body(RunCtx *c, cudaStream_t s, cudaGraphConditionalHandle h, int ig) {
+  switch (ppr_vl(c->ppr_lanes)) {
+    case 4: return ppr_step<4>(c, s, h, ig);
+    case 2: return ppr_step<2>(c, s, h, ig);
+    default: return ppr_step<1>(c, s, h, ig);
+  }
 }
 
 struct Loop {
@@ -1421,15 +1738,30 @@ gas_status_t run_direct(RunCtx *c, const Loop *loops, const int *which, int n, c
   return GAS_OK;
 }
 
+// Resident CTAs of the PPR kernels.
+template <int VL>
+void ppr_grids(const gas_engine *e, RunCtx *c) {
+  int per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ppr_pieces<VL>, kNT, 0);
+  c->grid_pieces = e->num_sms * (per_sm > 0 ? per_sm : 1);
+  per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ppr_fix<VL>, kNT, 0);
+  c->grid_fix = e->num_sms * (per_sm > 0 ? per_sm : 1);
+  per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ppr_rows<VL>, kNT, 0);
+  c->grid_rows = e->num_sms * (per_sm > 0 ? per_sm : 1);
+}
+
 void grids(gas_batch *b, RunCtx *c) {
   gas_engine *e = b->eng;
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ms_push, kNT, 0);
   c->slab_grid = e->num_sms * (per_sm > 0 ? per_sm : 1);
-  per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ppr_pieces, kNT, 0);
-  c->grid_pieces = e->num_sms * (per_sm > 0 ? per_sm : 1);
-  c->grid_fix = 8 * e->num_sms;
+  switch (ppr_vl(c->ppr_lanes)) {
+    case 4: ppr_grids<4>(e, c); break;
+    case 2: ppr_grids<2>(e, c); break;
+    default: ppr_grids<1>(e, c); break;
+  }
   per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mss_push<MssPushPolStaged<2>>, kNT,
                                                 0);
@@ -1468,7 +1800,17 @@ gas_status_t check_job(const gas_batch *b, const gas_batch_job *j) {
   return GAS_OK;
 }
 
-int default_piece(const gas_batch *b) { return b->tuned_piece > 0 ? b->tuned_piece : 256; }
+// Untuned piece size: 256, halved down to 64 while there would be fewer than
+// 1.5 pieces per resident group (16 lanes on 600 K edges: 64 takes 0.87 ms
+// per run, 256 1.37; on 64 M edges 19.4 and 16.9).
+int default_piece(const gas_batch *b, const RunCtx &c) {
+  if (b->tuned_piece > 0) return b->tuned_piece;
+  const int L = std::max(1, c.ppr_lanes);
+  const int64_t groups = (int64_t)c.grid_pieces * (kNT / (lane_group(L) / ppr_vl(L)));
+  int P = 256;
+  while (P > 64 && (int64_t)b->eng->nE / P * 2 < groups * 3) P /= 2;
+  return P;
+}
 
 }  // namespace
 
@@ -1610,7 +1952,7 @@ gas_status_t gas_batch_run(gas_batch *b, const gas_batch_job *job, int32_t *dept
   c.ppr_lanes = LP;
   c.sssp_lanes = LS;
   grids(b, &c);
-  const int P = job->piece_edges > 0 ? job->piece_edges : default_piece(b);
+  const int P = job->piece_edges > 0 ? job->piece_edges : default_piece(b, c);
   BatchParams prm{};
   prm.damping = LP ? job->damping : 0.85;
   prm.tol = LP ? job->tol : 1.0;
@@ -1619,6 +1961,7 @@ gas_status_t gas_batch_run(gas_batch *b, const gas_batch_job *job, int32_t *dept
   prm.n_sources = G * LB;
   prm.sssp_max_iter = job->max_sssp_iterations > 0 ? job->max_sssp_iterations : nV + 2;
   prm.n_sssp_sources = G * LS;
+  prm.n_seeds = G * LP;
   std::vector<int32_t> sg, ss;
   if (LB) {
     GAS_TRY(ensure_bfs(b, LB, G * LB));
@@ -1638,14 +1981,14 @@ gas_status_t gas_batch_run(gas_batch *b, const gas_batch_job *job, int32_t *dept
         ss[(size_t)g * LS + l] = v < 0 ? -1 : v + b->v_off[g];
       }
   }
-  std::vector<uint32_t> mask;
+  std::vector<int32_t> pg;
   if (LP) {
-    GAS_TRY(ensure_ppr(b, LP, P, c.grid_pieces, c.grid_fix));
-    mask.assign((size_t)std::max(1, nV), 0u);
+    GAS_TRY(ensure_ppr(b, LP, P, G * LP, c.grid_rows, s));
+    pg.resize((size_t)G * LP);
     for (int g = 0; g < G; ++g)
       for (int l = 0; l < LP; ++l) {
         const int32_t v = job->ppr_seeds[(size_t)g * LP + l];
-        if (v >= 0) mask[(size_t)v + b->v_off[g]] |= 1u << l;
+        pg[(size_t)g * LP + l] = v < 0 ? -1 : v + b->v_off[g];
       }
     c.ppr = ppr_args(b, LP);
   }
@@ -1670,8 +2013,7 @@ gas_status_t gas_batch_run(gas_batch *b, const gas_batch_job *job, int32_t *dept
   if (LS)
     CUDA_TRY(cudaMemcpyAsync(b->sssp_srcs, ss.data(), ss.size() * 4, cudaMemcpyHostToDevice, s));
   if (LP)
-    CUDA_TRY(cudaMemcpyAsync(b->seed_mask, mask.data(), mask.size() * 4, cudaMemcpyHostToDevice,
-                             s));
+    CUDA_TRY(cudaMemcpyAsync(b->seeds, pg.data(), pg.size() * 4, cudaMemcpyHostToDevice, s));
   if (direct) {
     GAS_TRY(run_direct(&c, loops, which, n, s));
   } else {
@@ -1695,7 +2037,7 @@ gas_status_t gas_batch_run(gas_batch *b, const gas_batch_job *job, int32_t *dept
     CUDA_TRY(cudaMemcpy2DAsync(dist_out, (size_t)LS * 4, b->dist, (size_t)b->dist_ls * 4,
                                (size_t)LS * 4, (size_t)nV, cudaMemcpyDefault, s));
   if (rank_out && LP)
-    CUDA_TRY(cudaMemcpyAsync(rank_out, b->rank[cp.iteration & 1], (size_t)nV * LP * 4,
+    CUDA_TRY(cudaMemcpyAsync(rank_out, b->rank, (size_t)nV * LP * 4,
                              cudaMemcpyDefault, s));
   CUDA_TRY(cudaStreamSynchronize(s));
   if (stats) {
@@ -1709,9 +2051,9 @@ gas_status_t gas_batch_run(gas_batch *b, const gas_batch_job *job, int32_t *dept
     for (int l = 0; l < LS; ++l) stats->sssp_lane_iterations[l] = rounds[l];
     // BFS: prologue 5 kernels (reset, seed, 3 compaction), 4 per level;
     // SSSP: prologue 6 (reset, init, seed, 3 compaction), 4 per iteration;
-    // PPR: prologue 3, 3 per iteration
+    // PPR: prologue 4 (reset, seeds, init, condition), 3 per iteration
     stats->kernel_launches = (LB ? 5 + 4 * cb.iteration : 0) +
-                             (LS ? 6 + 4 * cs.iteration : 0) + (LP ? 3 + 3 * cp.iteration : 0);
+                             (LS ? 6 + 4 * cs.iteration : 0) + (LP ? 4 + 3 * cp.iteration : 0);
     stats->graph_launches = direct ? 0 : 1;
     for (int l = 0; l < LP; ++l) stats->ppr_lane_residual[l] = resid[1 + l];
   }
@@ -1768,6 +2110,7 @@ gas_status_t gas_batch_tune(gas_batch *b, int32_t ppr_lanes, double damping, int
   prm.damping = damping;
   prm.tol = 0.0;
   prm.ppr_max_iter = INT_MAX;
+  prm.n_seeds = 1;
   CUDA_TRY(cudaMemcpyAsync(b->prm, &prm, sizeof(prm), cudaMemcpyHostToDevice, s));
   const int cands[] = {64, 128, 256, 512, 1024, 2048};
   int best = 0;
@@ -1777,13 +2120,12 @@ gas_status_t gas_batch_tune(gas_batch *b, int32_t ppr_lanes, double damping, int
   CUDA_TRY(cudaEventCreate(&ev[1]));
   gas_status_t st = GAS_OK;
   for (int P : cands) {
-    st = ensure_ppr(b, ppr_lanes, P, c.grid_pieces, c.grid_fix);
+    st = ensure_ppr(b, ppr_lanes, P, 1, c.grid_rows, s);
     if (st != GAS_OK) break;
     c.ppr = ppr_args(b, ppr_lanes);
     // a seed in lane 0 of vertex 0 makes the timed iterations do real work
-    const uint32_t one = 1u;
-    if (cudaMemsetAsync(b->seed_mask, 0, (size_t)std::max(1, e->nV) * 4, s) != cudaSuccess ||
-        cudaMemcpyAsync(b->seed_mask, &one, 4, cudaMemcpyHostToDevice, s) != cudaSuccess) {
+    const int32_t zero = 0;
+    if (cudaMemcpyAsync(b->seeds, &zero, 4, cudaMemcpyHostToDevice, s) != cudaSuccess) {
       st = fail(GAS_ERR_CUDA, "batch_tune: seed upload");
       break;
     }

@@ -470,7 +470,8 @@ typedef struct {
   double tol;                  /* PPR: stop when every lane's L1 step <= tol */
   int32_t max_bfs_levels;      /* <= 0: union V + 2                         */
   int32_t max_ppr_iterations;  /* <= 0: 1000                                */
-  int32_t piece_edges;         /* PPR edges per piece; 0: tuned or 256      */
+  int32_t piece_edges;         /* PPR edges per piece; 0: tuned, or 64 to   */
+                               /* 256 by the graphs' size                   */
   int32_t sssp_lanes;          /* 0..32 SSSP sources per graph (0: no SSSP) */
   const int32_t *sssp_sources; /* [graphs][sssp_lanes] local ids, -1 unused */
   int32_t max_sssp_iterations; /* <= 0: union V + 2                         */
