@@ -55,7 +55,9 @@ struct gas_engine {
   bool edges_dirty = false;            // a user scatter may have changed edge data
   int edge_place = GAS_EDGES_DEVICE;   // placement for the next set_graph
   bool edges_on_host = false;          // csc_src/csr_dst/csc_ed/csr_ed are pinned host memory
-  std::vector<int32_t> h_csc_off;  // for host-side counts in setActive
+  // one allocation for the arrays every graph has, and the pointers into it
+  void *arena = nullptr;
+  std::vector<void **> arena_ptrs;
 
   // device graph
   int32_t *csc_off = nullptr, *csc_src = nullptr, *csr_off = nullptr,
@@ -104,6 +106,7 @@ struct gas_engine {
   // non-empty in-edge rows of the CSC (dense slab passes)
   int32_t *ne_vid = nullptr, *ne_end = nullptr;
   int32_t n_ne = 0;
+  int32_t *ne_scratch = nullptr;
   // warp-slab chunk state: partitions of the dense CSC and of the push
   // queue, per-chunk carries (8-byte values) and fixup rows
   int32_t *slab_dpart = nullptr, *slab_qpart = nullptr, *slab_a0 = nullptr;
@@ -173,13 +176,17 @@ gas_status_t engine_commit(gas_engine *e, void *stream);
 gas_status_t engine_sync_counts(gas_engine *e, void *stream);
 int engine_grid(int64_t work_items, int per_block, int cap);
 // CSR/CSC on the device (gas_build.cu): fills csc_off/csc_src/csr_off/
-// csr_dst (+ csc_ed/csr_ed), which must be allocated, and h_csc_off; the
-// permutations (edge-list index per CSC / CSR position) when asked for.
+// csr_dst (+ csc_ed/csr_ed), which must be allocated; the permutations
+// (edge-list index per CSC / CSR position) when asked for.
 gas_status_t build_graph_device(gas_engine *e, const int32_t *srcs, const int32_t *dsts,
                                 const void *edge_data, std::vector<int32_t> *csc_perm,
                                 std::vector<int32_t> *csr_perm, void *stream);
+// Rows of the CSC with in-edges (ne_vid, ne_end; their number to the device
+// word n_out); part: ne_blocks(nV) words of scratch.
+gas_status_t build_ne_rows(gas_engine *e, int32_t *part, int32_t *n_out, void *stream);
+int ne_blocks(int nV);
 // Whether set_graph builds on the device: GAS_GRAPH_BUILD=host|device, else
-// from 1M edges up.
+// from 16,384 edges up.
 bool device_build_for(int64_t n_edges);
 // grid of a k_partition launch (fixed while capturing)
 int engine_partition_grid(gas_engine *e, int64_t items, int tile);
