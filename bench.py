@@ -1381,7 +1381,7 @@ def run_lanes24(args):
                                                   "bfs_push", pe.push_bytes, pe.push_ms,
                                                   pe.push_launches, f"rmat-s{scale}",
                                                   {"pull_launches": pe.pull_launches}),
-                  "roofline": roofline("k_ms_push (16-lane BFS push)", "ms_push",
+                  "roofline": roofline("k_ms_level (16-lane BFS, top-down levels)", "ms_push",
                                        pb.push_bytes, pb.push_ms, pb.push_launches,
                                        f"rmat-s{scale}",
                                        {"push_share_of_run": round(pb.push_ms / ms_b, 3)})}

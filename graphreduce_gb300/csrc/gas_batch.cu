@@ -13,7 +13,9 @@
 //     bitmap; a two-pass compaction over that bitmap writes the level into
 //     depth[v][l] for every new lane, folds the lanes into visited and
 //     builds the next queue (lane mask, inclusive out-edge ends, CSR offset).
-//     Depths equal those of one BFS per source.
+//     Levels with a heavy frontier run bottom-up: every vertex looks for the
+//     lanes it lacks in its in-neighbours' frontier masks and stops when it
+//     has them.  Depths equal those of one BFS per source.
 //   * multi-source SSSP (integer weights, unweighted graphs count 1 per
 //     edge): dist[v][l] rows of LS = L rounded up to 4 lanes, cmask[v] the
 //     lanes of v that changed in the current iteration.  One bulk-synchronous
@@ -89,6 +91,7 @@ __global__ void k_b_reset(gas_counters *cnt, const BatchParams *prm, int which,
   cnt->cond = 0;
   cnt->n_changed = 0;
   cnt->n_scatter_edges = 0;
+  cnt->mode = 0;
   cnt->max_iter = which == 0 ? prm->bfs_max_iter
                  : which == 1 ? prm->ppr_max_iter : prm->sssp_max_iter;
   if (edges) *edges = 0ull;
@@ -124,10 +127,7 @@ struct MsPushPol {
   }
 };
 
-__global__ void __launch_bounds__(kNT)
-    k_ms_push(MsPushPol pol, gasdev::SlabSource src) {
-  gasdev::slab_loop<MsPushPol, false>(pol, src, nullptr, nullptr, nullptr, nullptr, nullptr);
-}
+enum { kModePush = 0, kModePull = 1 };
 
 // Level 0: every (graph, lane) source.
 __global__ void k_ms_seed(const int32_t *src_global, const BatchParams *prm, int L,
@@ -141,43 +141,157 @@ __global__ void k_ms_seed(const int32_t *src_global, const BatchParams *prm, int
   }
 }
 
-// The touched-vertex traversal shared by the two compaction passes: a warp
-// owns a run of 16 words of the touched bitmap (lanes 0..15 load them) and
-// walks it in two rounds of 8 words, skipping a round whose words are all
-// clear; lane l takes vertex 32 w + l of each word, and a round's 8 words'
-// loads are issued before any is used.  For a touched vertex: its new lanes
-// and out-edge range.  The count pass keeps each warp's totals, so the
-// write passes take their offsets without counting again.
-constexpr int kMsWarpWords = 16;
-constexpr int kMsRound = 8;
-constexpr int kMsWarps = kNT / 32;
-constexpr int kMsBlockWords = kMsWarpWords * kMsWarps;  // 128 words
-
-struct MsRound {
-  uint32_t nw[kMsRound];  // new lanes (0: not touched or nothing new)
-  int off[kMsRound];
-  int deg[kMsRound];
+// The direction of the next level (Beamer, Asanovic & Patterson, SC'12, with
+// edges counted once per lane): bottom-up once the new frontier's lane-edges
+// exceed 1/kMsAlpha of those not yet explored, top-down again when the
+// frontier shrinks below V / kMsBeta vertices.  alpha: on R-MAT and
+// Erdos-Renyi graphs with 2 to 32 lanes every level with a ratio of 0.25 or
+// more reads fewer edges bottom-up (0.02 to 0.7 E against 0.4 to 1.0 E), every
+// one at 0.08 or less more.
+// A wrong bottom-up level costs more than a wrong top-down one (16 lanes on
+// 5 R-MAT graphs of 30 edges per vertex: 1.02 ms with alpha 6, 0.43 with 3,
+// 0.53 top-down only); 16 R-MAT graphs, 16 lanes: 0.66 ms with 3 to 8, 1.08
+// top-down only.
+constexpr int kMsAlpha = 3;
+constexpr int kMsBeta = 24;
+struct MsDir {
+  unsigned long long frontier;  // lane-edges of the new frontier (summed by the count pass)
+  unsigned long long explored;  // of every frontier so far
 };
 
-// The lane's word of the warp's run (lanes 0..15; 0 past the bitmap).
+// One bottom-up level: a thread per vertex looks, among its in-neighbours,
+// for the lanes it still lacks in the frontier's lane masks fr[], and stops
+// when it has them all.  Only lanes alive in its graph (with a frontier) are
+// looked for, so a source in a small component costs nothing once it is
+// done.  The first in-edge alone (sources are in id order, low ids are the
+// hubs), then four at a time; a row unfinished after 29 in-edges is taken
+// over by its whole warp, 128 at a time, or one thread would walk a hub's
+// row alone.  Writes the new lanes and whole words of the touched bitmap, as
+// the push leaves them, without an atomic.
+struct MsPull {
+  const int32_t *csc_off, *csc_src;
+  const uint32_t *fr, *alive;
+  const int32_t *g_off;
+  int G, nV;
+};
+
+__device__ __forceinline__ void ms_pull(const MsPull &a, uint32_t *vn, uint32_t *tbits) {
+  const int32_t *csc_off = a.csc_off, *csc_src = a.csc_src, *g_off = a.g_off;
+  const uint32_t *fr = a.fr, *alive = a.alive;
+  const int G = a.G, nV = a.nV;
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int kAlone = 29;
+  const int lane = threadIdx.x & 31;
+  const int nW = (nV + 31) / 32;
+  const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
+  for (int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); w < nW; w += nwarps) {
+    // the graph of the word's first vertex: the last one starting at or before it
+    int g = 0;
+    for (int lo = 0, hi = G - 1; lo < hi;) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (__ldg(g_off + mid) <= w * 32)
+        lo = mid;
+      else
+        hi = mid - 1;
+      g = lo;
+    }
+    const int v = w * 32 + lane;
+    uint32_t want = 0u, found = 0u;
+    int i = 0, end = 0;
+    if (v < nV) {
+      while (v >= __ldg(g_off + g + 1)) ++g;
+      want = __ldg(alive + g) & ~vn[2 * (size_t)v];
+      if (want) {
+        i = __ldg(csc_off + v);
+        end = __ldg(csc_off + v + 1);
+      }
+    }
+    const int stop = end - i > kAlone ? i + kAlone : end;
+    if (i < end) found = __ldg(fr + __ldg(csc_src + i)) & want;
+    for (++i; i < stop && found != want; i += 4) {
+      int u[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) u[j] = i + j < stop ? __ldg(csc_src + i + j) : -1;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) found |= u[j] >= 0 ? __ldg(fr + u[j]) & want : 0u;
+    }
+    for (unsigned rest = __ballot_sync(FULL, found != want && stop < end); rest;
+         rest &= rest - 1) {
+      const int l = __ffs(rest) - 1;
+      const uint32_t lw = __shfl_sync(FULL, want, l);
+      const int le = __shfl_sync(FULL, end, l);
+      uint32_t lf = __shfl_sync(FULL, found, l);
+      for (int p = __shfl_sync(FULL, stop, l); p < le && lf != lw; p += 128) {
+        int u[4];
+        uint32_t f = 0u;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int q = p + 32 * j + lane;
+          u[j] = q < le ? __ldg(csc_src + q) : -1;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) f |= u[j] >= 0 ? __ldg(fr + u[j]) : 0u;
+        lf |= __reduce_or_sync(FULL, f) & lw;
+      }
+      if (lane == l) found = lf;
+    }
+    if (found) vn[2 * (size_t)v + 1] = found;
+    const unsigned t = __ballot_sync(FULL, found != 0u);
+    if (lane == 0 && t) tbits[w] = t;
+  }
+}
+
+// One level in the direction the spine chose (one kernel: a node less per
+// level than a push and a pull of which one returns at once).
+__global__ void __launch_bounds__(kNT)
+    k_ms_level(MsPushPol pol, gasdev::SlabSource src, MsPull pull, const gas_counters *cnt) {
+  if (cnt->mode == kModePull)
+    ms_pull(pull, pol.vn, pol.tbits);
+  else
+    gasdev::slab_loop<MsPushPol, false>(pol, src, nullptr, nullptr, nullptr, nullptr, nullptr);
+}
+
+// The touched-vertex traversal shared by the two compaction passes: a warp
+// owns a run of WW words of the touched bitmap (lanes 0..WW-1 load them) and
+// walks it in rounds of up to 8 words, skipping a round whose words are all
+// clear; lane l takes vertex 32 w + l of each word, and a round's loads are
+// issued before any is used.  For a touched vertex: its new lanes and
+// out-edge range.  The count pass keeps each warp's totals, so the write
+// passes take their offsets without counting again.  WW is 16 on large
+// unions and less where that would leave fewer than four blocks per SM
+// (ms_words): 16 BFS lanes on 50 K vertices, 13 blocks of 16-word runs,
+// spent a fifth of the run in this pass.
+constexpr int kMsWarps = kNT / 32;
+
+template <int WW>
+struct MsRound {
+  static constexpr int R = WW < 8 ? WW : 8;
+  uint32_t nw[R];  // new lanes (0: not touched or nothing new)
+  int off[R];
+  int deg[R];
+};
+
+// The lane's word of the warp's run (lanes 0..WW-1; 0 past the bitmap).
+template <int WW>
 __device__ __forceinline__ uint32_t ms_word(const uint32_t *tbits, int nW, int w0) {
   const int lane = threadIdx.x & 31;
-  return lane < kMsWarpWords && w0 + lane < nW ? tbits[w0 + lane] : 0u;
+  return lane < WW && w0 + lane < nW ? tbits[w0 + lane] : 0u;
 }
 
+template <int WW>
 __device__ __forceinline__ bool ms_round_live(unsigned nz, int r) {
-  return ((nz >> r) & ((1u << kMsRound) - 1u)) != 0u;
+  return ((nz >> r) & ((1u << MsRound<WW>::R) - 1u)) != 0u;
 }
 
-// Round r (words w0 + r .. w0 + r + 7).  next: the SSSP's changed-lane
-// words; vn (BFS, next unused): the {visited, next} pairs, new lanes =
-// next & ~visited.
+// Round r (words w0 + r .. ).  next: the SSSP's changed-lane words; vn (BFS,
+// next unused): the {visited, next} pairs, new lanes = next & ~visited.
+template <int WW>
 __device__ __forceinline__ void ms_round_load(uint32_t myword, const uint32_t *next,
                                               const uint32_t *vn, const int32_t *csr_off,
-                                              int w0, int r, MsRound &m) {
+                                              int w0, int r, MsRound<WW> &m) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int i = 0; i < kMsRound; ++i) {
+  for (int i = 0; i < MsRound<WW>::R; ++i) {
     const uint32_t word = __shfl_sync(0xffffffffu, myword, r + i);
     m.nw[i] = 0u;
     m.off[i] = 0;
@@ -199,28 +313,32 @@ __device__ __forceinline__ void ms_round_load(uint32_t myword, const uint32_t *n
 // Pass 1: per block (queue entries, out-edges) for the spine and per warp
 // for the write pass; with lanes_active, also the OR of the new lanes of the
 // queue's entries (the SSSP loop).
+template <int WW>
 __global__ void __launch_bounds__(kNT)
     k_ms_count(const uint32_t *tbits, const uint32_t *next, const uint32_t *vn,
                const int32_t *csr_off, int nW, int32_t *part, int2 *wpart,
-               uint32_t *lanes_active) {
+               uint32_t *lanes_active, MsDir *dir) {
+  __shared__ unsigned long long s_m[kMsWarps];
   __shared__ int s_q[kMsWarps], s_d[kMsWarps];
   __shared__ uint32_t s_l[kMsWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int w0 = (blockIdx.x * kMsWarps + warp) * kMsWarpWords;
-  const uint32_t myword = ms_word(tbits, nW, w0);
+  const int w0 = (blockIdx.x * kMsWarps + warp) * WW;
+  const uint32_t myword = ms_word<WW>(tbits, nW, w0);
   const unsigned nz = __ballot_sync(0xffffffffu, myword != 0u);
   int q = 0, d = 0;
+  unsigned long long le = 0ull;  // out-edges times new lanes
   uint32_t lanes = 0u;
 #pragma unroll 1
-  for (int r = 0; r < kMsWarpWords; r += kMsRound) {
-    if (!ms_round_live(nz, r)) continue;  // warp-uniform
-    MsRound m;
-    ms_round_load(myword, next, vn, csr_off, w0, r, m);
+  for (int r = 0; r < WW; r += MsRound<WW>::R) {
+    if (!ms_round_live<WW>(nz, r)) continue;  // warp-uniform
+    MsRound<WW> m;
+    ms_round_load<WW>(myword, next, vn, csr_off, w0, r, m);
 #pragma unroll
-    for (int i = 0; i < kMsRound; ++i) {
+    for (int i = 0; i < MsRound<WW>::R; ++i) {
       const bool in = m.nw[i] && m.deg[i] > 0;
       q += in;
       d += in ? m.deg[i] : 0;
+      le += (unsigned long long)m.deg[i] * __popc(m.nw[i]);
       if (m.deg[i] > 0) lanes |= m.nw[i];
     }
   }
@@ -229,8 +347,10 @@ __global__ void __launch_bounds__(kNT)
     q += __shfl_xor_sync(0xffffffffu, q, o);
     d += __shfl_xor_sync(0xffffffffu, d, o);
     lanes |= __shfl_xor_sync(0xffffffffu, lanes, o);
+    le += __shfl_xor_sync(0xffffffffu, le, o);
   }
   if (lane == 0) {
+    s_m[warp] = le;
     s_q[warp] = q;
     s_d[warp] = d;
     s_l[warp] = lanes;
@@ -248,6 +368,11 @@ __global__ void __launch_bounds__(kNT)
     part[2 * blockIdx.x] = tq;
     part[2 * blockIdx.x + 1] = td;
     if (lanes_active && tl) atomicOr(lanes_active, tl);
+    if (dir) {
+      unsigned long long tm = 0ull;
+      for (int k = 0; k < kMsWarps; ++k) tm += s_m[k];
+      if (tm) atomicAdd(&dir->frontier, tm);
+    }
   }
 }
 
@@ -264,47 +389,114 @@ __device__ __forceinline__ int2 ms_warp_base(const int32_t *part, const int2 *wp
   return b;
 }
 
+// The new lanes' depths of a word's 32 vertices (nw per lane, `live` their
+// ballot): the warp walks the rows 32 / G at a time, lane by lane, so that a
+// row's lanes leave in one store (a thread storing its own row's lanes one by
+// one wrote a sector per depth: 118 us for 13 M depths, 49 now).
+__device__ __forceinline__ void ms_store_depths(int32_t *depth, int L, int G, int v0, uint32_t nw,
+                                                unsigned live, int level) {
+  const int lane = threadIdx.x & 31;
+  const int rows = 32 / G, l = lane % G, sub = lane / G;
+  for (int r = 0; r < 32; r += rows) {
+    if (!((live >> r) & (rows == 32 ? 0xffffffffu : (1u << rows) - 1u))) continue;  // uniform
+    const uint32_t m = __shfl_sync(0xffffffffu, nw, r + sub);
+    if ((m >> l) & 1u) depth[(size_t)(v0 + r + sub) * L + l] = level;
+  }
+}
+
 // Pass 2: depths of the new lanes (level = the iteration the spine just
-// counted), visited, the next queue and the push's chunk partition at the
-// chunk size the spine chose; clears next and the touched bitmap.
+// counted) and visited; for a top-down next level the queue and the push's
+// chunk partition at the chunk size the spine chose, for a bottom-up one
+// every vertex's frontier mask and the graphs' alive lanes; clears next and
+// the touched bitmap.
+template <int WW>
 __global__ void __launch_bounds__(kNT, 5)
     k_ms_write(uint32_t *tbits, uint32_t *vn, const int32_t *csr_off,
-               int nW, const int32_t *part, const int2 *wpart, int L, const gas_counters *cnt,
+               int nW, const int32_t *part, const int2 *wpart, int L, int G, const gas_counters *cnt,
                int32_t *depth, int32_t *q_mask, int32_t *q_end, int32_t *q_delta,
-               int32_t *chunk_row) {
+               int32_t *chunk_row, uint32_t *fr, uint32_t *alive, const int32_t *g_off,
+               int n_graphs, int nV) {
   // rows spanning many chunks (hubs), written by the whole warp at the end
   constexpr int kBig = 64;
   __shared__ int3 s_big[kMsWarps][kBig];
   __shared__ int s_nbig[kMsWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int w0 = (blockIdx.x * kMsWarps + warp) * kMsWarpWords;
-  const uint32_t myword = ms_word(tbits, nW, w0);
+  const int w0 = (blockIdx.x * kMsWarps + warp) * WW;
+  const uint32_t myword = ms_word<WW>(tbits, nW, w0);
   const unsigned nz = __ballot_sync(0xffffffffu, myword != 0u);
-  if (!nz) return;  // warp-uniform: nothing touched in the run
   const int level = cnt->iteration;
+  if (myword) tbits[w0 + lane] = 0u;
+  if (cnt->mode == kModePull) {  // grid-uniform
+    int g = 0;  // of the run's first vertex; the graphs are in vertex order
+    for (int lo = 0, hi = n_graphs - 1; lo < hi;) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (__ldg(g_off + mid) <= w0 * 32)
+        lo = mid;
+      else
+        hi = mid - 1;
+      g = lo;
+    }
+    constexpr int R = MsRound<WW>::R;
+#pragma unroll 1
+    for (int r = 0; r < WW; r += R) {
+      uint32_t nws[R];
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        const uint32_t word = __shfl_sync(0xffffffffu, myword, r + i);
+        const int v = (w0 + r + i) * 32 + lane;
+        nws[i] = 0u;
+        if ((word >> lane) & 1u) {
+          const uint2 p = reinterpret_cast<const uint2 *>(vn)[v];
+          nws[i] = p.y & ~p.x;
+          reinterpret_cast<uint2 *>(vn)[v] = make_uint2(p.x | nws[i], 0u);
+        }
+        if (v < nV) fr[v] = nws[i];
+      }
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        const uint32_t nw = nws[i];
+        const int v = (w0 + r + i) * 32 + lane;
+        const unsigned live = __ballot_sync(0xffffffffu, nw != 0u);
+        if (!live) continue;  // warp-uniform
+        ms_store_depths(depth, L, G, (w0 + r + i) * 32, nw, live, level);
+        int gv = g;
+        if (nw)
+          while (v >= __ldg(g_off + gv + 1)) ++gv;
+        const int g0 = __shfl_sync(0xffffffffu, gv, __ffs(live) - 1);
+        if (__all_sync(0xffffffffu, !nw || gv == g0)) {
+          const uint32_t all = __reduce_or_sync(0xffffffffu, nw);
+          if (lane == 0 && (__ldcg(alive + g0) & all) != all) atomicOr(alive + g0, all);
+        } else if (nw) {
+          atomicOr(alive + gv, nw);
+        }
+        g = g0;
+      }
+    }
+    return;
+  }
+  if (!nz) return;  // warp-uniform: nothing touched in the run
   const int cl = cnt->push_chunk_log2;
   if (lane == 0) s_nbig[warp] = 0;
   __syncwarp();
   const int2 base = ms_warp_base(part, wpart, warp);
   int bq = base.x, bd = base.y;
-  if (myword) tbits[w0 + lane] = 0u;
 #pragma unroll 1
-  for (int r = 0; r < kMsWarpWords; r += kMsRound) {
-    if (!ms_round_live(nz, r)) continue;  // warp-uniform
-    MsRound m;
-    ms_round_load(myword, nullptr, vn, csr_off, w0, r, m);
+  for (int r = 0; r < WW; r += MsRound<WW>::R) {
+    if (!ms_round_live<WW>(nz, r)) continue;  // warp-uniform
+    MsRound<WW> m;
+    ms_round_load<WW>(myword, nullptr, vn, csr_off, w0, r, m);
 #pragma unroll
-    for (int i = 0; i < kMsRound; ++i) {
+    for (int i = 0; i < MsRound<WW>::R; ++i) {
       const int v = (w0 + r + i) * 32 + lane;
       const uint32_t word = __shfl_sync(0xffffffffu, myword, r + i);
       if (!word) continue;  // warp-uniform
       const bool touched = (word >> lane) & 1u;
       const uint32_t nw = m.nw[i];
       if (touched) vn[2 * (size_t)v + 1] = 0u;
-      if (nw) {
-        vn[2 * (size_t)v] |= nw;
-        for (uint32_t k = nw; k; k &= k - 1) depth[(size_t)v * L + (__ffs(k) - 1)] = level;
-      }
+      if (nw) vn[2 * (size_t)v] |= nw;
+      const unsigned live = __ballot_sync(0xffffffffu, nw != 0u);
+      if (!live) continue;  // warp-uniform
+      ms_store_depths(depth, L, G, (w0 + r + i) * 32, nw, live, level);
       const int deg = nw ? m.deg[i] : 0;
       const unsigned qb = __ballot_sync(0xffffffffu, deg > 0);
       if (!qb) continue;
@@ -530,6 +722,7 @@ __global__ void k_mss_seed(const int32_t *src_global, const BatchParams *prm, in
 // out-edge ends, CSR offset; the changed lanes for rows wider than 8 lanes)
 // and the push's chunk partition at the chunk size the spine chose; clears
 // cmask and the touched bitmap.
+template <int WW>
 __global__ void __launch_bounds__(kNT, 4)
     k_mss_write(uint32_t *tbits, uint32_t *cmask, const int32_t *csr_off, int nW,
                 const int32_t *part, const int2 *wpart, int LS, const int32_t *dist,
@@ -540,8 +733,8 @@ __global__ void __launch_bounds__(kNT, 4)
   __shared__ int3 s_big[kMsWarps][kBig];
   __shared__ int s_nbig[kMsWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int w0 = (blockIdx.x * kMsWarps + warp) * kMsWarpWords;
-  const uint32_t myword = ms_word(tbits, nW, w0);
+  const int w0 = (blockIdx.x * kMsWarps + warp) * WW;
+  const uint32_t myword = ms_word<WW>(tbits, nW, w0);
   const unsigned nz = __ballot_sync(0xffffffffu, myword != 0u);
   if (!nz) return;  // warp-uniform: nothing touched in the run
   const int cl = cnt->push_chunk_log2;
@@ -551,12 +744,12 @@ __global__ void __launch_bounds__(kNT, 4)
   int bq = base.x, bd = base.y;
   if (myword) tbits[w0 + lane] = 0u;
 #pragma unroll 1
-  for (int r = 0; r < kMsWarpWords; r += kMsRound) {
-    if (!ms_round_live(nz, r)) continue;  // warp-uniform
-    MsRound m;
-    ms_round_load(myword, cmask, nullptr, csr_off, w0, r, m);
+  for (int r = 0; r < WW; r += MsRound<WW>::R) {
+    if (!ms_round_live<WW>(nz, r)) continue;  // warp-uniform
+    MsRound<WW> m;
+    ms_round_load<WW>(myword, cmask, nullptr, csr_off, w0, r, m);
 #pragma unroll
-    for (int i = 0; i < kMsRound; ++i) {
+    for (int i = 0; i < MsRound<WW>::R; ++i) {
       const int v = (w0 + r + i) * 32 + lane;
       const uint32_t word = __shfl_sync(0xffffffffu, myword, r + i);
       if (!word) continue;  // warp-uniform
@@ -612,7 +805,10 @@ constexpr int kMssSpineRegs = 8;
 __global__ void __launch_bounds__(kMssSpineNT)
     k_mss_spine(int2 *part, int nb, gas_counters *cnt, int push_warps,
                 unsigned long long *edges, uint32_t *lanes_active, int32_t *lane_rounds,
+                MsDir *dir, uint32_t *alive, int G, unsigned long long lane_edges, int nV,
                 cudaGraphConditionalHandle h, int in_graph, int first) {
+  if (alive)  // gathered again by the write pass
+    for (int g = threadIdx.x; g < G; g += kMssSpineNT) alive[g] = 0u;
   const int per = (nb + kMssSpineNT - 1) / kMssSpineNT;
   const int b0 = threadIdx.x * per, b1 = min(nb, b0 + per);
   const bool in_regs = per <= kMssSpineRegs;
@@ -685,6 +881,15 @@ __global__ void __launch_bounds__(kMssSpineNT)
       *lanes_active = 0u;
       for (int l = 0; l < kMaxLanes; ++l)
         if ((la >> l) & 1u) ++lane_rounds[l];
+    }
+    if (dir) {  // BFS: the next level's direction
+      const unsigned long long f = dir->frontier, seen = (first ? 0ull : dir->explored) + f;
+      const bool pulling = !first && cnt->mode == kModePull;
+      const bool pull = pulling ? (long long)tq * kMsBeta > nV
+                                : f * kMsAlpha > (lane_edges > seen ? lane_edges - seen : 0ull);
+      cnt->mode = pull && td > 0 ? kModePull : kModePush;
+      dir->explored = seen;
+      dir->frontier = 0ull;
     }
     const int it = first ? 0 : ++cnt->iteration;
     set_cond(cnt, td > 0, it, h, in_graph);
@@ -1215,6 +1420,11 @@ struct gas_batch {
   int32_t *depth = nullptr, *q_mask = nullptr, *q_end = nullptr,
           *q_delta = nullptr, *part = nullptr, *qpart = nullptr, *srcs = nullptr;
   int32_t depth_lanes = 0, srcs_cap = 0;
+  // bottom-up levels: frontier masks [V], alive lanes [graphs], the graphs'
+  // first vertices, the direction rule's sums
+  uint32_t *fr = nullptr, *alive = nullptr;
+  int32_t *g_off = nullptr;
+  MsDir *dir = nullptr;
   // SSSP (shares the frontier arrays above; next is the changed-lane mask)
   int32_t *dist = nullptr, *q_vals = nullptr, *sssp_srcs = nullptr, *lane_rounds = nullptr;
   uint32_t *lanes_active = nullptr;
@@ -1255,6 +1465,7 @@ void drop_graph(gas_batch *b) {
 
 void free_state(gas_batch *b) {
   drop_graph(b);
+  bfree(b->fr); bfree(b->alive); bfree(b->g_off); bfree(b->dir);
   bfree(b->vn); bfree(b->next); bfree(b->tbits); bfree(b->depth);
   bfree(b->q_mask); bfree(b->q_end); bfree(b->q_delta);
   bfree(b->part); bfree(b->qpart); bfree(b->srcs);
@@ -1283,8 +1494,14 @@ int lane_group(int L) {
 }
 
 int nwords(const gas_batch *b) { return (b->eng->nV + 31) / 32; }
+// Bitmap words per warp of the compaction passes.
+int ms_words(const gas_batch *b) {
+  const int64_t room = 4LL * b->eng->num_sms * kMsWarps;  // warps of four blocks per SM
+  return nwords(b) <= 2 * room ? 2 : nwords(b) <= 4 * room ? 4 : 16;
+}
 int ms_blocks(const gas_batch *b) {
-  return std::max(1, (nwords(b) + kMsBlockWords - 1) / kMsBlockWords);
+  const int words = ms_words(b) * kMsWarps;
+  return std::max(1, (nwords(b) + words - 1) / words);
 }
 // qpart: the blocks' (entries, out-edges) pairs, one spare pair, then the
 // blocks' per-warp pairs
@@ -1341,6 +1558,14 @@ gas_status_t ensure_bfs(gas_batch *b, int lanes, int n_sources) {
   const size_t nV = std::max(1, e->nV);
   GAS_TRY(ensure_frontier(b));
   if (!b->vn) CUDA_TRY(cudaMalloc(&b->vn, nV * 8));
+  if (!b->dir) {
+    CUDA_TRY(cudaMalloc(&b->fr, nV * 4));
+    CUDA_TRY(cudaMalloc(&b->alive, b->v_off.size() * 4));
+    CUDA_TRY(cudaMalloc(&b->g_off, b->v_off.size() * 4));
+    CUDA_TRY(cudaMemcpy(b->g_off, b->v_off.data(), b->v_off.size() * 4, cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMalloc(&b->dir, sizeof(MsDir)));
+    CUDA_TRY(cudaMemset(b->dir, 0, sizeof(MsDir)));
+  }
   if (b->depth_lanes != lanes) {
     drop_graph(b);
     bfree(b->depth);
@@ -1472,21 +1697,34 @@ typedef gas_status_t (*StepFn)(RunCtx *, cudaStream_t, cudaGraphConditionalHandl
 
 // The next frontier of new lanes, then the loop control (first: the
 // prologue's sources, level 0).
-gas_status_t bfs_compact(RunCtx *c, cudaStream_t s, cudaGraphConditionalHandle h, int ig,
-                         int first) {
+template <int WW>
+gas_status_t bfs_compact_w(RunCtx *c, cudaStream_t s, cudaGraphConditionalHandle h, int ig,
+                           int first) {
   gas_batch *b = c->b;
   gas_engine *e = b->eng;
   const int nb = ms_blocks(b);
-  k_ms_count<<<nb, kNT, 0, s>>>(b->tbits, nullptr, b->vn, e->csr_off, nwords(b), b->qpart,
-                                ms_wpart(b), nullptr);
+  const int L = c->bfs_lanes, ng = (int)b->v_off.size() - 1;
+  k_ms_count<WW><<<nb, kNT, 0, s>>>(b->tbits, nullptr, b->vn, e->csr_off, nwords(b), b->qpart,
+                                ms_wpart(b), nullptr, b->dir);
   k_mss_spine<<<1, kMssSpineNT, 0, s>>>(reinterpret_cast<int2 *>(b->qpart), nb, b->cnt,
                                         c->slab_grid * (kNT / 32), b->edges, nullptr, nullptr,
-                                        h, ig, first);
-  k_ms_write<<<nb, kNT, 0, s>>>(b->tbits, b->vn, e->csr_off, nwords(b), b->qpart,
-                               ms_wpart(b), c->bfs_lanes, b->cnt, b->depth, b->q_mask, b->q_end, b->q_delta,
-                               b->part);
+                                        b->dir, b->alive, ng, (unsigned long long)e->nE * L,
+                                        e->nV, h, ig, first);
+  k_ms_write<WW><<<nb, kNT, 0, s>>>(b->tbits, b->vn, e->csr_off, nwords(b), b->qpart,
+                               ms_wpart(b), L, lane_group(L), b->cnt, b->depth, b->q_mask,
+                               b->q_end, b->q_delta, b->part, b->fr, b->alive, b->g_off, ng,
+                               e->nV);
   CUDA_TRY(cudaGetLastError());
   return GAS_OK;
+}
+
+gas_status_t bfs_compact(RunCtx *c, cudaStream_t s, cudaGraphConditionalHandle h, int ig,
+                         int first) {
+  switch (ms_words(c->b)) {
+    case 2: return bfs_compact_w<2>(c, s, h, ig, first);
+    case 4: return bfs_compact_w<4>(c, s, h, ig, first);
+    default: return bfs_compact_w<16>(c, s, h, ig, first);
+  }
 }
 
 gas_status_t bfs_prologue(RunCtx *c, cudaStream_t s, cudaGraphConditionalHandle h, int ig) {
@@ -1509,7 +1747,9 @@ gas_status_t bfs_push(RunCtx *c, cudaStream_t s) {
       b->q_end, nullptr, b->q_delta, 0, 0, &b->cnt->n_changed, &b->cnt->n_scatter_edges,
       b->part, &b->cnt->push_chunk_log2);
   MsPushPol pol{e->csr_dst, b->q_mask, b->vn, b->tbits};
-  k_ms_push<<<c->slab_grid, kNT, 0, s>>>(pol, q);
+  const MsPull pull{e->csc_off, e->csc_src, b->fr, b->alive, b->g_off,
+                    (int)b->v_off.size() - 1, e->nV};
+  k_ms_level<<<c->slab_grid, kNT, 0, s>>>(pol, q, pull, b->cnt);
   CUDA_TRY(cudaGetLastError());
   return GAS_OK;
 }
@@ -1526,9 +1766,15 @@ gas_status_t bfs_body(RunCtx *c, cudaStream_t s, cudaGraphConditionalHandle h, i
     CUDA_TRY(cudaEventSynchronize(b->pev[1]));
     float ms = 0.f;
     CUDA_TRY(cudaEventElapsedTime(&ms, b->pev[0], b->pev[1]));
-    b->prof.push_ms += ms;
-    b->prof.push_bytes += (int64_t)k.n_scatter_edges * 12 + (int64_t)k.n_changed * 12;
-    b->prof.push_launches += 1;
+    if (k.mode == kModePull) {  // the dense reads only: visited, next, offsets
+      b->prof.pull_ms += ms;
+      b->prof.pull_bytes += 12LL * b->eng->nV;
+      b->prof.pull_launches += 1;
+    } else {
+      b->prof.push_ms += ms;
+      b->prof.push_bytes += (int64_t)k.n_scatter_edges * 12 + (int64_t)k.n_changed * 12;
+      b->prof.push_launches += 1;
+    }
   } else {
     GAS_TRY(bfs_push(c, s));
   }
@@ -1537,21 +1783,32 @@ gas_status_t bfs_body(RunCtx *c, cudaStream_t s, cudaGraphConditionalHandle h, i
 
 // The queue of the changed lanes, then the loop control (first: the
 // prologue's queue).
-gas_status_t sssp_compact(RunCtx *c, cudaStream_t s, cudaGraphConditionalHandle h, int ig,
-                          int first) {
+template <int WW>
+gas_status_t sssp_compact_w(RunCtx *c, cudaStream_t s, cudaGraphConditionalHandle h, int ig,
+                            int first) {
   gas_batch *b = c->b;
   gas_engine *e = b->eng;
   const int nb = ms_blocks(b);
-  k_ms_count<<<nb, kNT, 0, s>>>(b->tbits, b->next, nullptr, e->csr_off, nwords(b), b->qpart,
-                                ms_wpart(b), b->lanes_active);
+  k_ms_count<WW><<<nb, kNT, 0, s>>>(b->tbits, b->next, nullptr, e->csr_off, nwords(b), b->qpart,
+                                ms_wpart(b), b->lanes_active, nullptr);
   k_mss_spine<<<1, kMssSpineNT, 0, s>>>(reinterpret_cast<int2 *>(b->qpart), nb, b->cnt + 2,
                                         c->sssp_grid * (kNT / 32), b->sssp_edges,
-                                        b->lanes_active, b->lane_rounds, h, ig, first);
-  k_mss_write<<<nb, kNT, 0, s>>>(b->tbits, b->next, e->csr_off, nwords(b), b->qpart,
+                                        b->lanes_active, b->lane_rounds, nullptr, nullptr, 0,
+                                        0ull, 0, h, ig, first);
+  k_mss_write<WW><<<nb, kNT, 0, s>>>(b->tbits, b->next, e->csr_off, nwords(b), b->qpart,
                                  ms_wpart(b), b->dist_ls, b->dist, b->q_mask, b->q_vals, b->q_end,
                                  b->q_delta, b->part, b->cnt + 2);
   CUDA_TRY(cudaGetLastError());
   return GAS_OK;
+}
+
+gas_status_t sssp_compact(RunCtx *c, cudaStream_t s, cudaGraphConditionalHandle h, int ig,
+                          int first) {
+  switch (ms_words(c->b)) {
+    case 2: return sssp_compact_w<2>(c, s, h, ig, first);
+    case 4: return sssp_compact_w<4>(c, s, h, ig, first);
+    default: return sssp_compact_w<16>(c, s, h, ig, first);
+  }
 }
 
 gas_status_t sssp_prologue(RunCtx *c, cudaStream_t s, cudaGraphConditionalHandle h, int ig) {
@@ -1755,7 +2012,7 @@ void ppr_grids(const gas_engine *e, RunCtx *c) {
 void grids(gas_batch *b, RunCtx *c) {
   gas_engine *e = b->eng;
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ms_push, kNT, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ms_level, kNT, 0);
   c->slab_grid = e->num_sms * (per_sm > 0 ? per_sm : 1);
   switch (ppr_vl(c->ppr_lanes)) {
     case 4: ppr_grids<4>(e, c); break;
