@@ -1430,6 +1430,9 @@ struct gas_batch {
   uint32_t *lanes_active = nullptr;
   unsigned long long *sssp_edges = nullptr;
   int32_t dist_ls = 0, sssp_srcs_cap = 0;
+  // the arrays above and below by what allocates them: the frontier, the SSSP
+  // rows, the BFS state, the PPR rows and plan
+  DeviceGroup frontier_mem, dist_mem, bfs_mem, ppr_mem, plan_mem;
   // profiling of the SSSP pushes (direct launches, events around each push)
   bool profiling = false;
   cudaEvent_t pev[2] = {nullptr, nullptr};
@@ -1465,17 +1468,16 @@ void drop_graph(gas_batch *b) {
 
 void free_state(gas_batch *b) {
   drop_graph(b);
-  bfree(b->fr); bfree(b->alive); bfree(b->g_off); bfree(b->dir);
-  bfree(b->vn); bfree(b->next); bfree(b->tbits); bfree(b->depth);
-  bfree(b->q_mask); bfree(b->q_end); bfree(b->q_delta);
-  bfree(b->part); bfree(b->qpart); bfree(b->srcs);
-  bfree(b->first_row); bfree(b->split_row); bfree(b->split_last);
-  bfree(b->head); bfree(b->tail); bfree(b->row_bits);
-  bfree(b->seed_mask); bfree(b->seeds); bfree(b->l1); bfree(b->ticket);
-  bfree(b->dist); bfree(b->q_vals); bfree(b->sssp_srcs); bfree(b->lane_rounds);
+  b->frontier_mem.free();
+  b->dist_mem.free();
+  b->bfs_mem.free();
+  b->ppr_mem.free();
+  b->plan_mem.free();
+  bfree(b->depth); bfree(b->srcs);
+  bfree(b->seed_mask); bfree(b->seeds); bfree(b->l1); bfree(b->ticket); bfree(b->row_bits);
+  bfree(b->sssp_srcs); bfree(b->lane_rounds);
   bfree(b->lanes_active);
   b->dist_ls = b->sssp_srcs_cap = 0;
-  bfree(b->rank); bfree(b->contrib); bfree(b->sum);
   b->n_pieces = b->piece_edges = b->ppr_lanes = b->depth_lanes = 0;
   b->srcs_cap = b->l1_cap = b->seeds_cap = 0;
 }
@@ -1515,14 +1517,13 @@ gas_status_t ensure_frontier(gas_batch *b) {
   gas_engine *e = b->eng;
   const size_t nV = std::max(1, e->nV), nW = std::max(1, nwords(b));
   if (!b->next) {
-    CUDA_TRY(cudaMalloc(&b->next, nV * 4));
-    CUDA_TRY(cudaMalloc(&b->tbits, nW * 4));
-    for (int32_t **p : {&b->q_mask, &b->q_end, &b->q_delta})
-      CUDA_TRY(cudaMalloc(p, nV * 4));
-    // the SSSP push cuts its queue's edges into chunks of 64 to 512 edges
-    CUDA_TRY(cudaMalloc(&b->part, (((size_t)e->nE >> gasdev::kSlabChunkMinLog2) + 2) * 4));
-    CUDA_TRY(cudaMalloc(&b->qpart,
-                        2 * ((size_t)ms_blocks(b) + 1 + (size_t)ms_blocks(b) * kMsWarps) * 4));
+    // part: the SSSP push cuts its queue's edges into chunks of 64 to 512 edges
+    CUDA_TRY(b->frontier_mem.alloc(
+        {GROUP_PART(b->next, nV * 4), GROUP_PART(b->tbits, nW * 4), GROUP_PART(b->q_mask, nV * 4),
+         GROUP_PART(b->q_end, nV * 4), GROUP_PART(b->q_delta, nV * 4),
+         GROUP_PART(b->part, (((size_t)e->nE >> gasdev::kSlabChunkMinLog2) + 2) * 4),
+         GROUP_PART(b->qpart,
+                    2 * ((size_t)ms_blocks(b) + 1 + (size_t)ms_blocks(b) * kMsWarps) * 4)}));
   }
   return GAS_OK;
 }
@@ -1534,10 +1535,9 @@ gas_status_t ensure_sssp(gas_batch *b, int lanes, int n_sources) {
   const int LS = (lanes + 3) & ~3;
   if (b->dist_ls != LS) {
     drop_graph(b);
-    bfree(b->dist);
-    bfree(b->q_vals);
-    CUDA_TRY(cudaMalloc(&b->dist, nV * LS * 4));
-    CUDA_TRY(cudaMalloc(&b->q_vals, nV * LS * 4));
+    b->dist_ls = 0;
+    CUDA_TRY(b->dist_mem.alloc(
+        {GROUP_PART(b->dist, nV * LS * 4), GROUP_PART(b->q_vals, nV * LS * 4)}));
     b->dist_ls = LS;
   }
   if (!b->lane_rounds) {
@@ -1557,13 +1557,12 @@ gas_status_t ensure_bfs(gas_batch *b, int lanes, int n_sources) {
   gas_engine *e = b->eng;
   const size_t nV = std::max(1, e->nV);
   GAS_TRY(ensure_frontier(b));
-  if (!b->vn) CUDA_TRY(cudaMalloc(&b->vn, nV * 8));
-  if (!b->dir) {
-    CUDA_TRY(cudaMalloc(&b->fr, nV * 4));
-    CUDA_TRY(cudaMalloc(&b->alive, b->v_off.size() * 4));
-    CUDA_TRY(cudaMalloc(&b->g_off, b->v_off.size() * 4));
+  if (!b->vn) {
+    const size_t ng = b->v_off.size();
+    CUDA_TRY(b->bfs_mem.alloc({GROUP_PART(b->vn, nV * 8), GROUP_PART(b->fr, nV * 4),
+                               GROUP_PART(b->alive, ng * 4), GROUP_PART(b->g_off, ng * 4),
+                               GROUP_PART(b->dir, sizeof(MsDir))}));
     CUDA_TRY(cudaMemcpy(b->g_off, b->v_off.data(), b->v_off.size() * 4, cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMalloc(&b->dir, sizeof(MsDir)));
     CUDA_TRY(cudaMemset(b->dir, 0, sizeof(MsDir)));
   }
   if (b->depth_lanes != lanes) {
@@ -1591,13 +1590,10 @@ gas_status_t ensure_ppr(gas_batch *b, int lanes, int P, int n_seeds, int grid_ro
   const size_t nE = std::max(1, e->nE);
   if (b->ppr_lanes != lanes) {
     drop_graph(b);
-    bfree(b->rank);
-    bfree(b->contrib);
-    bfree(b->sum);
     b->ppr_lanes = 0;
-    CUDA_TRY(cudaMalloc(&b->rank, nV * lanes * 4));
-    CUDA_TRY(cudaMalloc(&b->contrib, nV * lanes * 4));
-    CUDA_TRY(cudaMalloc(&b->sum, n_ne * lanes * 4));
+    const size_t row = (size_t)lanes * 4;
+    CUDA_TRY(b->ppr_mem.alloc({GROUP_PART(b->rank, nV * row), GROUP_PART(b->contrib, nV * row),
+                               GROUP_PART(b->sum, n_ne * row)}));
     b->ppr_lanes = lanes;
     b->piece_edges = 0;  // head/tail are sized by lanes
   }
@@ -1635,15 +1631,10 @@ gas_status_t ensure_ppr(gas_batch *b, int lanes, int P, int n_seeds, int grid_ro
   const int Pu = (P + kPprU - 1) / kPprU * kPprU;
   const int32_t n_pieces = (int32_t)(((int64_t)e->nE + Pu - 1) / Pu);
   const size_t np = std::max(1, n_pieces);
-  bfree(b->first_row);
-  bfree(b->split_row);
-  bfree(b->split_last);
-  bfree(b->head);
-  bfree(b->tail);
-  for (int32_t **p : {&b->first_row, &b->split_row, &b->split_last})
-    CUDA_TRY(cudaMalloc(p, np * 4));
-  CUDA_TRY(cudaMalloc(&b->head, np * lanes * sizeof(CVal)));
-  CUDA_TRY(cudaMalloc(&b->tail, np * lanes * sizeof(CVal)));
+  CUDA_TRY(b->plan_mem.alloc(
+      {GROUP_PART(b->first_row, np * 4), GROUP_PART(b->split_row, np * 4),
+       GROUP_PART(b->split_last, np * 4), GROUP_PART(b->head, np * lanes * sizeof(CVal)),
+       GROUP_PART(b->tail, np * lanes * sizeof(CVal))}));
   k_ppr_plan<<<8 * e->num_sms, 256, 0, s>>>(e->ne_end, e->n_ne, n_pieces, Pu, e->nE,
                                            b->first_row, b->split_row, b->split_last);
   CUDA_TRY(cudaGetLastError());
@@ -2161,6 +2152,7 @@ gas_status_t gas_batch_build(gas_batch *b, void *stream) {
     gas_engine_destroy(b->eng);
     b->eng = we;
   }
+  b->eng->graph_only = true;
   std::vector<int32_t> vd((size_t)std::max(1, nV), -1);
   GAS_TRY(gas_engine_set_graph(b->eng, nV, vd.data(), (int64_t)b->src.size(),
                                b->weighted ? b->w.data() : nullptr, b->src.data(),
@@ -2177,6 +2169,13 @@ gas_status_t gas_batch_build(gas_batch *b, void *stream) {
   std::vector<int32_t>().swap(b->src);
   std::vector<int32_t>().swap(b->dst);
   std::vector<int32_t>().swap(b->w);
+  // the traversals' frontier, so that the first run finds it (tight memory:
+  // that run asks again)
+  if (ensure_frontier(b) != GAS_OK) {
+    b->frontier_mem.free();
+    cudaGetLastError();
+    gas::clear_error();
+  }
   b->built = true;
   return GAS_OK;
 }

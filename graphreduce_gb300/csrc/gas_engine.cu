@@ -647,8 +647,7 @@ void free_graph(gas_engine *e) {
   e->h_csr_to_csc.clear();
   e->host_ed = nullptr;
   e->edges_dirty = false;
-  dfree(e->q_ids); dfree(e->q_vals); dfree(e->q_end); dfree(e->q_delta); dfree(e->snap);
-  dfree(e->qpart); dfree(e->cbits);
+  e->fast_mem.free();
   e->n_ne = e->slab_cap = 0;
   for (int i = 0; i < kGraphSlots; ++i) {
     if (e->graphs[i]) cudaGraphExecDestroy(e->graphs[i]);
@@ -1077,6 +1076,7 @@ gas_status_t gas_engine_set_graph(gas_engine *e, int32_t nV, void *vertex_data,
   // the host vectors are released at return: wait for the copies
   CUDA_TRY(cudaStreamSynchronize(st));
   e->n_ne = *h_ne;
+  gas::reserve_fast_buffers(e);
   e->n_active = 0;
   e->n_edges = 0;
   e->counts_dirty = false;

@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include <initializer_list>
 #include <vector>
 
 #include "gas.h"
@@ -23,6 +24,43 @@
     gas_status_t s_ = (call);          \
     if (s_ != GAS_OK) return s_;       \
   } while (0)
+
+// Device arrays that are allocated and freed together, in one cudaMalloc (each
+// costs 50 to 200 us, and a first run makes up to a dozen).
+struct DeviceGroup {
+  struct Part {
+    void **p;
+    size_t bytes;
+  };
+  void *base = nullptr;
+  std::vector<void **> ptrs;
+  cudaError_t alloc(std::initializer_list<Part> parts) {
+    free();
+    size_t total = 0;
+    for (const Part &x : parts) total += round(x.bytes);
+    const cudaError_t ce = cudaMalloc(&base, total);
+    if (ce != cudaSuccess) {
+      base = nullptr;
+      return ce;
+    }
+    size_t at = 0;
+    for (const Part &x : parts) {
+      *x.p = static_cast<char *>(base) + at;
+      ptrs.push_back(x.p);
+      at += round(x.bytes);
+    }
+    return cudaSuccess;
+  }
+  void free() {
+    if (base) cudaFree(base);
+    base = nullptr;
+    for (void **p : ptrs) *p = nullptr;
+    ptrs.clear();
+  }
+  static size_t round(size_t n) { return (n + 255) / 256 * 256 + (n == 0 ? 256 : 0); }
+};
+#define GROUP_PART(ptr, bytes) \
+  DeviceGroup::Part { reinterpret_cast<void **>(&(ptr)), (size_t)(bytes) }
 
 // ---------------------------------------------------------------------------
 // The engine object.
@@ -101,6 +139,8 @@ struct gas_engine {
   int32_t *q_ids = nullptr, *q_vals = nullptr, *q_end = nullptr, *q_delta = nullptr;
   int32_t *snap = nullptr, *qpart = nullptr;
   uint32_t *cbits = nullptr;
+  DeviceGroup fast_mem;  // all of them
+  bool graph_only = false;  // holds a batch's union graph: never runs itself
   int32_t pull_div = 4;
 
   // non-empty in-edge rows of the CSC (dense slab passes)
@@ -175,6 +215,9 @@ gas_status_t engine_commit(gas_engine *e, void *stream);
 // host copy of the counters (synchronises the stream)
 gas_status_t engine_sync_counts(gas_engine *e, void *stream);
 int engine_grid(int64_t work_items, int per_block, int cap);
+// the fast schedule's buffers, with the graph's arrays where a run will want
+// them (large BFS, SSSP and CC graphs), so that the first run finds them
+void reserve_fast_buffers(gas_engine *e);
 // CSR/CSC on the device (gas_build.cu): fills csc_off/csc_src/csr_off/
 // csr_dst (+ csc_ed/csr_ed), which must be allocated; the permutations
 // (edge-list index per CSC / CSR position) when asked for.

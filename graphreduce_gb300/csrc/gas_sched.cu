@@ -1035,14 +1035,11 @@ gas_status_t ensure_fast_buffers(gas_engine *e) {
   if (e->q_ids) return GAS_OK;
   const size_t V = (size_t)e->nV, nW = (V + 31) / 32;
   const size_t nqb = (nW + kQWordsPerBlock - 1) / kQWordsPerBlock;
-  CUDA_TRY(cudaMalloc(&e->q_ids, (V ? V : 1) * 4));
-  CUDA_TRY(cudaMalloc(&e->q_vals, (V ? V : 1) * 4));
-  CUDA_TRY(cudaMalloc(&e->q_end, (V ? V : 1) * 4));
-  CUDA_TRY(cudaMalloc(&e->q_delta, (V ? V : 1) * 4));
-  CUDA_TRY(cudaMalloc(&e->snap, (V ? V : 1) * 4));
-  CUDA_TRY(cudaMalloc(&e->cbits, (nW ? nW : 1) * 4));
-  // block totals, then the blocks' per-warp totals
-  CUDA_TRY(cudaMalloc(&e->qpart, (nqb ? nqb : 1) * (1 + kQWarpsPerBlock) * sizeof(int4)));
+  // qpart: block totals, then the blocks' per-warp totals
+  CUDA_TRY(e->fast_mem.alloc(
+      {GROUP_PART(e->q_ids, V * 4), GROUP_PART(e->q_vals, V * 4), GROUP_PART(e->q_end, V * 4),
+       GROUP_PART(e->q_delta, V * 4), GROUP_PART(e->snap, V * 4), GROUP_PART(e->cbits, nW * 4),
+       GROUP_PART(e->qpart, nqb * (1 + kQWarpsPerBlock) * sizeof(int4))}));
   CUDA_TRY(cudaMemset(e->cbits, 0, (nW ? nW : 1) * 4));
   return GAS_OK;
 }
@@ -1050,6 +1047,18 @@ gas_status_t ensure_fast_buffers(gas_engine *e) {
 }  // namespace
 
 namespace gas {
+
+void reserve_fast_buffers(gas_engine *e) {
+  const bool sized = e->prog == GAS_PROG_BFS ? e->nV > kBfsSmallMaxV
+                     : (e->prog == GAS_PROG_SSSP || e->prog == GAS_PROG_CC) &&
+                           e->nV > kMinSmallLearnedMaxV;
+  if (!sized || e->graph_only) return;
+  if (ensure_fast_buffers(e) != GAS_OK) {  // tight memory: the first run asks again
+    e->fast_mem.free();
+    cudaGetLastError();
+    clear_error();
+  }
+}
 
 // WHILE graph with a captured prologue before the loop node.
 static gas_status_t build_fast_graph(gas_engine *e, FastCtx *ctx,
