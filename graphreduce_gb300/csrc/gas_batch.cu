@@ -29,13 +29,13 @@
 //   * multi-seed personalized PageRank, r_l = (1-d) e_{s_l} + d A^T D^-1 r_l
 //     for every lane l at once: ranks and contributions are [V][L] rows, so
 //     the L lanes of an in-edge's source are one contiguous 4L-byte read.
-//     The CSC edge range is cut into pieces of P edges (P autotuned); a group
-//     of L threads (one per lane) folds a piece in edge order with FP32
-//     two-sum compensation and stores the sum of every row that lies inside
-//     the piece; rows cut by piece boundaries leave per-piece partials that a
-//     second pass folds in a fixed order; a streaming pass turns the rows'
-//     sums into ranks, contributions and residuals.  The sums are
-//     deterministic.  The loop runs until the largest per-lane FP64 L1
+//     Rows are cut into units of at most 128 in-edges, sorted by length in
+//     windows, and the groups of a warp (a thread for one, two or four lanes)
+//     walk equally long units side by side with FP32 two-sum compensation,
+//     P edges per group and piece (P autotuned); rows of several units leave
+//     partials that a second pass folds in a fixed order; a streaming pass
+//     turns the rows' sums into ranks, contributions and residuals.  The sums
+//     are deterministic.  The loop runs until the largest per-lane L1
 //     residual is <= tol.
 //
 // The loops are WHILE nodes of one CUDA graph (BFS, SSSP, then PPR), each
@@ -913,19 +913,16 @@ __device__ __forceinline__ CVal two_sum_add(CVal a, CVal b) {
 }
 
 struct PprArgs {
-  const int32_t *csc_src, *csc_off, *csr_off;
-  // the rows with in-edges (vertex, end of its in-edges), and one bit per
-  // in-edge: the last of its row
-  const int32_t *ne_vid, *ne_end;
-  const uint32_t *row_bits;
-  // pieces of P edges (a multiple of kPprU): row of the first edge; and for
-  // a row that starts in the piece and goes on past it, the row and the last
-  // piece with an edge of it (-1: none)
-  const int32_t *first_row, *split_row, *split_last;
-  int32_t n_pieces, P, E, L, G, n_ne, nV;
-  CVal *head, *tail;  // [n_pieces][L] partials of cut rows
+  const int32_t *csc_off, *csr_off;
+  const int32_t *ne_vid;  // the rows with in-edges
+  // the plan (below): sources in walking order, the slices' first steps, the
+  // units' destinations, the pieces' first slices, the rows of several units
+  // and their first partials
+  const int32_t *idx, *step_off, *unit_dst, *piece_start, *long_row, *long_slot;
+  int32_t n_pieces, n_long, L, G, n_ne, nV;
+  CVal *partial;      // [slots][L] partial sums of the units of long rows
   float *sum;         // [n_ne][L] the rows' sums of an iteration
-  float *rank, *contrib;  // [V][L]
+  float *rank, *contrib;  // [V][L], [V + 1][L]: the last row stays 0
   const uint32_t *seed_mask;
   const BatchParams *prm;
   gas_counters *cnt;
@@ -934,25 +931,21 @@ struct PprArgs {
   unsigned int *ticket;   // blocks of k_ppr_rows done (left at 0)
 };
 
-constexpr int kPprU = 8;      // in-edges of a step of the gather
-constexpr int kPprLong = 16;  // rows over more pieces are folded by a whole CTA
-
-// Eight CSC sources from edge e (a multiple of 8): one 32-byte load, the
-// same address in every thread of the group.
-__device__ __forceinline__ void ppr_src8(const PprArgs &a, int e, int end, int (&u)[kPprU]) {
-  const int n = end - e;  // (differences: e + 8 may not fit an int)
-  if (a.E - e >= kPprU) {
-    nc8(a.csc_src + e, u);
-  } else {
-#pragma unroll
-    for (int j = 0; j < kPprU; ++j) u[j] = j < n ? __ldg(a.csc_src + e + j) : -1;
-  }
-  if (n < kPprU) {
-#pragma unroll
-    for (int j = 0; j < kPprU; ++j)
-      if (j >= n) u[j] = -1;
-  }
-}
+// The gather's plan.  A row's in-edges are cut into units of at most 128
+// edges; the units of a window of 2,048 are sorted by their number of steps
+// (8 edges each), and S units that follow one another in that order, S the
+// groups of a warp, form a slice: the warp walks them side by side, and since
+// they are (nearly) equally long their rows end at the same step.  The
+// sources are stored step by step, S x 8 to a step, short rows padded with
+// the index of a contribution row of zeros: a warp's reads of them are whole
+// lines and need no bounds.  (A walk of consecutive rows by 8 groups finds a
+// row end in three of four steps, in one group, and all wait for it: 630 us
+// per iteration at 64 M edges and 16 lanes, issue slots half busy with 16
+// warps per SM, against 367.)
+constexpr int kPprU = 8;          // in-edges of a step of the gather
+constexpr int kPprUnit = 128;     // in-edges of a unit
+constexpr int kPprWindow = 2048;  // units sorted together
+constexpr int kPprLong = 16;      // rows of more units are folded by a whole CTA
 
 // VL consecutive lanes of a row, one load or store.
 template <int VL>
@@ -989,105 +982,93 @@ template <int VL>
 __device__ __forceinline__ void ppr_contrib8(const PprArgs &a, const int (&u)[kPprU], int l,
                                              Lanes<VL> (&x)[kPprU]) {
 #pragma unroll
-  for (int j = 0; j < kPprU; ++j) {
-    if (u[j] >= 0) {
-      x[j] = ppr_ld<VL>(a.contrib + (size_t)u[j] * a.L + l);
-    } else {
-#pragma unroll
-      for (int q = 0; q < VL; ++q) x[j].f[q] = 0.f;
-    }
-  }
+  for (int j = 0; j < kPprU; ++j) x[j] = ppr_ld<VL>(a.contrib + (size_t)u[j] * a.L + l);
 }
 
-// The gather: a group of G / VL threads (VL lanes each) walks a piece in
-// steps of 8 in-edges whatever the rows are, two steps' contribution rows,
-// two steps' sources and the next 32 row ends in flight; the row ends come
-// from a bit per edge.  A step inside one row is summed pairwise in FP32
+// The gather: a warp takes a piece of consecutive slices, a group of G / VL
+// threads (VL lanes each) a unit of each, with the next step's contribution
+// rows and two steps' sources in flight.  A step is summed pairwise in FP32
 // (relative error <= 3 u of the step's sum, the terms being non-negative),
-// other steps term by term; both go into the row's sum by two-sum, so a
-// row's error stays near 3 u of its value.  Rows that end in the piece they
-// start in store their sum (by row, no dependent load); the others leave
+// the last step of a slice term by term; both go into the unit's sum by
+// two-sum, so a row's error stays near 3 u of its value.  Rows of one unit
+// store their sum (by row, no dependent load), units of longer rows leave
 // partials for k_ppr_fix.  What follows a row's sum (rank, contribution,
 // residual) is k_ppr_rows', a streaming pass: done here, each row end
 // stalled the walk on four loads.
 template <int VL>
-__global__ void __launch_bounds__(kNT) k_ppr_pieces(PprArgs a) {
-  const int T = a.G / VL;
-  const int l = threadIdx.x % T * VL;
-  if (l >= a.L) return;
-  const int per_block = kNT / T;
-  for (int k = blockIdx.x * per_block + (int)threadIdx.x / T; k < a.n_pieces;
-       k += gridDim.x * per_block) {
-    const int e0 = k * a.P;
-    const int end = a.E - e0 < a.P ? a.E : e0 + a.P;
-    int r = __ldg(a.first_row + k);
-    bool cont = e0 > 0 && !((__ldg(a.row_bits + ((e0 - 1) >> 5)) >> ((e0 - 1) & 31)) & 1u);
-    uint32_t word = __ldg(a.row_bits + (e0 >> 5)), word2 = 0u;
-    if (((end - 1) >> 5) > (e0 >> 5)) word2 = __ldg(a.row_bits + (e0 >> 5) + 1);
+__global__ void __launch_bounds__(kNT) k_ppr_units(PprArgs a) {
+  const int T = a.G / VL, S = 32 / T;
+  const int lane = threadIdx.x & 31, g = lane / T;
+  const int l = lane % T * VL;
+  const bool on = l < a.L;
+  const int lc = on ? l : 0;
+  const int nwarps = (int)((gridDim.x * kNT) >> 5);
+  for (int k = (int)((blockIdx.x * kNT + threadIdx.x) >> 5); k < a.n_pieces; k += nwarps) {
+    int s = __ldg(a.piece_start + k);
+    const int s_end = __ldg(a.piece_start + k + 1);
+    if (s == s_end) continue;  // warp-uniform
+    int t = __ldg(a.step_off + s);
+    const int t_end = __ldg(a.step_off + s_end);
+    int next = __ldg(a.step_off + s + 1), next2 = 0;
+    int dst = __ldg(a.unit_dst + (size_t)s * S + g), dst2 = 0;
+    if (s + 1 < s_end) {
+      next2 = __ldg(a.step_off + s + 2);
+      dst2 = __ldg(a.unit_dst + (size_t)(s + 1) * S + g);
+    }
+    const int32_t *p = a.idx + ((size_t)t * S + g) * kPprU;
     int u[kPprU], u2[kPprU];
     Lanes<VL> x[kPprU], y[kPprU];
-    ppr_src8(a, e0, end, u);
-    if (end - e0 > kPprU) ppr_src8(a, e0 + kPprU, end, u2);
-    ppr_contrib8<VL>(a, u, l, x);
+    nc8(p, u);
+    if (t + 1 < t_end) nc8(p + S * kPprU, u2);
+    ppr_contrib8<VL>(a, u, lc, x);
     CVal acc[VL];
 #pragma unroll
     for (int q = 0; q < VL; ++q) acc[q] = CVal{0.f, 0.f};
-    bool open = true;  // the piece's last edge does not end its row
-    for (int e = e0;; e += kPprU) {
-      const uint32_t ends = (word >> (e & 31)) & 0xFFu;
-      const bool more = end - e > kPprU;
+    for (;;) {
+      const bool more = t + 1 < t_end;
       if (more) {
 #pragma unroll
         for (int j = 0; j < kPprU; ++j) u[j] = u2[j];
-        if (end - e > 2 * kPprU) ppr_src8(a, e + 2 * kPprU, end, u2);
-        ppr_contrib8<VL>(a, u, l, y);
-        if ((e & 31) == 32 - kPprU) {
-          word = word2;
-          if (((end - 1) >> 5) > ((e + kPprU) >> 5))
-            word2 = __ldg(a.row_bits + ((e + kPprU) >> 5) + 1);
-        }
+        if (t + 2 < t_end) nc8(p + 2 * S * kPprU, u2);
+        ppr_contrib8<VL>(a, u, lc, y);
       }
-      if (!ends) {
+      if (t + 1 < next) {  // warp-uniform
 #pragma unroll
         for (int q = 0; q < VL; ++q) {
-          const float g = __fadd_rn(
+          const float h = __fadd_rn(
               __fadd_rn(__fadd_rn(x[0].f[q], x[1].f[q]), __fadd_rn(x[2].f[q], x[3].f[q])),
               __fadd_rn(__fadd_rn(x[4].f[q], x[5].f[q]), __fadd_rn(x[6].f[q], x[7].f[q])));
-          acc[q] = two_sum_add(acc[q], CVal{g, 0.f});
+          acc[q] = two_sum_add(acc[q], CVal{h, 0.f});
         }
       } else {
 #pragma unroll
-        for (int j = 0; j < kPprU; ++j) {
+        for (int j = 0; j < kPprU; ++j)
 #pragma unroll
           for (int q = 0; q < VL; ++q) acc[q] = two_sum_add(acc[q], CVal{x[j].f[q], 0.f});
-          if ((ends >> j) & 1u) {
-            if (cont) {
+        if (on && dst >= 0) {
+          Lanes<VL> o;
 #pragma unroll
-              for (int q = 0; q < VL; ++q) a.head[(size_t)k * a.L + l + q] = acc[q];
-            } else {
-              Lanes<VL> o;
+          for (int q = 0; q < VL; ++q) o.f[q] = __fadd_rn(acc[q].s, acc[q].c);
+          ppr_st<VL>(a.sum + (size_t)dst * a.L + l, o);
+        } else if (on && dst != INT_MIN) {
 #pragma unroll
-              for (int q = 0; q < VL; ++q) o.f[q] = __fadd_rn(acc[q].s, acc[q].c);
-              ppr_st<VL>(a.sum + (size_t)r * a.L + l, o);
-            }
-            cont = false;
-            ++r;
+          for (int q = 0; q < VL; ++q) a.partial[(size_t)~dst * a.L + l + q] = acc[q];
+        }
 #pragma unroll
-            for (int q = 0; q < VL; ++q) acc[q] = CVal{0.f, 0.f};
-          }
+        for (int q = 0; q < VL; ++q) acc[q] = CVal{0.f, 0.f};
+        ++s;
+        next = next2;
+        dst = dst2;
+        if (s + 1 < s_end) {
+          next2 = __ldg(a.step_off + s + 2);
+          dst2 = __ldg(a.unit_dst + (size_t)(s + 1) * S + g);
         }
       }
-      if (!more) {
-        open = !((ends >> (end - 1 - e)) & 1u);
-        break;
-      }
+      if (!more) break;
 #pragma unroll
       for (int j = 0; j < kPprU; ++j) x[j] = y[j];
-    }
-    if (open) {
-      CVal *to = (cont ? a.head : a.tail) + (size_t)k * a.L + l;
-#pragma unroll
-      for (int q = 0; q < VL; ++q) to[q] = acc[q];
+      ++t;
+      p += S * kPprU;
     }
   }
 }
@@ -1114,38 +1095,37 @@ __device__ __forceinline__ Partials<VL> ppr_partials(const CVal *p) {
   return o;
 }
 
-// Rows cut by piece boundaries, their partials folded in a fixed order: a
-// group per row, or the whole CTA (every group a strided share, then the
-// groups' sums) for rows over more than kPprLong pieces -- one group folding
-// a hub's 1,200 partials one after the other took 90 us.  Nearly every piece
-// cuts a row and nearly every cut row ends in the next piece, so its two
-// partials are loaded with the row's number, not after it.
+// Rows of several units, their partials folded in a fixed order: a group per
+// row, or the whole CTA (every group a strided share, then the groups' sums)
+// for rows of more than kPprLong units -- one group folding a hub's 1,200
+// partials one after the other took 90 us.  Rows next to one another go to
+// different CTAs: hubs have neighbouring ids, and a CTA folds its hubs one
+// after the other.
 template <int VL>
 __global__ void __launch_bounds__(kNT) k_ppr_fix(PprArgs a) {
   __shared__ Partials<VL> s_part[kNT];
-  __shared__ int s_last[kNT];
+  __shared__ int s_end[kNT];
   const int T = a.G / VL;
   const int l = threadIdx.x % T * VL, g = threadIdx.x / T, groups = kNT / T;
   const bool on = l < a.L;
-  for (int k0 = blockIdx.x * groups; k0 < a.n_pieces; k0 += gridDim.x * groups) {
-    const int k = k0 + g;
-    int r = -1, last = -1;
-    Partials<VL> acc, next;
-    if (k < a.n_pieces) {
-      r = __ldg(a.split_row + k);
-      last = __ldg(a.split_last + k);
-      if (on) {
-        acc = ppr_partials<VL>(a.tail + (size_t)k * a.L + l);
-        next = ppr_partials<VL>(a.head + (size_t)min(k + 1, a.n_pieces - 1) * a.L + l);
-      }
+  for (int k0 = blockIdx.x; k0 < a.n_long; k0 += gridDim.x * groups) {
+    const int k = k0 + g * gridDim.x;
+    int r = -1, b = 0, e = 0;
+    if (k < a.n_long) {
+      r = __ldg(a.long_row + k);
+      b = __ldg(a.long_slot + k);
+      e = __ldg(a.long_slot + k + 1);
     }
-    const bool lng = r >= 0 && last - k > kPprLong;
+    const bool lng = e - b > kPprLong;
+    Partials<VL> acc, next;
+#pragma unroll
+    for (int i = 0; i < VL; ++i) acc.p[i] = CVal{0.f, 0.f};
     if (r >= 0 && !lng && on) {
-      for (int q = k + 1;; ++q) {
+#pragma unroll 2
+      for (int q = b; q < e; ++q) {
+        next = ppr_partials<VL>(a.partial + (size_t)q * a.L + l);
 #pragma unroll
         for (int i = 0; i < VL; ++i) acc.p[i] = two_sum_add(acc.p[i], next.p[i]);
-        if (q == last) break;
-        next = ppr_partials<VL>(a.head + (size_t)(q + 1) * a.L + l);
       }
       Lanes<VL> o;
 #pragma unroll
@@ -1153,18 +1133,19 @@ __global__ void __launch_bounds__(kNT) k_ppr_fix(PprArgs a) {
       ppr_st<VL>(a.sum + (size_t)r * a.L + l, o);
     }
     if (!__syncthreads_or(lng)) continue;  // CTA-uniform
-    if (l == 0) s_last[g] = lng ? last : -1;
+    if (l == 0) s_end[g] = lng ? e : -1;
     __syncthreads();
     for (int h = 0; h < groups; ++h) {
-      const int hl = s_last[h];
-      if (hl < 0) continue;  // CTA-uniform
-      const int kh = k0 + h;
+      const int he = s_end[h];
+      if (he < 0) continue;  // CTA-uniform
+      const int kh = k0 + h * gridDim.x;
+      const int hb = __ldg(a.long_slot + kh);
 #pragma unroll
       for (int i = 0; i < VL; ++i) acc.p[i] = CVal{0.f, 0.f};
       if (on)
 #pragma unroll 4
-        for (int q = kh + 1 + g; q <= hl; q += groups) {
-          next = ppr_partials<VL>(a.head + (size_t)q * a.L + l);
+        for (int q = hb + g; q < he; q += groups) {
+          next = ppr_partials<VL>(a.partial + (size_t)q * a.L + l);
 #pragma unroll
           for (int i = 0; i < VL; ++i) acc.p[i] = two_sum_add(acc.p[i], next.p[i]);
         }
@@ -1180,14 +1161,11 @@ __global__ void __launch_bounds__(kNT) k_ppr_fix(PprArgs a) {
         __syncthreads();
       }
       if (g == 0 && on) {
-        const Partials<VL> t = ppr_partials<VL>(a.tail + (size_t)kh * a.L + l);
         Lanes<VL> o;
 #pragma unroll
-        for (int i = 0; i < VL; ++i) {
-          const CVal c = two_sum_add(t.p[i], s_part[threadIdx.x].p[i]);
-          o.f[i] = __fadd_rn(c.s, c.c);
-        }
-        ppr_st<VL>(a.sum + (size_t)__ldg(a.split_row + kh) * a.L + l, o);
+        for (int i = 0; i < VL; ++i)
+          o.f[i] = __fadd_rn(s_part[threadIdx.x].p[i].s, s_part[threadIdx.x].p[i].c);
+        ppr_st<VL>(a.sum + (size_t)__ldg(a.long_row + kh) * a.L + l, o);
       }
       __syncthreads();
     }
@@ -1330,40 +1308,141 @@ __global__ void __launch_bounds__(kNT)
   }
 }
 
-// The plan, once per piece size: a bit at every row's last in-edge ...
-__global__ void k_ppr_row_bits(const int32_t *ne_end, int n_ne, uint32_t *bits) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n_ne; r += gridDim.x * blockDim.x) {
-    const int e = ne_end[r] - 1;
-    atomicOr(bits + (e >> 5), 1u << (e & 31));
+// The plan's kernels, in order.  Units of each row, and the rows of several.
+__global__ void k_plan_count(const int32_t *ne_end, int n_ne, int32_t *units, int32_t *slots,
+                             int32_t *longs) {
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r <= n_ne; r += gridDim.x * blockDim.x) {
+    int n = 0;
+    if (r < n_ne) n = (ne_end[r] - (r > 0 ? ne_end[r - 1] : 0) + kPprUnit - 1) / kPprUnit;
+    units[r] = n;
+    slots[r] = n > 1 ? n : 0;
+    longs[r] = n > 1 ? 1 : 0;
   }
 }
 
-// The row of in-edge e: the first whose end is past it.
-__device__ __forceinline__ int ppr_row_of(const int32_t *ne_end, int n_ne, int e) {
-  int lo = 0, hi = n_ne;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (ne_end[mid] <= e)
-      lo = mid + 1;
-    else
-      hi = mid;
+// (After scans of the three.)  The units' rows; the long rows.
+__global__ void k_plan_units(const int32_t *units, const int32_t *slots, const int32_t *longs,
+                             int n_ne, int32_t *unit_row, int32_t *long_row, int32_t *long_slot) {
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r <= n_ne; r += gridDim.x * blockDim.x) {
+    if (r == n_ne) {
+      long_slot[longs[r]] = slots[r];
+      break;
+    }
+    const int b = units[r], e = units[r + 1];
+    for (int u = b; u < e; ++u) unit_row[u] = r;
+    if (e - b > 1) {
+      long_row[longs[r]] = r;
+      long_slot[longs[r]] = slots[r];
+    }
   }
-  return lo;
 }
 
-// ... and the pieces' first rows and the rows they cut.
-__global__ void k_ppr_plan(const int32_t *ne_end, int n_ne, int n_pieces, int P, int E,
-                           int32_t *first_row, int32_t *split_row, int32_t *split_last) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n_pieces;
+// A window's units in order of their steps (stable): (first edge, edges) and
+// destination of every place.
+__global__ void __launch_bounds__(kNT)
+    k_plan_sort(const int32_t *ne_end, const int32_t *units, const int32_t *slots,
+                const int32_t *unit_row, int U, int2 *place, int32_t *unit_dst) {
+  constexpr int kSteps = kPprUnit / kPprU;   // 1 .. 16
+  constexpr int kItems = kPprWindow / kNT;   // consecutive units of a thread
+  __shared__ int cnt[kSteps][kNT];
+  __shared__ int tot[kSteps];
+  const int t = threadIdx.x, u0 = blockIdx.x * kPprWindow;
+  int2 at[kItems];
+  int dst[kItems], key[kItems];
+#pragma unroll
+  for (int j = 0; j < kSteps; ++j) cnt[j][t] = 0;
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    const int u = u0 + t * kItems + i;
+    key[i] = -1;
+    if (u < U) {
+      const int r = unit_row[u], c = u - units[r], n = units[r + 1] - units[r];
+      const int e0 = (r > 0 ? ne_end[r - 1] : 0) + c * kPprUnit;
+      const int len = min(kPprUnit, ne_end[r] - e0);
+      at[i] = make_int2(e0, len);
+      dst[i] = n == 1 ? r : ~(slots[r] + c);
+      key[i] = (len + kPprU - 1) / kPprU - 1;
+      ++cnt[key[i]][t];
+    }
+  }
+  __syncthreads();
+  // exclusive scan in (key, thread) order: a warp scans two keys
+  const int lane = t & 31, warp = t >> 5;
+  for (int k = warp; k < kSteps; k += kNT / 32) {
+    int run = 0;
+    for (int b = 0; b < kNT; b += 32) {
+      const int x = cnt[k][b + lane];
+      int incl = x;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += o;
+      }
+      cnt[k][b + lane] = run + incl - x;
+      run += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) tot[k] = run;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    if (key[i] < 0) continue;
+    int pos = u0 + cnt[key[i]][t]++;
+    for (int k = 0; k < key[i]; ++k) pos += tot[k];
+    place[pos] = at[i];
+    unit_dst[pos] = dst[i];
+  }
+}
+
+// Steps of every slice of S units (the longest's).
+__global__ void k_plan_steps(const int2 *place, int U, int S, int n_slices, int32_t *step_off) {
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s <= n_slices;
+       s += gridDim.x * blockDim.x) {
+    int m = 0;
+    if (s < n_slices)
+      for (int g = 0; g < S && s * S + g < U; ++g) m = max(m, place[s * S + g].y);
+    step_off[s] = (m + kPprU - 1) / kPprU;
+  }
+}
+
+// (After a scan of the steps.)  The sources in walking order, a warp per
+// slice; places past the last unit have no destination.
+__global__ void __launch_bounds__(kNT)
+    k_plan_index(const int2 *place, const int32_t *step_off, const int32_t *csc_src, int U, int S,
+                 int n_slices, int nV, int32_t *idx, int32_t *unit_dst) {
+  const int lane = threadIdx.x & 31, nwarps = (int)((gridDim.x * kNT) >> 5);
+  for (int s = (int)((blockIdx.x * kNT + threadIdx.x) >> 5); s < n_slices; s += nwarps) {
+    const int t0 = step_off[s], t1 = step_off[s + 1];
+    const int n = (t1 - t0) * S * kPprU;
+    for (int i = lane; i < n; i += 32) {
+      const int step = i / (S * kPprU), g = i / kPprU % S, j = i % kPprU;
+      int v = nV;
+      if (s * S + g < U) {
+        const int2 p = place[s * S + g];
+        const int e = step * kPprU + j;
+        if (e < p.y) v = csc_src[p.x + e];
+      }
+      idx[(size_t)t0 * S * kPprU + i] = v;
+    }
+    if (lane < S && s * S + lane >= U) unit_dst[s * S + lane] = INT_MIN;
+  }
+}
+
+// The first slice of every piece of `steps` steps.
+__global__ void k_plan_pieces(const int32_t *step_off, int n_slices, int n_pieces, int steps,
+                              int32_t *piece_start) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k <= n_pieces;
        k += gridDim.x * blockDim.x) {
-    const int e0 = k * P;
-    const int end = E - e0 < P ? E : e0 + P;
-    first_row[k] = ppr_row_of(ne_end, n_ne, e0);
-    const int r = ppr_row_of(ne_end, n_ne, end - 1);
-    const int row_start = r > 0 ? ne_end[r - 1] : 0, row_end = ne_end[r];
-    const bool cut = row_start >= e0 && row_end > end;
-    split_row[k] = cut ? r : -1;
-    split_last[k] = cut ? (row_end - 1) / P : -1;
+    const long long want = (long long)k * steps;
+    int lo = 0, hi = n_slices;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (step_off[mid] < want)
+        lo = mid + 1;
+      else
+        hi = mid;
+    }
+    piece_start[k] = lo;
   }
 }
 
@@ -1379,6 +1458,7 @@ __global__ void k_ppr_seed(const int32_t *seeds, const BatchParams *prm, int L,
 __global__ void k_ppr_init(const uint32_t *seed_mask, const int32_t *csr_off, int nV, int L,
                            float *rank, float *contrib) {
   const size_t n = (size_t)nV * L;
+  if (blockIdx.x == 0 && threadIdx.x < L) contrib[n + threadIdx.x] = 0.f;  // the plan's padding
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n;
        k += (size_t)gridDim.x * blockDim.x) {
     const int v = (int)(k / L), l = (int)(k % L);
@@ -1432,16 +1512,20 @@ struct gas_batch {
   int32_t dist_ls = 0, sssp_srcs_cap = 0;
   // the arrays above and below by what allocates them: the frontier, the SSSP
   // rows, the BFS state, the PPR rows and plan
-  DeviceGroup frontier_mem, dist_mem, bfs_mem, ppr_mem, plan_mem;
+  DeviceGroup frontier_mem, dist_mem, bfs_mem, ppr_mem, plan_mem, piece_mem;
   // profiling of the SSSP pushes (direct launches, events around each push)
   bool profiling = false;
   cudaEvent_t pev[2] = {nullptr, nullptr};
   gas_kernel_profile prof{};
   // PPR
-  int32_t *first_row = nullptr, *split_row = nullptr, *split_last = nullptr;
-  CVal *head = nullptr, *tail = nullptr;
+  // the gather's plan (plan_mem), for slices of plan_S units, and its pieces
+  // (piece_mem) of piece_edges edges per group
+  int32_t *pp_idx = nullptr, *pp_step_off = nullptr, *pp_unit_dst = nullptr,
+          *pp_long_row = nullptr, *pp_long_slot = nullptr, *pp_piece_start = nullptr;
+  CVal *partial = nullptr;
+  int32_t plan_S = 0, n_slices = 0, n_steps = 0, n_long = 0, n_slots = 0;
   float *rank = nullptr, *contrib = nullptr, *sum = nullptr;
-  uint32_t *seed_mask = nullptr, *row_bits = nullptr;
+  uint32_t *seed_mask = nullptr;
   int32_t *seeds = nullptr;
   double *l1 = nullptr;
   unsigned int *ticket = nullptr;
@@ -1473,21 +1557,21 @@ void free_state(gas_batch *b) {
   b->bfs_mem.free();
   b->ppr_mem.free();
   b->plan_mem.free();
+  b->piece_mem.free();
   bfree(b->depth); bfree(b->srcs);
-  bfree(b->seed_mask); bfree(b->seeds); bfree(b->l1); bfree(b->ticket); bfree(b->row_bits);
+  bfree(b->seed_mask); bfree(b->seeds); bfree(b->l1); bfree(b->ticket);
   bfree(b->sssp_srcs); bfree(b->lane_rounds);
   bfree(b->lanes_active);
   b->dist_ls = b->sssp_srcs_cap = 0;
-  b->n_pieces = b->piece_edges = b->ppr_lanes = b->depth_lanes = 0;
+  b->n_pieces = b->piece_edges = b->ppr_lanes = b->depth_lanes = b->plan_S = 0;
   b->srcs_cap = b->l1_cap = b->seeds_cap = 0;
 }
 
-// Lanes per thread of the PPR kernels (four: 16-byte loads).  A walk of 8
-// pieces per warp beats one of 2 although their row ends diverge: 16 graphs,
-// 16 lanes 16.9 ms per run with 4 lanes a thread, 17.8 with 2, 22.7 with 1;
-// 4 lanes 2.53 / 2.75 / 2.92.  Two lanes go one to a thread (2.25 ms against
-// 2.49).
-int ppr_vl(int L) { return L % 4 == 0 ? 4 : L % 2 == 0 && L > 2 ? 2 : 1; }
+// Lanes per thread of the PPR kernels: four (16-byte loads) from 12 lanes up,
+// two below, where a warp of 16 or 32 groups has too few rows in flight per
+// register (per run, 1 / 2 / 4 lanes a thread: 16 lanes - / 11.7 / 9.9 ms, 8
+// lanes - / 3.1 / 3.5, 4 lanes - / 2.2 / 2.6).  Two lanes go one to a thread.
+int ppr_vl(int L) { return L % 4 == 0 && L > 8 ? 4 : L % 2 == 0 && L > 2 ? 2 : 1; }
 
 int lane_group(int L) {
   int g = 1;
@@ -1580,22 +1664,108 @@ gas_status_t ensure_bfs(gas_batch *b, int lanes, int n_sources) {
   return GAS_OK;
 }
 
-// Ranks, contributions and row sums of the lanes; pieces of P edges over the
-// CSC (P rounded up to whole steps of the gather), their first rows and the
-// rows they cut.
+// The gather's plan for slices of S units; reads three counts back, so it
+// waits for the stream.
+gas_status_t build_ppr_plan(gas_batch *b, int S, cudaStream_t s) {
+  gas_engine *e = b->eng;
+  const int n_ne = e->n_ne, grid = 8 * e->num_sms;
+  b->plan_S = 0;
+  b->plan_mem.free();
+  DeviceGroup tmp, tmp2;
+  struct Guard {
+    DeviceGroup &a, &b;
+    ~Guard() { a.free(); b.free(); }
+  } guard{tmp, tmp2};
+  int32_t *units = nullptr, *slots = nullptr, *longs = nullptr, *part = nullptr;
+  CUDA_TRY(tmp.alloc({GROUP_PART(units, ((size_t)n_ne + 1) * 4),
+                      GROUP_PART(slots, ((size_t)n_ne + 1) * 4),
+                      GROUP_PART(longs, ((size_t)n_ne + 1) * 4),
+                      GROUP_PART(part, (size_t)gas::device_scan_parts(n_ne + 1) * 4)}));
+  k_plan_count<<<grid, 256, 0, s>>>(e->ne_end, n_ne, units, slots, longs);
+  CUDA_TRY(cudaGetLastError());
+  int32_t total[3];  // units, partial slots, long rows
+  int32_t *scanned[3] = {units, slots, longs};
+  for (int i = 0; i < 3; ++i) {
+    GAS_TRY(gas::device_scan_excl(scanned[i], n_ne + 1, part, s));
+    CUDA_TRY(cudaMemcpyAsync(&total[i], scanned[i] + n_ne, 4, cudaMemcpyDeviceToHost, s));
+  }
+  CUDA_TRY(cudaStreamSynchronize(s));
+  const int U = total[0], n_slices = (int)(((long long)U + S - 1) / S);
+  int32_t *unit_row = nullptr, *spart = nullptr, *steps = nullptr;
+  int2 *place = nullptr;
+  CUDA_TRY(tmp2.alloc({GROUP_PART(unit_row, (size_t)U * 4), GROUP_PART(place, (size_t)U * 8),
+                       GROUP_PART(steps, ((size_t)n_slices + 1) * 4),
+                       GROUP_PART(spart, (size_t)gas::device_scan_parts(n_slices + 1) * 4)}));
+  // the destinations are made with the places and the number of steps known
+  // after them: two groups, the long rows with the first
+  int32_t *unit_dst = nullptr, *long_row = nullptr, *long_slot = nullptr;
+  DeviceGroup dests;
+  struct Guard1 {
+    DeviceGroup &a;
+    ~Guard1() { a.free(); }
+  } guard1{dests};
+  CUDA_TRY(dests.alloc({GROUP_PART(unit_dst, (size_t)n_slices * S * 4),
+                        GROUP_PART(long_row, (size_t)total[2] * 4),
+                        GROUP_PART(long_slot, ((size_t)total[2] + 1) * 4)}));
+  k_plan_units<<<grid, 256, 0, s>>>(units, slots, longs, n_ne, unit_row, long_row, long_slot);
+  if (U > 0)
+    k_plan_sort<<<(U + kPprWindow - 1) / kPprWindow, kNT, 0, s>>>(e->ne_end, units, slots,
+                                                                unit_row, U, place, unit_dst);
+  k_plan_steps<<<grid, 256, 0, s>>>(place, U, S, n_slices, steps);
+  CUDA_TRY(cudaGetLastError());
+  GAS_TRY(gas::device_scan_excl(steps, n_slices + 1, spart, s));
+  int32_t n_steps = 0;
+  CUDA_TRY(cudaMemcpyAsync(&n_steps, steps + n_slices, 4, cudaMemcpyDeviceToHost, s));
+  CUDA_TRY(cudaStreamSynchronize(s));
+  CUDA_TRY(b->plan_mem.alloc(
+      {GROUP_PART(b->pp_idx, (size_t)n_steps * S * kPprU * 4),
+       GROUP_PART(b->pp_step_off, ((size_t)n_slices + 1) * 4),
+       GROUP_PART(b->pp_unit_dst, (size_t)n_slices * S * 4),
+       GROUP_PART(b->pp_long_row, (size_t)total[2] * 4),
+       GROUP_PART(b->pp_long_slot, ((size_t)total[2] + 1) * 4)}));
+  if (n_slices > 0)
+    k_plan_index<<<grid, kNT, 0, s>>>(place, steps, e->csc_src, U, S, n_slices, e->nV, b->pp_idx,
+                                     unit_dst);
+  CUDA_TRY(cudaGetLastError());
+  const struct {
+    int32_t *to, *from;
+    size_t n;
+  } keep[] = {{b->pp_step_off, steps, (size_t)n_slices + 1},
+              {b->pp_unit_dst, unit_dst, (size_t)n_slices * S},
+              {b->pp_long_row, long_row, (size_t)total[2]},
+              {b->pp_long_slot, long_slot, (size_t)total[2] + 1}};
+  for (const auto &k : keep)
+    if (k.n) CUDA_TRY(cudaMemcpyAsync(k.to, k.from, k.n * 4, cudaMemcpyDeviceToDevice, s));
+  CUDA_TRY(cudaStreamSynchronize(s));  // the scratch is freed at return
+  b->n_slices = n_slices;
+  b->n_steps = n_steps;
+  b->n_slots = total[1];
+  b->n_long = total[2];
+  b->plan_S = S;
+  return GAS_OK;
+}
+
+// Ranks, contributions and row sums of the lanes; the gather's plan for their
+// groups and its pieces of P edges per group.
 gas_status_t ensure_ppr(gas_batch *b, int lanes, int P, int n_seeds, int grid_rows,
                         cudaStream_t s) {
   gas_engine *e = b->eng;
   const size_t nV = std::max(1, e->nV), n_ne = std::max(1, e->n_ne);
-  const size_t nE = std::max(1, e->nE);
+  const int G = lane_group(lanes), S = 32 / (G / ppr_vl(lanes));
+  if (b->plan_S != S) {
+    drop_graph(b);
+    b->ppr_lanes = 0;  // the partials are sized by the plan
+    GAS_TRY(build_ppr_plan(b, S, s));
+  }
   if (b->ppr_lanes != lanes) {
     drop_graph(b);
     b->ppr_lanes = 0;
     const size_t row = (size_t)lanes * 4;
-    CUDA_TRY(b->ppr_mem.alloc({GROUP_PART(b->rank, nV * row), GROUP_PART(b->contrib, nV * row),
-                               GROUP_PART(b->sum, n_ne * row)}));
+    CUDA_TRY(b->ppr_mem.alloc({GROUP_PART(b->rank, nV * row), GROUP_PART(b->contrib, (nV + 1) * row),
+                               GROUP_PART(b->sum, n_ne * row),
+                               GROUP_PART(b->partial, (size_t)b->n_slots * lanes * sizeof(CVal))}));
     b->ppr_lanes = lanes;
-    b->piece_edges = 0;  // head/tail are sized by lanes
+    b->piece_edges = 0;
   }
   if (!b->seed_mask) CUDA_TRY(cudaMalloc(&b->seed_mask, nV * 4));
   if (!b->ticket) {
@@ -1609,7 +1779,6 @@ gas_status_t ensure_ppr(gas_batch *b, int lanes, int P, int n_seeds, int grid_ro
     CUDA_TRY(cudaMalloc(&b->seeds, (size_t)n_seeds * 4));
     b->seeds_cap = n_seeds;
   }
-  const int G = lane_group(lanes);
   const int need_l1 = grid_rows * G;
   if (b->l1_cap < need_l1) {
     drop_graph(b);
@@ -1618,25 +1787,14 @@ gas_status_t ensure_ppr(gas_batch *b, int lanes, int P, int n_seeds, int grid_ro
     CUDA_TRY(cudaMalloc(&b->l1, (size_t)need_l1 * sizeof(double)));
     b->l1_cap = need_l1;
   }
-  if (!b->row_bits) {
-    const size_t words = (nE + 31) / 32;
-    CUDA_TRY(cudaMalloc(&b->row_bits, words * 4));
-    CUDA_TRY(cudaMemsetAsync(b->row_bits, 0, words * 4, s));
-    k_ppr_row_bits<<<8 * e->num_sms, 256, 0, s>>>(e->ne_end, e->n_ne, b->row_bits);
-    CUDA_TRY(cudaGetLastError());
-  }
   if (b->piece_edges == P) return GAS_OK;
   drop_graph(b);
   b->piece_edges = 0;
-  const int Pu = (P + kPprU - 1) / kPprU * kPprU;
-  const int32_t n_pieces = (int32_t)(((int64_t)e->nE + Pu - 1) / Pu);
-  const size_t np = std::max(1, n_pieces);
-  CUDA_TRY(b->plan_mem.alloc(
-      {GROUP_PART(b->first_row, np * 4), GROUP_PART(b->split_row, np * 4),
-       GROUP_PART(b->split_last, np * 4), GROUP_PART(b->head, np * lanes * sizeof(CVal)),
-       GROUP_PART(b->tail, np * lanes * sizeof(CVal))}));
-  k_ppr_plan<<<8 * e->num_sms, 256, 0, s>>>(e->ne_end, e->n_ne, n_pieces, Pu, e->nE,
-                                           b->first_row, b->split_row, b->split_last);
+  const int steps = (P + kPprU - 1) / kPprU;
+  const int n_pieces = (int)(((long long)b->n_steps + steps - 1) / steps);
+  CUDA_TRY(b->piece_mem.alloc({GROUP_PART(b->pp_piece_start, ((size_t)n_pieces + 1) * 4)}));
+  k_plan_pieces<<<8 * e->num_sms, 256, 0, s>>>(b->pp_step_off, b->n_slices, n_pieces, steps,
+                                              b->pp_piece_start);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaStreamSynchronize(s));  // the plan outlives this call and its stream
   b->n_pieces = n_pieces;
@@ -1654,24 +1812,22 @@ struct RunCtx {
 PprArgs ppr_args(gas_batch *b, int lanes) {
   gas_engine *e = b->eng;
   PprArgs a;
-  a.csc_src = e->csc_src;
   a.csc_off = e->csc_off;
   a.csr_off = e->csr_off;
   a.ne_vid = e->ne_vid;
-  a.ne_end = e->ne_end;
-  a.row_bits = b->row_bits;
-  a.first_row = b->first_row;
-  a.split_row = b->split_row;
-  a.split_last = b->split_last;
+  a.idx = b->pp_idx;
+  a.step_off = b->pp_step_off;
+  a.unit_dst = b->pp_unit_dst;
+  a.piece_start = b->pp_piece_start;
+  a.long_row = b->pp_long_row;
+  a.long_slot = b->pp_long_slot;
   a.n_pieces = b->n_pieces;
-  a.P = (b->piece_edges + kPprU - 1) / kPprU * kPprU;
-  a.E = e->nE;
+  a.n_long = b->n_long;
   a.L = lanes;
   a.G = lane_group(lanes);
   a.n_ne = e->n_ne;
   a.nV = e->nV;
-  a.head = b->head;
-  a.tail = b->tail;
+  a.partial = b->partial;
   a.sum = b->sum;
   a.rank = b->rank;
   a.contrib = b->contrib;
@@ -1879,7 +2035,7 @@ gas_status_t ppr_prologue(RunCtx *c, cudaStream_t s, cudaGraphConditionalHandle 
 
 template <int VL>
 gas_status_t ppr_step(RunCtx *c, cudaStream_t s, cudaGraphConditionalHandle h, int ig) {
-  k_ppr_pieces<VL><<<c->grid_pieces, kNT, 0, s>>>(c->ppr);
+  k_ppr_units<VL><<<c->grid_pieces, kNT, 0, s>>>(c->ppr);
   k_ppr_fix<VL><<<c->grid_fix, kNT, 0, s>>>(c->ppr);
   k_ppr_rows<VL><<<c->grid_rows, kNT, 0, s>>>(c->ppr, h, ig);
   CUDA_TRY(cudaGetLastError());
@@ -1990,7 +2146,7 @@ gas_status_t run_direct(RunCtx *c, const Loop *loops, const int *which, int n, c
 template <int VL>
 void ppr_grids(const gas_engine *e, RunCtx *c) {
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ppr_pieces<VL>, kNT, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ppr_units<VL>, kNT, 0);
   c->grid_pieces = e->num_sms * (per_sm > 0 ? per_sm : 1);
   per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ppr_fix<VL>, kNT, 0);
@@ -2049,8 +2205,8 @@ gas_status_t check_job(const gas_batch *b, const gas_batch_job *j) {
 }
 
 // Untuned piece size: 256, halved down to 64 while there would be fewer than
-// 1.5 pieces per resident group (16 lanes on 600 K edges: 64 takes 0.87 ms
-// per run, 256 1.37; on 64 M edges 19.4 and 16.9).
+// 1.5 pieces per resident group (16 lanes on 600 K edges: 64 takes 0.74 ms
+// per run, 256 0.96; on 64 M edges 11.3 and 10.0).
 int default_piece(const gas_batch *b, const RunCtx &c) {
   if (b->tuned_piece > 0) return b->tuned_piece;
   const int L = std::max(1, c.ppr_lanes);

@@ -339,7 +339,7 @@ struct Scratch {
 
 gas_status_t scan_excl(int32_t *a, int n, int32_t *part, cudaStream_t s) {
   if (n <= 0) return GAS_OK;
-  const int nb = (n + kScanTile - 1) / kScanTile;
+  const int nb = (int)(((long long)n + kScanTile - 1) / kScanTile);
   k_scan_reduce<<<nb, kRThreads, 0, s>>>(a, n, part);
   k_scan_spine<<<1, kRThreads, 0, s>>>(part, nb);
   k_scan_down<<<nb, kRThreads, 0, s>>>(a, n, part);
@@ -473,6 +473,12 @@ gas_status_t build_graph_device(gas_engine *e, const int32_t *srcs, const int32_
   CUDA_TRY(cudaStreamSynchronize(s));  // the work buffers are freed at return
   return GAS_OK;
 }
+
+gas_status_t device_scan_excl(int32_t *a, int n, int32_t *part, void *stream) {
+  return scan_excl(a, n, part, S(stream));
+}
+
+int device_scan_parts(int n) { return (int)(((long long)n + kScanTile - 1) / kScanTile) + 1; }
 
 gas_status_t build_ne_rows(gas_engine *e, int32_t *part, int32_t *n_out, void *stream) {
   const int nb = ne_blocks(e->nV);

@@ -228,6 +228,10 @@ gas_status_t build_graph_device(gas_engine *e, const int32_t *srcs, const int32_
 // word n_out); part: ne_blocks(nV) words of scratch.
 gas_status_t build_ne_rows(gas_engine *e, int32_t *part, int32_t *n_out, void *stream);
 int ne_blocks(int nV);
+// Exclusive scan of n device ints in place; part: device_scan_parts(n) ints of
+// scratch.
+gas_status_t device_scan_excl(int32_t *a, int n, int32_t *part, void *stream);
+int device_scan_parts(int n);
 // Whether set_graph builds on the device: GAS_GRAPH_BUILD=host|device, else
 // from 16,384 edges up.
 bool device_build_for(int64_t n_edges);

@@ -1,6 +1,6 @@
-"""Batched personalized PageRank on rows cut by pieces: hubs over more pieces
+"""Batched personalized PageRank on rows of several units: hubs over more units
 than one group folds (16) and than a CTA has groups, rows ending exactly at a
-piece's or a step's (8 in-edges) end, an edge count that is no multiple of 8,
+unit's (128 in-edges) or a step's (8) end, an edge count that is no multiple of 8,
 every vector width of the lanes, a graph without edges."""
 import numpy as np
 import pytest
