@@ -12,8 +12,7 @@ namespace gasfeat {
 
 // Degree-histogram bucket of a frontier vertex with out-degree d >= 1.
 __host__ __device__ inline int degree_bucket(int d) {
-  int l = 0;
-  while ((d >> (l + 1)) > 0 && l < 30) ++l;  // floor(log2 d)
+  const int l = 31 - __builtin_clz((unsigned)d);  // floor(log2 d)
   const int b = l / 2;
   return b < 7 ? b : 7;
 }
