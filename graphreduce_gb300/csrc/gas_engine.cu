@@ -27,6 +27,7 @@
 #include "gas_device.cuh"
 #include "gas_internal.h"
 #include "gas_engine_impl.h"
+#include "gas_sched.h"
 
 // ---------------------------------------------------------------------------
 // errors
@@ -639,8 +640,8 @@ void free_graph(gas_engine *e) {
   for (int i = 0; i < 2; ++i) { dfree(e->pr_rank[i]); dfree(e->pr_contrib[i]); }
   dfree(e->pr_seed); dfree(e->pr_inv_deg); dfree(e->pr_l1); dfree(e->csr_to_csc);
   dfree(e->pr_tile_row); dfree(e->pr_head); dfree(e->pr_tail);
-  dfree(e->sb_bits); dfree(e->sb_ctl); dfree(e->sb_heavy);
-  dfree(e->sm_vals); dfree(e->sm_queue); dfree(e->sm_ctl);
+  e->sb_mem.free();
+  e->sm_mem.free();
   e->sb_clean = e->sm_clean = false;
   e->pr_tile_cap = 0;
   e->h_csr_perm.clear();
@@ -1024,6 +1025,20 @@ gas_status_t gas_engine_set_graph(gas_engine *e, int32_t nV, void *vertex_data,
   plan.add(&e->trace, GAS_TRACE_CAP);
   plan.add(&e->hist, 8);
   plan.add(&e->ne_scratch, (size_t)gas::ne_blocks(nV) + 1);
+  if (!e->graph_only && !e->edges_on_host) {
+    const gas::SmallBytes sb = gas::bfs_small_bytes(nV, nE), sm = gas::min_small_bytes(nV, nE);
+    if (e->prog == GAS_PROG_BFS && sb.all() <= gas::kSmallWithGraph) {
+      plan.add((uint8_t **)&e->sb_bits, sb.values);
+      plan.add((uint8_t **)&e->sb_ctl, sb.ctl);
+      plan.add((uint8_t **)&e->sb_queue, sb.queues);
+    }
+    if ((e->prog == GAS_PROG_SSSP || e->prog == GAS_PROG_CC) &&
+        sm.all() <= gas::kSmallWithGraph) {
+      plan.add((uint8_t **)&e->sm_vals, sm.values);
+      plan.add((uint8_t **)&e->sm_ctl, sm.ctl);
+      plan.add((uint8_t **)&e->sm_queue, sm.queues);
+    }
+  }
   GAS_TRY(plan.alloc());
 
   if (dev_build)

@@ -65,19 +65,23 @@ struct DeviceGroup {
 // ---------------------------------------------------------------------------
 // The engine object.
 // ---------------------------------------------------------------------------
-// Instantiated CUDA graphs cached per engine (valid until the next
-// set_graph, since their kernels capture the engine's buffers).
-// BFS runs on graphs up to this many vertices take the one-kernel path.
-constexpr int kBfsSmallMaxV = 1 << 18;
+// BFS runs on graphs up to this many vertices take the one-kernel path
+// (figures in gas_small.cu; measured to 2^24, where it is 15 to 25 % faster).
+constexpr int kBfsSmallMaxV = 1 << 24;
+// ... but with tracing or profiling on, to which the multi-kernel loop gives
+// records per iteration, only up to this many.
+constexpr int kBfsSmallRecordsMaxV = 1 << 18;
 // SSSP and CC from the full active set likewise (figures in
 // gas_small_min.cu): under AUTO up to 2^21 vertices; the kernel still halves
 // the fixed heuristic's time at 2^22, but from there on LEARNED's
 // multi-kernel push is the faster schedule and the heuristic stays what it
 // is compared with.  Under LEARNED up to 2^20: at 2^21 the multi-kernel push
-// wins on R-MAT CC (752 against 835 us).
+// wins on R-MAT CC (731 against 824 us).
 constexpr int kMinSmallMaxV = 1 << 21;
 constexpr int kMinSmallLearnedMaxV = 1 << 20;
 
+// Instantiated CUDA graphs cached per engine (valid until the next
+// set_graph, since their kernels capture the engine's buffers).
 enum { kGraphGeneric = 0, kGraphOrdered = 1, kGraphPagerank = 2, kGraphUser = 3,
        kGraphFast0 = 4, kGraphSlots = 12 };
 
@@ -181,15 +185,16 @@ struct gas_engine {
   cudaGraphExec_t graphs[kGraphSlots] = {};
   bool level_from_counters = false;  // BFS level = counters.iteration
   // small-graph BFS (gas_small.cu): three frontier bitmaps, the control
-  // word, the level's members with many out-edges
+  // word, the two queues
   uint32_t *sb_bits = nullptr;
-  void *sb_ctl = nullptr;
-  int32_t *sb_heavy = nullptr;
+  void *sb_ctl = nullptr, *sb_queue = nullptr;
+  DeviceGroup sb_mem;
   bool sb_clean = false;  // the kernel left them clear for the next run
   // small-graph SSSP and CC (gas_small_min.cu): second value buffer, the two
   // queues, the control word
   int32_t *sm_vals = nullptr;
   void *sm_queue = nullptr, *sm_ctl = nullptr;
+  DeviceGroup sm_mem;
   bool sm_clean = false;
   // what graphs[kGraphUser] was captured with (gas_engine_run_user)
   gas_user_step_fn user_step = nullptr;

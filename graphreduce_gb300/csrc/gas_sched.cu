@@ -1050,10 +1050,15 @@ gas_status_t ensure_fast_buffers(gas_engine *e) {
 namespace gas {
 
 void reserve_fast_buffers(gas_engine *e) {
-  const bool sized = e->prog == GAS_PROG_BFS ? e->nV > kBfsSmallMaxV
-                     : (e->prog == GAS_PROG_SSSP || e->prog == GAS_PROG_CC) &&
-                           e->nV > kMinSmallLearnedMaxV;
-  if (!sized || e->graph_only) return;
+  if (e->graph_only) return;
+  if (e->prog == GAS_PROG_BFS && e->nV <= kBfsSmallMaxV && !e->edges_on_host) {
+    if (e->nV > kBfsSmallRecordsMaxV) bfs_small_reserve(e);
+    return;
+  }
+  const bool sized = (e->prog == GAS_PROG_BFS && e->nV > kBfsSmallRecordsMaxV) ||
+                     ((e->prog == GAS_PROG_SSSP || e->prog == GAS_PROG_CC) &&
+                      e->nV > kMinSmallLearnedMaxV);
+  if (!sized) return;
   if (ensure_fast_buffers(e) != GAS_OK) {  // tight memory: the first run asks again
     e->fast_mem.free();
     cudaGetLastError();
@@ -1145,9 +1150,9 @@ gas_status_t run_fast(gas_engine *e, gas_schedule_t schedule,
   if (e->prog == GAS_PROG_BFS && schedule == GAS_SCHED_LEARNED) schedule = GAS_SCHED_AUTO;
   if (schedule == GAS_SCHED_LEARNED && !e->sched_model)
     return fail(GAS_ERR_STATE, "LEARNED schedule without a schedule model");
-  if (bfs_small_eligible(e, schedule))
+  if (bfs_small_eligible(e, schedule) && bfs_small_reserve(e))
     return run_bfs_small(e, schedule, max_iterations, stats, stream);
-  if (min_small_eligible(e, schedule))
+  if (min_small_eligible(e, schedule) && min_small_reserve(e))
     return run_min_small(e, max_iterations, stats, stream);
   GAS_TRY(ensure_fast_buffers(e));
   FastCtx ctx;

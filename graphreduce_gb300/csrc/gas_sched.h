@@ -27,9 +27,25 @@ gas_status_t run_fast(gas_engine *e, gas_schedule_t schedule,
 
 bool host_loop_for(const gas_engine *e);
 
+// What the two one-kernel paths below keep with a graph: bitmaps or the second
+// values, the control word, both queues.
+struct SmallBytes {
+  size_t values, ctl, queues;
+  size_t all() const { return values + ctl + queues; }
+};
+// Up to this many bytes come with set_graph's one allocation: a cudaMalloc of
+// their own made the first BFS on R-MAT 2^16 take 242 us (167 us with little
+// to allocate).
+constexpr size_t kSmallWithGraph = (size_t)16 << 20;
+SmallBytes bfs_small_bytes(int64_t nV, int64_t nE);
+SmallBytes min_small_bytes(int64_t nV, int64_t nE);
+
 // BFS on a graph of at most kBfsSmallMaxV vertices as one cooperative
 // kernel (gas_small.cu): same depths and iteration count as run_fast.
+// reserve: the kernel's buffers, kept with the graph; false if there is no
+// memory for them (the multi-kernel loop needs less).
 bool bfs_small_eligible(const gas_engine *e, gas_schedule_t schedule);
+bool bfs_small_reserve(gas_engine *e);
 gas_status_t run_bfs_small(gas_engine *e, gas_schedule_t schedule, int32_t max_iterations,
                            gas_run_stats *stats, void *stream);
 
@@ -37,6 +53,7 @@ gas_status_t run_bfs_small(gas_engine *e, gas_schedule_t schedule, int32_t max_i
 // vertices as one cooperative kernel (gas_small_min.cu): same vertex data
 // and iteration count as run_fast.
 bool min_small_eligible(const gas_engine *e, gas_schedule_t schedule);
+bool min_small_reserve(gas_engine *e);
 gas_status_t run_min_small(gas_engine *e, int32_t max_iterations, gas_run_stats *stats,
                            void *stream);
 

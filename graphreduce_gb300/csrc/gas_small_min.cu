@@ -39,10 +39,10 @@
 // fewer CTAs is cheaper.  Big ones by L2 lookups (a random value per edge).
 // Measured against the fast schedule (us per run, SSSP, AUTO / LEARNED /
 // here): R-MAT 16 edges per vertex, 4,093 vertices 389 / 356 / 106, 262 K
-// 557 / 459 / 256, 1 M 1365 / 744 / 626, 2 M 1787 / 980 / 967, 4 M 3810 /
-// 1849 / 1896; Erdos-Renyi 12 per vertex, 65 K 736 / 744 / 242, 1 M 2385 /
-// 1532 / 1153, 2 M 4414 / 2455 / 2133.  CC on R-MAT, 65 K 285 / 265 / 119,
-// 1 M 958 / 492 / 468, 2 M 1561 / 752 / 835.
+// 557 / 459 / 256, 1 M 1365 / 743 / 597, 2 M 1787 / 978 / 901, 4 M 3747 /
+// 1756 / 1810; Erdos-Renyi 12 per vertex, 65 K 736 / 744 / 242, 1 M 2385 /
+// 1532 / 1020, 2 M 4414 / 2367 / 2092.  CC on R-MAT, 65 K 285 / 265 / 119,
+// 1 M 958 / 492 / 459, 2 M 1561 / 731 / 824, 4 M 2741 / 1358 / 1510.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -50,161 +50,21 @@
 
 #include "gas.h"
 #include "gas_engine_impl.h"
-#include "gas_grid.cuh"
 #include "gas_internal.h"
 #include "gas_sched.h"
+#include "gas_stage.cuh"
 
 namespace {
 
-constexpr int kNT = 1024;
-constexpr int kWarps = kNT / 32;
-constexpr int kLight = 32;        // out-edges of a light member
-constexpr int kEntryEdges = 128;
-constexpr int kHeavyMost = 8;     // heavy entries a warp takes at once (1: 20 %
-                                  // slower on R-MAT 4 M, 32: 8 % on 1 M)
-constexpr int kStage = 4096;      // members a CTA collects before it appends directly
+using namespace gasstage;
+
 constexpr int kCtaEdges = 2048;   // 8192 and more: 1.3x and more slower below 100 K edges
 constexpr int kDense = 8;         // 2: 4 % slower on Erdos-Renyi 65 K, even on R-MAT
-
-struct Count {
-  int light, heavy, edges, pad;
-};
 
 struct MinCtl {
   gasgrid::Barrier bar;
   Count q[3];  // of the queue being read, filled and cleared (rotating)
 };
-
-__device__ __forceinline__ int32_t ld_edge(const int32_t *p) {
-  int32_t v;
-  asm("ld.global.nc.L1::no_allocate.b32 %0, [%1];" : "=r"(v) : "l"(p));
-  return v;
-}
-
-// A queue: light members (at most kLight out-edges, none included), one entry
-// each, and the others as heavy entries of kEntryEdges edges.
-struct Queue {
-  int4 *light, *heavy;  // (vertex, CSR position, edges)
-};
-
-// Light entries, heavy entries and out-edges of one member per lane (v < 0:
-// none), and their inclusive sums over the warp.
-struct Member {
-  int v, off, deg, nl, nh;
-  int il, ih, ie;
-};
-
-__device__ __forceinline__ Member member(int v, const int32_t *csr_off) {
-  Member m;
-  m.v = v;
-  m.off = v >= 0 ? __ldg(csr_off + v) : 0;
-  m.deg = v >= 0 ? __ldg(csr_off + v + 1) - m.off : 0;
-  m.nl = v >= 0 && m.deg <= kLight ? 1 : 0;
-  m.nh = m.deg > kLight ? (m.deg + kEntryEdges - 1) / kEntryEdges : 0;
-  m.il = __popc(__ballot_sync(0xffffffffu, m.nl) & (0xffffffffu >> (31 - (threadIdx.x & 31))));
-  m.ih = gasgrid::warp_incl_sum(m.nh);
-  m.ie = gasgrid::warp_incl_sum(m.deg);
-  return m;
-}
-
-// Room for the sums of nl light and nh heavy entries with ne edges.
-__device__ __forceinline__ int2 reserve(Count *c, int nl, int nh, int ne) {
-  int2 at = make_int2(0, 0);
-  if (nh) at.y = atomicAdd(&c->heavy, nh);
-  if (nl) at.x = atomicAdd(&c->light, nl);
-  if (ne) atomicAdd(&c->edges, ne);
-  return at;
-}
-
-__device__ __forceinline__ void write_entries(const Queue &q, const Member &m, int al, int ah) {
-  if (m.nl) q.light[al + m.il - 1] = make_int4(m.v, m.off, m.deg, 0);
-  ah += m.ih - m.nh;
-  for (int e = 0; e < m.nh; ++e)
-    q.heavy[ah + e] = make_int4(m.v, m.off + e * kEntryEdges,
-                                min(m.deg - e * kEntryEdges, kEntryEdges), 0);
-}
-
-struct Stage {
-  int n;  // members offered this iteration (those past kStage went out directly)
-  int v[kStage];
-  int wl[kWarps], wh[kWarps], we[kWarps];
-  int2 base;
-};
-
-// All lanes of the warp call; v[h] >= 0: a new member.
-template <int K>
-__device__ __forceinline__ void offer(Stage &st, const int (&v)[K], const int32_t *csr_off,
-                                      const Queue &q, Count *c) {
-  const int lane = threadIdx.x & 31;
-  unsigned m[K];
-  int n = 0;
-#pragma unroll
-  for (int h = 0; h < K; ++h) {
-    m[h] = __ballot_sync(0xffffffffu, v[h] >= 0);
-    n += __popc(m[h]);
-  }
-  if (!n) return;
-  int at = 0;
-  if (lane == 0) at = atomicAdd(&st.n, n);
-  at = __shfl_sync(0xffffffffu, at, 0);
-  const bool over = at + n > kStage;  // warp-uniform
-#pragma unroll
-  for (int h = 0; h < K; ++h) {
-    const int pos = at + __popc(m[h] & ((1u << lane) - 1u));
-    at += __popc(m[h]);
-    if (!over) {
-      if (v[h] >= 0) st.v[pos] = v[h];
-    } else if (m[h]) {  // no room left in the stage: straight to the queue
-      if (v[h] >= 0 && pos < kStage) st.v[pos] = -1;
-      const Member mb = member(v[h], csr_off);
-      int2 to = make_int2(0, 0);
-      if (lane == 31) to = reserve(c, mb.il, mb.ih, mb.ie);
-      write_entries(q, mb, __shfl_sync(0xffffffffu, to.x, 31),
-                    __shfl_sync(0xffffffffu, to.y, 31));
-    }
-  }
-}
-
-// The collected members to the queue (every thread of the CTA calls).
-__device__ __forceinline__ void flush(Stage &st, const int32_t *csr_off, const Queue &q,
-                                      Count *c) {
-  __syncthreads();
-  const int n = min(st.n, kStage);
-  __syncthreads();        // every warp has the count before any goes on
-  if (n == 0) return;     // CTA-uniform
-  if (threadIdx.x == 0) st.n = 0;  // before the next offers: a barrier follows
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (n <= 32) {  // one warp's worth: the rest of the CTA waits at the caller's barrier
-    if (warp == 0) {
-      const Member m = member(lane < n ? st.v[lane] : -1, csr_off);
-      int2 at = make_int2(0, 0);
-      if (lane == 31) at = reserve(c, m.il, m.ih, m.ie);
-      write_entries(q, m, __shfl_sync(0xffffffffu, at.x, 31), __shfl_sync(0xffffffffu, at.y, 31));
-    }
-    __syncthreads();
-    return;
-  }
-  for (int i0 = 0; i0 < n; i0 += kNT) {  // CTA-uniform
-    const Member m = member(i0 + (int)threadIdx.x < n ? st.v[i0 + threadIdx.x] : -1, csr_off);
-    if (lane == 31) {
-      st.wl[warp] = m.il;
-      st.wh[warp] = m.ih;
-      st.we[warp] = m.ie;
-    }
-    __syncthreads();
-    if (warp == 0) {
-      const int l = st.wl[lane], h = st.wh[lane];
-      const int il = gasgrid::warp_incl_sum(l), ih = gasgrid::warp_incl_sum(h);
-      const int ie = gasgrid::warp_incl_sum(st.we[lane]);
-      st.wl[lane] = il - l;
-      st.wh[lane] = ih - h;
-      if (lane == 31) st.base = reserve(c, il, ih, ie);
-    }
-    __syncthreads();
-    write_entries(q, m, st.base.x + st.wl[warp], st.base.y + st.wh[warp]);
-    __syncthreads();
-  }
-}
 
 // One warp's share of a queue's light or heavy entries: up to 32 at a time,
 // as many as spread them over all warps, beginning with warp w0.
@@ -220,7 +80,7 @@ __device__ __forceinline__ void walk(const int4 *Q, int nq, int most, int w0,
   constexpr int kRounds = 4;
   const int lane = threadIdx.x & 31;
   const int nwarps = gridDim.x * kWarps;
-  int gwarp = ((blockIdx.x * kNT + threadIdx.x) >> 5) - w0;
+  int gwarp = dealt_warp() - w0;
   if (gwarp < 0) gwarp += nwarps;
   const int per = min(most, (nq + nwarps - 1) / nwarps);
   for (long long base = (long long)gwarp * per; base < nq; base += (long long)nwarps * per) {
@@ -232,35 +92,16 @@ __device__ __forceinline__ void walk(const int4 *Q, int nq, int most, int w0,
       val = R[e.x];
       atomicMin(W + e.x, val);
     }
-    // entries with edges, to consecutive lanes
-    const unsigned rb = __ballot_sync(FULL, deg > 0);
-    const int rows = __popc(rb);
-    const int incl = gasgrid::warp_incl_sum(deg);
-    const int T = __shfl_sync(FULL, incl, 31);
-    if (deg > 0) {
-      int *s = s_row[__popc(rb & ((1u << lane) - 1u))];
-      s[0] = incl - deg;
-      s[1] = start - (incl - deg);
-      s[2] = val;
-    }
-    __syncwarp();
-    const bool ok = lane < rows;
-    const int excl = ok ? s_row[lane][0] : 0;
-    const int shift = ok ? s_row[lane][1] : 0;
-    val = ok ? s_row[lane][2] : 0;
-    __syncwarp();
+    Rows rows;
+    const int T = lay_out(start, deg, val, s_row, rows);
     for (int r = 0; r < T; r += 32 * kRounds) {
       int v[kRounds], cand[kRounds], cur[kRounds];
 #pragma unroll
       for (int h = 0; h < kRounds; ++h) {
         const int r0 = r + 32 * h;
-        const int row0 = __popc(__ballot_sync(FULL, ok && excl <= r0)) - 1;
-        const int d = excl - r0;
-        const unsigned starts =
-            __reduce_or_sync(FULL, (ok && d >= 1 && d < 32) ? (1u << d) : 0u);
-        const int row = min(31, row0 + __popc(starts & ((2u << lane) - 1u)));
-        const int pos = r0 + lane + __shfl_sync(FULL, shift, row);
-        cand[h] = __shfl_sync(FULL, val, row);
+        const int row = row_of(rows, r0);
+        const int pos = r0 + lane + __shfl_sync(FULL, rows.shift, row);
+        cand[h] = __shfl_sync(FULL, rows.val, row);
         v[h] = -1;
         if (r0 + lane < T) {
           v[h] = ld_edge(csr_dst + pos);
@@ -408,17 +249,26 @@ bool min_small_eligible(const gas_engine *e, gas_schedule_t schedule) {
          e->nV <= (schedule == GAS_SCHED_AUTO ? kMinSmallMaxV : kMinSmallLearnedMaxV);
 }
 
+SmallBytes min_small_bytes(int64_t nV, int64_t nE) {
+  return {(size_t)nV * sizeof(int32_t), sizeof(MinCtl),
+          2 * ((size_t)nV + heavy_cap(nE)) * sizeof(int4)};
+}
+
+bool min_small_reserve(gas_engine *e) {
+  if (e->sm_vals) return true;
+  const SmallBytes n = min_small_bytes(e->nV, e->nE);
+  e->sm_clean = false;
+  if (e->sm_mem.alloc({GROUP_PART(e->sm_vals, n.values), GROUP_PART(e->sm_ctl, n.ctl),
+                       GROUP_PART(e->sm_queue, n.queues)}) == cudaSuccess)
+    return true;
+  cudaGetLastError();
+  return false;
+}
+
 gas_status_t run_min_small(gas_engine *e, int32_t max_iterations, gas_run_stats *stats,
                            void *stream) {
   cudaStream_t s = (cudaStream_t)stream;
-  // a heavy member has ceil(deg / kEntryEdges) <= deg / kLight entries
-  const size_t V = (size_t)e->nV, H = (size_t)e->nE / kLight + 1;
-  if (!e->sm_vals) CUDA_TRY(cudaMalloc(&e->sm_vals, V * sizeof(int32_t)));
-  if (!e->sm_queue) CUDA_TRY(cudaMalloc(&e->sm_queue, 2 * (V + H) * sizeof(int4)));
-  if (!e->sm_ctl) {
-    CUDA_TRY(cudaMalloc(&e->sm_ctl, sizeof(MinCtl)));
-    e->sm_clean = false;
-  }
+  const size_t V = (size_t)e->nV, H = heavy_cap(e->nE);
   // the kernel leaves its control word clear; cleared here at first and
   // after a run that failed
   if (!e->sm_clean) CUDA_TRY(cudaMemsetAsync(e->sm_ctl, 0, sizeof(MinCtl), s));

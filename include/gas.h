@@ -232,12 +232,12 @@ gas_status_t gas_engine_download_vertex_data_async(gas_engine *e, void *dst,
 
 /* Schedule of the built-in fast runs.  For BFS the pull is the bottom-up
  * level (each unvisited vertex stops at its first in-neighbour of the
- * previous level), and AUTO and LEARNED both take a direction rule: graphs
- * of more than 2^18 vertices Beamer, Asanovic and Patterson's (SC'12;
- * bottom-up once the frontier's out-edges exceed 1/14 of the edges not yet
- * explored, top-down again once it shrinks below V/24 vertices), smaller
- * ones (one cooperative kernel) "bottom-up while the frontier's out-edges
- * exceed E/16". */
+ * previous level), and AUTO and LEARNED both take Beamer, Asanovic and
+ * Patterson's direction rule (SC'12; bottom-up once the frontier's out-edges
+ * exceed 1/14 of the edges not yet explored, top-down again once it shrinks
+ * below V/24 vertices).  Graphs of up to 2^24 vertices run as one cooperative
+ * kernel under every schedule but PUSH (of up to 2^18 with tracing or
+ * profiling on). */
 typedef enum {
   GAS_SCHED_AUTO = 0,      /* fixed heuristic per iteration                */
   GAS_SCHED_GENERIC = 1,   /* the step-API kernels (pull over active set)  */
