@@ -130,11 +130,19 @@ struct gas_engine {
   float *pr_inv_deg = nullptr;  // [V] RN(1 / out-degree) (0: none)
   double *pr_l1 = nullptr;
   int32_t pr_l1_cap = 0;
-  // merge-path tiles of the CSC: start rows [tiles + 1], head and tail
-  // carry records [tiles]
+  // tiles of the in-edges: rows ended before each, head and tail carry records
   int32_t *pr_tile_row = nullptr;
   void *pr_head = nullptr, *pr_tail = nullptr;
-  int32_t pr_tile_cap = 0;
+  uint32_t *pr_end_bits = nullptr;  // the last in-edges of the rows
+  DeviceGroup pr_tiles;
+  // hot sources of the graph (gas_runs.cu): their numbers, the iteration's
+  // contributions, the in-edges with their slots
+  void *pr_hot_ctl = nullptr;
+  int32_t *pr_hot_id = nullptr, *pr_hot_src = nullptr;
+  float *pr_hot_val = nullptr;
+  DeviceGroup pr_hot_mem;
+  int32_t pr_hot_n = 0;
+  bool pr_hot_known = false;
   double pr_damping = 0.0;
 
   // fast-schedule state (lazily allocated): frontier queue of C_k with the

@@ -367,37 +367,166 @@ __device__ __forceinline__ void pr_bind(PrPol &pol, const PrBufs &b,
 }
 
 __device__ __forceinline__ void block_sum_store(double v, double *out) {
-  __shared__ double s_w[kNT / 32];
+  __shared__ double s_w[32];
   for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
   if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = v;
   __syncthreads();
   if (threadIdx.x == 0) {
     double t = 0.0;
-    for (int w = 0; w < kNT / 32; ++w) t += s_w[w];
+    for (int w = 0; w < (int)blockDim.x / 32; ++w) t += s_w[w];
     *out = t;
   }
 }
 
-// ---- merge-path gather (Merrill & Garland, "Merge-based parallel sparse
-// matrix-vector multiplication", SC'16) ----
-// The CSC is walked as one merge path of nV row ends and nE in-edges (an
-// edge is taken while its index is below the current row's end offset).  A
-// warp owns a tile of kPrW consecutive path items, a lane kPrK of them; the
-// warps of a CTA never wait for one another.  A tile stages its row end
-// offsets and the gathered contributions of its edges in the warp's shared
-// memory (coalesced index loads, kPrK independent gathers per lane), each
-// lane sums its items sequentially, a segmented warp scan of the lanes'
-// open-row partials joins rows that span lanes, and the rows that start and
-// end inside the tile are finished there with coalesced writes.  A row that
-// spans tiles leaves its first part as the tile's tail record and the
-// following parts as head records; k_pr_merge_fix joins them.
+// ---- gather ----
+// A warp owns a tile of kPrW consecutive in-edges, a lane kPrK of them; the
+// warps of a CTA never wait for one another.  A tile stages the gathered
+// contributions in the warp's shared memory (coalesced index loads, kPrK
+// independent gathers per lane), each lane sums its edges sequentially, with
+// a bit per edge telling where a row ends, a segmented warp scan of the
+// lanes' open-row partials joins rows that span lanes, and the rows that
+// start and end inside the tile are finished there with coalesced accesses.
+// A row that spans tiles leaves its first part as the tile's tail record and
+// the following parts as head records; k_pr_join joins them.  Rows are the
+// ones with in-edges (ne_vid); the others' ranks settle in two iterations.
+//
+// Bound by the L1 data pipe: a wavefront per random contribution (fewer where
+// neighbours in a sorted row share a line) and the staging's.  So a row's end
+// is a bit, not an item of a merge path with its offset in shared memory and
+// a search per lane: 400 instructions a tile where 256 items of the merge
+// path took 610, 12 M shared wavefronts where they took 22 M (R-MAT 4 M).
+// Measured, ms per run of 45 to 51 iterations, merge path / row-end bits:
+// R-MAT 1 M, 8 edges per vertex 2.80 / 2.48, 4 M, 16 per vertex 14.97 /
+// 13.12, 16.8 M directed 58.5 / 52.8; with the hot sources below 2.48, 11.3,
+// 47.3.
 constexpr int kPrK = 8;
+constexpr int kPrCtas = 4;
 constexpr int kPrW = 32 * kPrK;
-constexpr int kPrWarps = kNT / 32;
 // s_val is padded by one word per kPrK: a lane reads about kPrK words past
 // its neighbour, which without the pad puts 32 / kPrK lanes on one bank
 __device__ __forceinline__ int pr_pad(int j) { return j + j / kPrK; }
 constexpr int kPrValWords = kPrW + kPrW / kPrK;
+
+// A warp's staging: contributions, sums of the rows that end in the tile.
+struct PrStage {
+  float val[kPrValWords];
+  float sum[kPrW];
+};
+
+// Hot sources: the contributions of the kHotSlots sources with the most
+// out-edges are copied into each CTA's shared memory, where 32 of them take
+// about 3 wavefronts and not up to 32.  A copy of the in-edges, made once per
+// graph, has their slots.  163 KB of shared memory with the staging of 32
+// warps, for L1 has to hold the lines in flight: with 227 KB (45,000 slots)
+// R-MAT 16.8 M took 98 ms, with 99 KB 48.4, with 163 KB 47.3; without hot
+// sources 52.8.
+constexpr int kHotWarps = 32;
+constexpr int kHotSlots =
+    (int)((162 * 1024 - 256 - kHotWarps * sizeof(PrStage)) / sizeof(float) / 1024) * 1024;
+constexpr size_t kHotSmem = kHotSlots * sizeof(float) + kHotWarps * sizeof(PrStage);
+constexpr int kHotBuckets = 1024;
+// In-edges from which on, and the share of them with a hot source from which
+// on, the copy is made.  us per run without / with: R-MAT, 4.3 M edges 1680 /
+// 1715, 7.9 M 2479 / 2385, 12 M 3269 / 2950; Erdos-Renyi, 9 to 18 M edges, a
+// share of 78 % 250 / 262 (the contributions fit L1), 47 % 312 / 297, 29 % 426
+// / 407, 20 % 563 / 585, 12 % 549 / 556.
+constexpr int kHotMinEdges = 1 << 23;
+constexpr double kHotMinShare = 0.25;
+
+struct PrHot {
+  uint32_t count[kHotBuckets];  // vertices by out-degree bucket
+  uint32_t edges[kHotBuckets];  // and their out-edges
+  int32_t bucket;               // hot: buckets from this one on
+  int32_t n;                    // hot vertices
+  uint32_t covered;             // their out-edges
+  int32_t next;                 // slots given out
+};
+
+// Out-degree buckets: exact below 64, 32 to an octave above.
+__device__ __forceinline__ int hot_bucket(int d) {
+  if (d < 64) return d;
+  const int l = 31 - __clz(d);
+  return 64 + (l - 6) * 32 + ((d >> (l - 5)) & 31);
+}
+
+__global__ void __launch_bounds__(kNT) k_hot_count(const int32_t *csr_off, int nV, PrHot *h) {
+  __shared__ uint32_t s_n[kHotBuckets], s_e[kHotBuckets];
+  for (int i = threadIdx.x; i < kHotBuckets; i += kNT) s_n[i] = s_e[i] = 0u;
+  __syncthreads();
+  for (int v = blockIdx.x * kNT + threadIdx.x; v < nV; v += gridDim.x * kNT) {
+    const int d = csr_off[v + 1] - csr_off[v];
+    if (d == 0) continue;
+    const int b = hot_bucket(d);
+    atomicAdd(&s_n[b], 1u);
+    atomicAdd(&s_e[b], (uint32_t)d);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kHotBuckets; i += kNT)
+    if (s_n[i]) {
+      atomicAdd(&h->count[i], s_n[i]);
+      atomicAdd(&h->edges[i], s_e[i]);
+    }
+}
+
+// The lowest bucket from which on all vertices have a slot.
+__global__ void __launch_bounds__(kHotBuckets) k_hot_pick(PrHot *h) {
+  __shared__ uint32_t s_n[kHotBuckets], s_e[kHotBuckets];
+  s_n[threadIdx.x] = h->count[threadIdx.x];
+  s_e[threadIdx.x] = h->edges[threadIdx.x];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int b = kHotBuckets;
+    uint32_t n = 0, e = 0;
+    while (b > 1 && n + s_n[b - 1] <= (uint32_t)kHotSlots) {
+      --b;
+      n += s_n[b];
+      e += s_e[b];
+    }
+    h->bucket = b;
+    h->n = (int32_t)n;
+    h->covered = e;
+  }
+}
+
+__global__ void __launch_bounds__(kNT)
+    k_hot_assign(const int32_t *csr_off, int nV, PrHot *h, int32_t *hot_id, int32_t *slot_of) {
+  const int bucket = h->bucket;
+  for (int v = blockIdx.x * kNT + threadIdx.x; v < nV; v += gridDim.x * kNT) {
+    const int d = csr_off[v + 1] - csr_off[v];
+    int s = -1;
+    if (d > 0 && hot_bucket(d) >= bucket) {
+      s = atomicAdd(&h->next, 1);
+      hot_id[s] = v;
+    }
+    slot_of[v] = s;
+  }
+}
+
+// In-edges with a hot source's slot (complemented) in place of its number.
+__global__ void __launch_bounds__(kNT)
+    k_hot_sources(const int32_t *__restrict__ csc_src, int nE,
+                  const int32_t *__restrict__ slot_of, int32_t *__restrict__ out) {
+  const long long stride = (long long)gridDim.x * kNT;
+  for (long long i = blockIdx.x * (long long)kNT + threadIdx.x; i < nE; i += 4 * stride) {
+    int u[4], s[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) u[k] = i + k * stride < nE ? __ldg(csc_src + i + k * stride) : 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) s[k] = __ldg(slot_of + u[k]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (i + k * stride < nE) out[i + k * stride] = s[k] >= 0 ? ~s[k] : u[k];
+  }
+}
+
+// The hot sources' contributions of this iteration, next to one another.
+__global__ void __launch_bounds__(kNT)
+    k_hot_values(PrBufs bufs, const int32_t *hot_id, int n, float *hot,
+                 const gas_counters *cnt) {
+  const float *contrib = bufs.contrib[cnt->iteration & 1];
+  const int i = blockIdx.x * kNT + threadIdx.x;
+  if (i < n) hot[i] = contrib[hot_id[i]];
+}
 
 struct PrCarry {
   int32_t row;   // -1: no record
@@ -405,22 +534,26 @@ struct PrCarry {
   float s, c;
 };
 
-// Merge-path coordinate (rows ended) of each tile start, once per run.
-__global__ void k_pr_tiles(const int32_t *csc_off, int nV, int nE, int n_tiles,
-                           int32_t *tile_row) {
-  const long long path = (long long)nV + nE;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t <= n_tiles;
-       t += gridDim.x * blockDim.x) {
-    const long long d = min((long long)t * kPrW, path);
-    long long lo = max(d - nE, 0LL), hi = min(d, (long long)nV);
+// Rows ended before each tile, and the row-end bits (zero before).
+__global__ void __launch_bounds__(kNT)
+    k_pr_tiles(const int32_t *ne_end, int n_ne, int n_tiles, int32_t *tile_row,
+               uint32_t *end_bits) {
+  const int tid = blockIdx.x * kNT + threadIdx.x, nthr = gridDim.x * kNT;
+  for (int t = tid; t < n_tiles; t += nthr) {
+    const int e0 = t * kPrW;
+    int lo = 0, hi = n_ne;
     while (lo < hi) {
-      const long long p = (lo + hi) >> 1;
-      if (csc_off[p + 1] <= d - p - 1)
-        lo = p + 1;
+      const int m = (lo + hi) >> 1;
+      if (ne_end[m] <= e0)
+        lo = m + 1;
       else
-        hi = p;
+        hi = m;
     }
-    tile_row[t] = (int32_t)lo;
+    tile_row[t] = lo;
+  }
+  for (int i = tid; i < n_ne; i += nthr) {
+    const int last = ne_end[i] - 1;
+    atomicOr(end_bits + (last >> 5), 1u << (last & 31));
   }
 }
 
@@ -430,165 +563,153 @@ __device__ __forceinline__ int32_t pr_ld_stream(const int32_t *p) {
   return v;
 }
 
-__global__ void __launch_bounds__(kNT, 3)
-    k_pr_merge(PrPol pol, PrBufs bufs, const int32_t *csc_off, int nV, int nE,
-               const int32_t *tile_row, int n_tiles, PrCarry *head, PrCarry *tail,
-               const gas_counters *cnt, double *l1_part) {
-  __shared__ int32_t s_end_all[kPrWarps][kPrW + 1];
-  __shared__ float s_val_all[kPrWarps][kPrValWords];
-  __shared__ float2 s_sum_all[kPrWarps][kPrW];
+// kHot: pol.csc_src holds slots of hot sources, whose contributions are read
+// from the CTA's copy.
+template <bool kHot>
+__global__ void __launch_bounds__(kHot ? kHotWarps * 32 : kNT, kHot ? 1 : kPrCtas)
+    k_pr_gather(PrPol pol, PrBufs bufs, const int32_t *ne_vid, const uint32_t *end_bits, int nE,
+                const int32_t *tile_row, int n_tiles, PrCarry *head, PrCarry *tail,
+                const float *hot, int n_hot, const gas_counters *cnt, double *l1_part) {
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int kPrWarps = kHot ? kHotWarps : kNT / 32;
+  extern __shared__ float4 s_dyn[];
+  float *s_hot = reinterpret_cast<float *>(s_dyn);
   pr_bind(pol, bufs, cnt);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int32_t *s_end = s_end_all[warp];
-  float *s_val = s_val_all[warp];
-  float2 *s_sum = s_sum_all[warp];
-  const long long path = (long long)nV + nE;
+  PrStage &stage = reinterpret_cast<PrStage *>(s_hot + (kHot ? kHotSlots : 0))[warp];
+  float *s_val = stage.val;
+  float *s_sum = stage.sum;
   const int nwarps = gridDim.x * kPrWarps;
-  // software pipeline: the next tile's coordinates and edge indices load
+  // software pipeline: the next tile's edge indices, row and row ends load
   // while this tile's gathers and sums run
   int tile = blockIdx.x * kPrWarps + warp;
-  int r0 = 0, r1 = 0;
+  int r0 = 0;
+  uint32_t word = 0;  // row ends of the tile's edges [32 (lane / 4), + 32)
+  bool split = false; // row r0 started in an earlier tile
   int idx[kPrK];
   if (tile < n_tiles) {
     r0 = tile_row[tile];
-    r1 = tile_row[tile + 1];
-    const int e0 = (int)((long long)tile * kPrW - r0);
-    const int ne = (int)(min((long long)tile * kPrW + kPrW, path) - r1) - e0;
+    word = end_bits[tile * (kPrW / 32) + lane / 4];
+    split = tile > 0 && !(end_bits[tile * (kPrW / 32) - 1] >> 31);
 #pragma unroll
     for (int k = 0; k < kPrK; ++k) {
       const int j = lane + 32 * k;
-      idx[k] = j < ne ? pr_ld_stream(pol.csc_src + e0 + j) : 0;
+      idx[k] = j < nE - tile * kPrW ? pr_ld_stream(pol.csc_src + tile * kPrW + j) : 0;
     }
   }
+  if constexpr (kHot) {  // hot has room for a whole number of float4
+    const float4 *from = reinterpret_cast<const float4 *>(hot);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < (n_hot + 3) / 4; i += kHotWarps * 32) s_dyn[i] = from[i];
+    __syncthreads();
+  }
   for (; tile < n_tiles; tile += nwarps) {
-    const long long D0 = (long long)tile * kPrW;
-    const long long D1 = min(D0 + kPrW, path);
-    const int e0 = (int)(D0 - r0), e1 = (int)(D1 - r1);
-    const int nrows = r1 - r0, ne = e1 - e0;
+    const int ne = nE - tile * kPrW;
     float val[kPrK];
 #pragma unroll
     for (int k = 0; k < kPrK; ++k) {
       const int j = lane + 32 * k;
-      val[k] = j < ne ? __ldg(pol.contrib + idx[k]) : 0.0f;
+      val[k] = j < ne && (!kHot || idx[k] >= 0) ? __ldg(pol.contrib + idx[k]) : 0.0f;
     }
-    const int off0 = csc_off[r0];
+    // in registers of their own: a load into val would wait for the first one
+    float near[kPrK];
+    if constexpr (kHot) {
 #pragma unroll
-    for (int k = 0; k < kPrK; ++k) {
-      const int j = lane + 32 * k;
-      if (j < nrows) s_end[j] = csc_off[r0 + 1 + j];
+      for (int k = 0; k < kPrK; ++k) near[k] = idx[k] < 0 ? s_hot[~idx[k]] : 0.0f;
     }
-    if (lane == 0) s_end[nrows] = INT_MAX;
+    // rows that end before this lane's edges, and in the tile
+    const unsigned mine = (word >> (8 * (lane & 3))) & 0xffu;
+    int upto = __popc(word);
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(FULL, upto, o);
+      if (lane >= o) upto += u;
+    }
+    const int nrows = __shfl_sync(FULL, upto, 31);
+    int r = upto - __popc(word >> (8 * (lane & 3)));
+    const bool open = !(__shfl_sync(FULL, word, 31) >> 31) && ne > kPrW;
     const int next = tile + nwarps;
-    int nr0 = 0, nr1 = 0;
+    int nr0 = 0;
+    uint32_t nword = 0;
+    bool nsplit = false;
     if (next < n_tiles) {
       nr0 = tile_row[next];
-      nr1 = tile_row[next + 1];
-      const int ne0 = (int)((long long)next * kPrW - nr0);
-      const int nne = (int)(min((long long)next * kPrW + kPrW, path) - nr1) - ne0;
+      nword = end_bits[next * (kPrW / 32) + lane / 4];
+      nsplit = !(end_bits[next * (kPrW / 32) - 1] >> 31);
 #pragma unroll
       for (int k = 0; k < kPrK; ++k) {
         const int j = lane + 32 * k;
-        idx[k] = j < nne ? pr_ld_stream(pol.csc_src + ne0 + j) : 0;
+        idx[k] = j < nE - next * kPrW ? pr_ld_stream(pol.csc_src + next * kPrW + j) : 0;
       }
     }
-#pragma unroll
-    for (int k = 0; k < kPrK; ++k) {
-      const int j = lane + 32 * k;
-      if (j < ne) s_val[pr_pad(j)] = val[k];
-    }
     // the epilogue's inputs for the tile's first 32 rows
+    int v0 = 0;
     float inv0 = 0.0f, old0 = 0.0f;
     if (lane < nrows) {
-      inv0 = __ldg(pol.inv_deg + r0 + lane);
-      old0 = pol.rank_old[r0 + lane];
+      v0 = __ldg(ne_vid + r0 + lane);
+      inv0 = __ldg(pol.inv_deg + v0);
+      old0 = pol.rank_old[v0];
     }
-    __syncwarp();
-    // this lane's kPrK items: find its start on the tile's path
-    const int tlen = nrows + ne;
-    const int dt = min(lane * kPrK, tlen), dend = min(dt + kPrK, tlen);
-    int lo = max(dt - ne, 0), hi = min(dt, nrows);
-    while (lo < hi) {
-      const int p = (lo + hi) >> 1;
-      if (s_end[p] <= e0 + dt - p - 1)
-        lo = p + 1;
-      else
-        hi = p;
-    }
-    int r = lo, e = e0 + dt - lo;
-    int end_r = s_end[r];
-    float acc = 0.0f, first = 0.0f;
-    int first_r = 0;
-    bool ended = false;
 #pragma unroll
     for (int k = 0; k < kPrK; ++k) {
-      if (dt + k < dend) {
-        if (e < end_r) {
-          acc = __fadd_rn(acc, s_val[pr_pad(e - e0)]);
-          ++e;
-        } else {
-          if (!ended) {
-            first = acc;
-            first_r = r;
-          } else {
-            s_sum[r] = make_float2(acc, 0.0f);
-          }
-          ended = true;
-          acc = 0.0f;
-          ++r;
-          end_r = s_end[r];
-        }
+      if constexpr (kHot) val[k] = __int_as_float(__float_as_int(val[k]) | __float_as_int(near[k]));
+      s_val[pr_pad(lane + 32 * k)] = val[k];
+    }
+    __syncwarp();
+    float acc = 0.0f, first = 0.0f;
+    const int first_r = r;
+#pragma unroll
+    for (int k = 0; k < kPrK; ++k) {
+      acc = __fadd_rn(acc, s_val[pr_pad(lane * kPrK + k)]);
+      if ((mine >> k) & 1u) {
+        if (r == first_r)
+          first = acc;
+        else
+          s_sum[r] = acc;
+        acc = 0.0f;
+        ++r;
       }
     }
     // segmented inclusive scan of the open-row partials (a lane that ended
     // a row starts a segment)
+    const unsigned starts = __ballot_sync(FULL, mine != 0) & (FULL >> (31 - lane));
+    const int reach = lane - (starts ? 31 - __clz(starts) : 0);
     PrVal v{acc, 0.0f};
-    int f = ended;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const PrVal u{__shfl_up_sync(0xffffffffu, v.s, o), __shfl_up_sync(0xffffffffu, v.c, o)};
-      const int g = __shfl_up_sync(0xffffffffu, f, o);
-      if (lane >= o) {
-        if (!f) v = two_sum_add(u, v);
-        f |= g;
-      }
+      const PrVal u{__shfl_up_sync(FULL, v.s, o), __shfl_up_sync(FULL, v.c, o)};
+      if (o <= reach) v = two_sum_add(u, v);
     }
-    PrVal cin{__shfl_up_sync(0xffffffffu, v.s, 1), __shfl_up_sync(0xffffffffu, v.c, 1)};
+    PrVal cin{__shfl_up_sync(FULL, v.s, 1), __shfl_up_sync(FULL, v.c, 1)};
     if (lane == 0) cin = PrVal{0.0f, 0.0f};
-    if (ended) {
-      const PrVal t = two_sum_add(cin, PrVal{first, 0.0f});
-      s_sum[first_r] = make_float2(t.s, t.c);
+    PrVal row0{0.0f, 0.0f};
+    if (mine) {
+      row0 = two_sum_add(cin, PrVal{first, 0.0f});
+      s_sum[first_r] = __fadd_rn(row0.s, row0.c);
     }
-    const PrVal tot{__shfl_sync(0xffffffffu, v.s, 31), __shfl_sync(0xffffffffu, v.c, 31)};
+    const PrVal tot{__shfl_sync(FULL, v.s, 31), __shfl_sync(FULL, v.c, 31)};
     __syncwarp();
-    // rows that start and end in this tile; row r0 started in an earlier
-    // tile when e0 is past its first edge
-    const bool split = e0 > off0;
-    if (lane < nrows && !(lane == 0 && split)) {
-      const float2 t = s_sum[lane];
-      pol.emit(r0 + lane, PrVal{t.x, t.y}, inv0, old0);
-    }
-    for (int i = lane + 32; i < nrows; i += 32) {
-      const float2 t = s_sum[i];
-      pol.emit(r0 + i, PrVal{t.x, t.y});
-    }
+    // rows that start and end in this tile
+    if (lane < nrows && !(lane == 0 && split))
+      pol.emit(v0, PrVal{s_sum[lane], 0.0f}, inv0, old0);
+    for (int i = lane + 32; i < nrows; i += 32)
+      pol.emit(__ldg(ne_vid + r0 + i), PrVal{s_sum[i], 0.0f});
+    // the lane that ended the tile's first row has the head record, if that
+    // row came from an earlier tile
+    if (mine && first_r == 0)
+      head[tile] = split ? PrCarry{__ldg(ne_vid + r0), 1, row0.s, row0.c}
+                         : PrCarry{-1, 0, 0.0f, 0.0f};
     if (lane == 0) {
-      PrCarry h{-1, 0, 0.0f, 0.0f}, tl{-1, 0, 0.0f, 0.0f};
-      if (split) {
-        if (nrows > 0)
-          h = PrCarry{r0, 1, s_sum[0].x, s_sum[0].y};
-        else
-          h = PrCarry{r0, 0, tot.s, tot.c};
-      }
-      if (r1 < nV && !(split && nrows == 0)) {
-        const int off_r1 = nrows > 0 ? s_end[nrows - 1] : off0;
-        if (e1 > max(off_r1, e0)) tl = PrCarry{r1, 0, tot.s, tot.c};
-      }
-      head[tile] = h;
+      PrCarry tl{-1, 0, 0.0f, 0.0f};
+      if (nrows == 0) head[tile] = split ? PrCarry{__ldg(ne_vid + r0), 0, tot.s, tot.c} : tl;
+      if (open && !(split && nrows == 0))
+        tl = PrCarry{__ldg(ne_vid + r0 + nrows), 0, tot.s, tot.c};
       tail[tile] = tl;
     }
     __syncwarp();
     r0 = nr0;
-    r1 = nr1;
+    word = nword;
+    split = nsplit;
   }
   block_sum_store(pol.l1, l1_part + blockIdx.x);
 }
@@ -597,10 +718,12 @@ __global__ void __launch_bounds__(kNT, 3)
 // next tile's head ends the row (a row of fewer than about kPrW in-edges),
 // the two parts are the row.  Longer rows are walked by the whole warp, 32
 // head records at a time, up to the tile the row ends in.  A broken chain
-// sets the device error word instead of a rank.
+// sets the device error word instead of a rank.  And in the first two
+// iterations the rows without in-edges, whose ranks (in both buffers) are
+// the same ever after.
 __global__ void __launch_bounds__(kNT)
-    k_pr_merge_fix(PrPol pol, PrBufs bufs, const PrCarry *head, const PrCarry *tail,
-                   int n_tiles, gas_counters *cnt, double *l1_part) {
+    k_pr_join(PrPol pol, PrBufs bufs, const PrCarry *head, const PrCarry *tail, int n_tiles,
+              const int32_t *csc_off, int nV, gas_counters *cnt, double *l1_part) {
   pr_bind(pol, bufs, cnt);
   const int lane = threadIdx.x & 31;
   const int stride = gridDim.x * kNT;
@@ -658,6 +781,9 @@ __global__ void __launch_bounds__(kNT)
       }
     }
   }
+  if (cnt->iteration < 2)
+    for (int v = blockIdx.x * kNT + threadIdx.x; v < nV; v += stride)
+      if (csc_off[v] == csc_off[v + 1]) pol.emit(v, PrVal{0.0f, 0.0f});
   if (bad) atomicExch(&cnt->error, (int32_t)GAS_ERR_DEVICE);
   block_sum_store(pol.l1, l1_part + blockIdx.x);
 }
@@ -714,6 +840,7 @@ struct PrCtx {
   int n_tiles;
   int merge_grid;
   int fix_grid;
+  int n_hot;  // 0: every contribution is gathered from global memory
   double *residual;
 };
 
@@ -724,11 +851,19 @@ gas_status_t pr_body(gas_engine *e, cudaStream_t cs,
   // source's contribution; per vertex offsets, old and new rank, new
   // contribution
   gas::prof_begin(e, cs, gas::kProfPagerank, 8LL * e->nE + 16LL * e->nV);
-  k_pr_merge<<<c->merge_grid, kNT, 0, cs>>>(c->pol, c->bufs, e->csc_off, e->nV, e->nE,
-                                            c->tile_row, c->n_tiles, c->head, c->tail,
-                                            e->cnt, e->pr_l1);
-  k_pr_merge_fix<<<c->fix_grid, kNT, 0, cs>>>(c->pol, c->bufs, c->head, c->tail, c->n_tiles,
-                                              e->cnt, e->pr_l1 + c->merge_grid);
+  if (c->n_hot) {
+    k_hot_values<<<(c->n_hot + kNT - 1) / kNT, kNT, 0, cs>>>(c->bufs, e->pr_hot_id, c->n_hot,
+                                                             e->pr_hot_val, e->cnt);
+    k_pr_gather<true><<<c->merge_grid, kHotWarps * 32, kHotSmem, cs>>>(
+        c->pol, c->bufs, e->ne_vid, e->pr_end_bits, e->nE, c->tile_row, c->n_tiles, c->head,
+        c->tail, e->pr_hot_val, c->n_hot, e->cnt, e->pr_l1);
+  } else {
+    k_pr_gather<false><<<c->merge_grid, kNT, kNT / 32 * sizeof(PrStage), cs>>>(
+        c->pol, c->bufs, e->ne_vid, e->pr_end_bits, e->nE, c->tile_row, c->n_tiles, c->head,
+        c->tail, nullptr, 0, e->cnt, e->pr_l1);
+  }
+  k_pr_join<<<c->fix_grid, kNT, 0, cs>>>(c->pol, c->bufs, c->head, c->tail, c->n_tiles,
+                                         e->csc_off, e->nV, e->cnt, e->pr_l1 + c->merge_grid);
   gas::prof_end(e, cs);
   k_pr_finish<<<1, kNT, 0, cs>>>(e->pr_l1, c->merge_grid + c->fix_grid, c->residual + 1,
                                  e->cnt, c->residual, nullptr, h, e->in_graph ? 1 : 0);
@@ -746,6 +881,48 @@ extern "C" gas_status_t gas_engine_pagerank_precision(
 }
 
 namespace {
+
+// Chooses the hot sources of the graph and rewrites a copy of its in-edges,
+// once per graph; *n_hot = 0 where that does not pay or has no memory.
+// scratch: nV words.
+gas_status_t pr_hot_plan(gas_engine *e, int32_t *scratch, cudaStream_t s, int *n_hot) {
+  *n_hot = 0;
+  if (e->nE < kHotMinEdges || e->edges_on_host) return GAS_OK;
+  if (e->pr_hot_known) {
+    *n_hot = e->pr_hot_n;
+    return GAS_OK;
+  }
+  e->pr_hot_mem.free();
+  if (e->pr_hot_mem.alloc({GROUP_PART(e->pr_hot_ctl, sizeof(PrHot)),
+                           GROUP_PART(e->pr_hot_id, kHotSlots * sizeof(int32_t)),
+                           GROUP_PART(e->pr_hot_val, kHotSlots * sizeof(float)),
+                           GROUP_PART(e->pr_hot_src, (size_t)e->nE * sizeof(int32_t))}) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    e->pr_hot_known = true;
+    e->pr_hot_n = 0;
+    return GAS_OK;
+  }
+  PrHot *h = static_cast<PrHot *>(e->pr_hot_ctl);
+  const int grid = 4 * e->num_sms;
+  CUDA_TRY(cudaMemsetAsync(h, 0, sizeof(PrHot), s));
+  k_hot_count<<<grid, kNT, 0, s>>>(e->csr_off, e->nV, h);
+  k_hot_pick<<<1, kHotBuckets, 0, s>>>(h);
+  int32_t got[3];  // bucket, n, covered
+  CUDA_TRY(cudaMemcpyAsync(got, &h->bucket, sizeof(got), cudaMemcpyDeviceToHost, s));
+  CUDA_TRY(cudaStreamSynchronize(s));
+  if ((double)(uint32_t)got[2] >= kHotMinShare * e->nE) {
+    k_hot_assign<<<grid, kNT, 0, s>>>(e->csr_off, e->nV, h, e->pr_hot_id, scratch);
+    k_hot_sources<<<8 * e->num_sms, kNT, 0, s>>>(e->csc_src, e->nE, scratch, e->pr_hot_src);
+    CUDA_TRY(cudaGetLastError());
+    *n_hot = e->pr_hot_n = got[1];
+  } else {
+    e->pr_hot_mem.free();
+    e->pr_hot_n = 0;
+  }
+  e->pr_hot_known = true;
+  return GAS_OK;
+}
 
 gas_status_t pagerank_run(gas_engine *e, double damping, double tol, int32_t max_iterations,
                           const float *init, int32_t seed, float *ranks, gas_run_stats *stats,
@@ -765,32 +942,33 @@ gas_status_t pagerank_run(gas_engine *e, double damping, double tol, int32_t max
   if (!e->pr_seed) CUDA_TRY(cudaMalloc(&e->pr_seed, sizeof(int32_t)));
   if (!e->pr_inv_deg) CUDA_TRY(cudaMalloc(&e->pr_inv_deg, (size_t)nV * 4));
   PrCtx c;
-  const long long path = (long long)nV + e->nE;
-  c.n_tiles = (int)((path + kPrW - 1) / kPrW);
-  if (!e->pr_tile_row || e->pr_tile_cap < c.n_tiles) {
-    if (e->pr_tile_row) cudaFree(e->pr_tile_row);
-    if (e->pr_head) cudaFree(e->pr_head);
-    if (e->pr_tail) cudaFree(e->pr_tail);
-    e->pr_tile_row = nullptr;
-    e->pr_head = e->pr_tail = nullptr;
-    e->pr_tile_cap = 0;
-    if (e->graphs[kGraphPagerank]) cudaGraphExecDestroy(e->graphs[kGraphPagerank]);
-    e->graphs[kGraphPagerank] = nullptr;
-    CUDA_TRY(cudaMalloc(&e->pr_tile_row, ((size_t)c.n_tiles + 1) * 4));
-    CUDA_TRY(cudaMalloc(&e->pr_head, (size_t)c.n_tiles * sizeof(PrCarry)));
-    CUDA_TRY(cudaMalloc(&e->pr_tail, (size_t)c.n_tiles * sizeof(PrCarry)));
-    e->pr_tile_cap = c.n_tiles;
+  c.n_tiles = (int)(((long long)e->nE + kPrW - 1) / kPrW);
+  if (!e->pr_tile_row) {  // once per graph
+    const size_t words = (size_t)c.n_tiles * (kPrW / 32);
+    CUDA_TRY(e->pr_tiles.alloc({GROUP_PART(e->pr_tile_row, (size_t)c.n_tiles * 4),
+                                GROUP_PART(e->pr_head, (size_t)c.n_tiles * sizeof(PrCarry)),
+                                GROUP_PART(e->pr_tail, (size_t)c.n_tiles * sizeof(PrCarry)),
+                                GROUP_PART(e->pr_end_bits, words * 4)}));
+    CUDA_TRY(cudaMemsetAsync(e->pr_end_bits, 0, words * 4, S(stream)));
+    k_pr_tiles<<<gas::engine_grid(std::max({c.n_tiles, e->n_ne, 1}), kNT, 8 * e->num_sms), kNT, 0,
+                 S(stream)>>>(e->ne_end, e->n_ne, c.n_tiles, e->pr_tile_row, e->pr_end_bits);
   }
   c.tile_row = e->pr_tile_row;
   c.head = static_cast<PrCarry *>(e->pr_head);
   c.tail = static_cast<PrCarry *>(e->pr_tail);
-  int per_sm = 0;
-  CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pr_merge, kNT, 0));
+  GAS_TRY(pr_hot_plan(e, reinterpret_cast<int32_t *>(e->pr_contrib[1]), S(stream), &c.n_hot));
+  int per_sm = 1;
+  if (c.n_hot)
+    CUDA_TRY(cudaFuncSetAttribute(k_pr_gather<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)kHotSmem));
+  else
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pr_gather<false>, kNT,
+                                                           kNT / 32 * sizeof(PrStage)));
   c.merge_grid = e->num_sms * (per_sm > 0 ? per_sm : 1);  // resident CTAs only
   // a thread per tile record, at most 16 CTAs per SM: the records' loads
   // are dependent chains, so they want many threads in flight
   c.fix_grid = (int)std::min<long long>(16LL * e->num_sms,
-                                        std::max(1, (c.n_tiles + kNT - 1) / kNT));
+                                        std::max(1, std::max(c.n_tiles, nV / 4) / kNT + 1));
   const int nparts = c.merge_grid + c.fix_grid;
   if (!e->pr_l1 || e->pr_l1_cap < nparts + 2) {
     if (e->pr_l1) cudaFree(e->pr_l1);
@@ -801,7 +979,7 @@ gas_status_t pagerank_run(gas_engine *e, double damping, double tol, int32_t max
     CUDA_TRY(cudaMalloc(&e->pr_l1, sizeof(double) * (size_t)e->pr_l1_cap));
   }
   c.residual = e->pr_l1 + nparts;
-  c.pol.csc_src = e->csc_src;
+  c.pol.csc_src = c.n_hot ? e->pr_hot_src : e->csc_src;
   c.pol.inv_deg = e->pr_inv_deg;
   c.pol.base = (float)((1.0 - damping) / (double)nV);
   c.pol.base_seed = (float)(1.0 - damping);
@@ -828,8 +1006,6 @@ gas_status_t pagerank_run(gas_engine *e, double damping, double tol, int32_t max
                            cudaMemcpyHostToDevice, S(stream)));
   CUDA_TRY(cudaMemcpyAsync(e->pr_seed, &seed, sizeof(int32_t), cudaMemcpyHostToDevice,
                            S(stream)));
-  k_pr_tiles<<<gas::engine_grid(c.n_tiles + 1, kNT, 2 * e->num_sms), kNT, 0, S(stream)>>>(
-      e->csc_off, nV, e->nE, c.n_tiles, e->pr_tile_row);
   if (init)
     CUDA_TRY(cudaMemcpyAsync(e->pr_rank[0], init, (size_t)nV * 4, cudaMemcpyDefault,
                              S(stream)));
@@ -861,7 +1037,7 @@ gas_status_t pagerank_run(gas_engine *e, double damping, double tol, int32_t max
   if (stats) {
     stats->iterations = cnt.iteration;
     stats->pull_iters = cnt.iteration;
-    stats->kernel_launches = 3 * cnt.iteration + 3;
+    stats->kernel_launches = (c.n_hot ? 4 : 3) * cnt.iteration + 3;
     stats->edges_processed = (int64_t)cnt.iteration * e->nE;
     stats->residual = resid;
     stats->graph_launches = host_loop ? 0 : 1;
