@@ -158,7 +158,8 @@ __device__ __forceinline__ int block_excl_sum(int v, int *total) {
 }
 
 __global__ void k_set_range(int32_t start, int32_t n, const int32_t *csc_off,
-                            int32_t *act, int32_t *scan, gas_counters *cnt) {
+                            int32_t *act, int32_t *scan, gas_counters *cnt,
+                            int32_t *expand_wait) {
   const int32_t base = csc_off[start];
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= n;
        i += gridDim.x * blockDim.x) {
@@ -168,6 +169,7 @@ __global__ void k_set_range(int32_t start, int32_t n, const int32_t *csc_off,
       cnt->n_active = n;
       cnt->n_edges = csc_off[start + n] - base;
       cnt->n_scatter_edges = 0;
+      *expand_wait = 0;
     }
   }
 }
@@ -200,9 +202,8 @@ __global__ void k_commit(const int32_t *act, const gas_counters *cnt,
 // out-neighbour of many active vertices, and on PageRank (200 K vertices,
 // 3 M edges, most of them active) nearly every edge finds its bit set; a
 // stale clear bit (plain, L1-cached load) only repeats the same OR.  (A
-// second test in L2 before the atomic measured 23 + 22 us for the two
-// kernels below against 19 + 18: the reduction is not waited for, the load
-// is.)
+// second test in L2 before the atomic measured 23 + 22 us for light rows and
+// chunks against 19 + 18: the reduction is not waited for, the load is.)
 __device__ __forceinline__ void activate(uint32_t *bits, uint32_t w) {
   uint32_t *p = bits + (w >> 5);
   const uint32_t m = 1u << (w & 31);
@@ -210,41 +211,94 @@ __device__ __forceinline__ void activate(uint32_t *bits, uint32_t w) {
 }
 
 // Rows of more than kXLight out-edges leave their edges as chunks of kXChunk
-// for k_expand_chunks: at most E / kXLight entries.
+// for expand_chunks: at most E / kXLight entries.
 constexpr int kXLight = 64;
 constexpr int kXChunk = 256;
 
-// k_expand_rows' results: chunks listed, out-edges of the applied vertices.
+// k_expand_mark's results: chunks listed, out-edges of the applied vertices.
 struct ExpandCtl {
   int32_t n_chunks, n_edges;
+  uint32_t missed;  // in-edges a pull looked at in vain
+  int32_t wait;     // iterations to push after a pull that missed much
 };
 
-// A warp takes 32 active slots: it commits their new vertex data (slot !=
-// null; vd[act[i]] = slot[i], after every gather of the iteration has read
-// the old values), lists the chunks of the heavy rows (one atomic per warp)
-// and walks the light rows' edges laid end to end, 64 per round.  This and
-// k_expand_chunks replace a commit, a three-kernel scan of the out-degrees,
-// a partition and a tile walk over it: the bits set do not depend on the
-// order, so no scan is needed.  Bound by the reductions on words that
-// several SMs fill at once: the two take 19 + 18 us on average over a
-// PageRank run (200 K vertices, 3 M edges), where the kernels before took
-// 132 us.
+// Whether the iteration may pull at all: not if the active vertices have few
+// in-edges, so that few out-edges are to be expected of those among them that
+// apply, nor just after a bad pull.  (Marking costs an iteration that then
+// pushes 2 to 3 us.  1/4, 1/8 and 1/16 of the edges within 1 % of one another.)
+constexpr int kXActiveDiv = 8;
+__device__ __forceinline__ bool expand_may_pull(const gas_counters *cnt, const ExpandCtl *ctl,
+                                                const int2 *list, int nE) {
+  return list && ctl->wait == 0 && (long long)cnt->n_edges * kXActiveDiv > nE;
+}
+
+// The light rows among a warp's 32 (off, deg), pushed: their edges laid end to
+// end, 64 per round.
+__device__ __forceinline__ void expand_light(int off, int deg, const int32_t *csr_dst,
+                                             uint32_t *bits, int *s_start, int *s_excl) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  // without the empty ones, to consecutive places
+  const bool light = deg > 0 && deg <= kXLight;
+  const unsigned lb = __ballot_sync(FULL, light);
+  if (!lb) return;  // warp-uniform
+  const int rows = __popc(lb);
+  const int incl = warp_incl_sum(light ? deg : 0);
+  const int T = __shfl_sync(FULL, incl, 31);
+  if (light) {
+    const int k = __popc(lb & ((1u << lane) - 1u));
+    s_excl[k] = incl - deg;
+    s_start[k] = off;
+  }
+  __syncwarp();
+  const bool ok = lane < rows;
+  const int excl = ok ? s_excl[lane] : 0;
+  const int shift = ok ? s_start[lane] - excl : 0;
+  __syncwarp();
+  for (int r = 0; r < T; r += 64) {
+    int w[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r0 = r + 32 * h;
+      // the row of edge r0 is the last one starting at or before it; a bit
+      // per row that starts inside the round gives the other lanes theirs
+      const int row0 = __popc(__ballot_sync(FULL, ok && excl <= r0)) - 1;
+      const int k = excl - r0;
+      const unsigned starts = __reduce_or_sync(FULL, (ok && k >= 1 && k < 32) ? (1u << k) : 0u);
+      int row = row0 + __popc(starts & ((2u << lane) - 1u));
+      row = row > 31 ? 31 : row;
+      const int pos = r0 + lane + __shfl_sync(FULL, shift, row);
+      w[h] = r0 + lane < T ? __ldg(csr_dst + pos) : -1;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (w[h] >= 0) activate(bits, (uint32_t)w[h]);
+  }
+}
+
+// First pass over the active slots, a warp 32 of them: commits their new
+// vertex data (slot != null; vd[act[i]] = slot[i], after every gather of the
+// iteration has read the old values), adds up the applied ones' out-edges and
+// lists the chunks of their heavy rows (one atomic per warp).  Where a pull
+// may follow it marks them in a bitmap, and k_expand chooses the direction;
+// elsewhere it pushes the light rows at once.
 __global__ void __launch_bounds__(kNT)
-    k_expand_rows(const int32_t *act, const gas_counters *cnt, const uint8_t *ret,
-                  const int32_t *csr_off, const int32_t *csr_dst, uint32_t *bits,
-                  const uint8_t *slot, uint8_t *vd, int vbytes, int2 *chunks,
-                  ExpandCtl *ctl) {
+    k_expand_mark(const int32_t *act, const gas_counters *cnt, const uint8_t *ret,
+                  const int32_t *csr_off, const int32_t *csr_dst, uint32_t *changed,
+                  uint32_t *bits, const uint8_t *slot, uint8_t *vd, int vbytes, int2 *chunks,
+                  const int2 *list, int nE, ExpandCtl *ctl) {
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ int s_start[kNT / 32][32], s_excl[kNT / 32][32];
+  const bool mark = expand_may_pull(cnt, ctl, list, nE);
   const int n = cnt->n_active;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
-  const unsigned below = (1u << lane) - 1u;
   int edges = 0;
   for (long long base = 32LL * gwarp; base < n; base += 32LL * nwarps) {
     const long long i = base + lane;
-    int off = 0, deg = 0;
+    int off = 0, deg = 0, word = -1;
+    uint32_t bit = 0;
     if (i < n) {
       const int v = act[i];
       if (slot) {
@@ -261,9 +315,17 @@ __global__ void __launch_bounds__(kNT)
       if (ret[i]) {
         off = csr_off[v];
         deg = csr_off[v + 1] - off;
+        word = v >> 5;
+        bit = 1u << (v & 31);
       }
     }
     edges += deg;
+    // the ids ascend, so a warp's bits are in few words: one reduction each
+    if (mark) {  // uniform
+      const unsigned same = __match_any_sync(FULL, word);
+      const uint32_t all = __reduce_or_sync(same, bit);
+      if (word >= 0 && lane == __ffs(same) - 1) atomicOr(changed + word, all);
+    }
     unsigned hb = __ballot_sync(FULL, deg > kXLight);
     if (hb) {  // warp-uniform
       const int nc = deg > kXLight ? (deg + kXChunk - 1) / kXChunk : 0;
@@ -279,54 +341,17 @@ __global__ void __launch_bounds__(kNT)
           chunks[p + k] = make_int2(o + k * kXChunk, o + min(d, (k + 1) * kXChunk));
       }
     }
-    // light rows, without the empty ones, to consecutive places
-    const bool light = deg > 0 && deg <= kXLight;
-    const unsigned lb = __ballot_sync(FULL, light);
-    if (!lb) continue;  // warp-uniform
-    const int rows = __popc(lb);
-    const int incl = warp_incl_sum(light ? deg : 0);
-    const int T = __shfl_sync(FULL, incl, 31);
-    if (light) {
-      const int k = __popc(lb & below);
-      s_excl[warp][k] = incl - deg;
-      s_start[warp][k] = off;
-    }
-    __syncwarp();
-    const bool ok = lane < rows;
-    const int excl = ok ? s_excl[warp][lane] : 0;
-    const int shift = ok ? s_start[warp][lane] - excl : 0;
-    __syncwarp();
-    for (int r = 0; r < T; r += 64) {
-      int w[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int r0 = r + 32 * h;
-        // the row of edge r0 is the last one starting at or before it; a bit
-        // per row that starts inside the round gives the other lanes theirs
-        const int row0 = __popc(__ballot_sync(FULL, ok && excl <= r0)) - 1;
-        const int k = excl - r0;
-        const unsigned starts =
-            __reduce_or_sync(FULL, (ok && k >= 1 && k < 32) ? (1u << k) : 0u);
-        int row = row0 + __popc(starts & ((2u << lane) - 1u));
-        row = row > 31 ? 31 : row;
-        const int pos = r0 + lane + __shfl_sync(FULL, shift, row);
-        w[h] = r0 + lane < T ? __ldg(csr_dst + pos) : -1;
-      }
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-        if (w[h] >= 0) activate(bits, (uint32_t)w[h]);
-    }
+    if (!mark) expand_light(off, deg, csr_dst, bits, s_start[warp], s_excl[warp]);
   }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) edges += __shfl_xor_sync(FULL, edges, d);
   if (lane == 0 && edges) atomicAdd(&ctl->n_edges, edges);
 }
 
-// The heavy rows' chunks, a warp each, all of a chunk's loads in flight.
-__global__ void __launch_bounds__(kNT)
-    k_expand_chunks(const int2 *chunks, const ExpandCtl *ctl, const int32_t *csr_dst,
-                    uint32_t *bits) {
-  const int n = ctl->n_chunks;
+// The heavy rows' chunks, pushed: a warp each, all of a chunk's loads in
+// flight.
+__device__ __forceinline__ void expand_chunks(const int2 *chunks, int n, const int32_t *csr_dst,
+                                              uint32_t *bits) {
   const int lane = threadIdx.x & 31;
   const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
@@ -342,6 +367,132 @@ __global__ void __launch_bounds__(kNT)
     for (int k = 0; k < kXChunk / 32; ++k)
       if (w[k] >= 0) activate(bits, (uint32_t)w[k]);
   }
+}
+
+// Pulled: a warp per word of the next frontier, a lane per vertex, which
+// looks for a marked in-neighbour among its first kXLight in-edges -- the
+// first alone, then four at a time -- and stops at the first.  The in-edges
+// after those are chunks of kXChunk, listed once per graph (k_expand_list), a
+// warp each, skipped where the vertex has its bit already: hubs that no
+// marked vertex leads to would leave whole rows to single warps (CC on R-MAT
+// 2^14 with grid islands 2.2 -> 4.3 ms).
+__device__ __forceinline__ void expand_pull(const int32_t *csc_off, const int32_t *csc_src,
+                                            const uint32_t *changed, int nV, const int2 *list,
+                                            int n_list, uint32_t *bits, uint32_t *missed) {
+  uint32_t vain = 0;
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
+  for (int w = gwarp; 32LL * w < nV; w += nwarps) {
+    const int v = 32 * w + lane;
+    // unsigned: the steps past the last edge must not wrap
+    uint32_t i = 0, stop = 0;
+    if (v < nV) {
+      i = csc_off[v];
+      stop = min((uint32_t)csc_off[v + 1], i + kXLight);
+    }
+    const uint32_t look = stop - i;
+    bool hit = false;
+    if (i < stop) {
+      const int u = __ldg(csc_src + i);
+      hit = (changed[u >> 5] >> (u & 31)) & 1u;
+    }
+    for (++i; i < stop && !hit; i += 4) {
+      int u[4];
+      uint32_t f[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) u[j] = i + j < stop ? __ldg(csc_src + i + j) : -1;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) f[j] = u[j] >= 0 ? changed[u[j] >> 5] : 0u;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) hit |= u[j] >= 0 && ((f[j] >> (u[j] & 31)) & 1u);
+    }
+    if (!hit) vain += look;
+    const unsigned word = __ballot_sync(FULL, hit);
+    if (lane == 0 && word) atomicOr(bits + w, word);
+  }
+  for (int c = gwarp; c < n_list; c += nwarps) {
+    const int2 e = list[c];  // vertex, first in-edge
+    uint32_t *p = bits + (e.x >> 5);
+    const uint32_t m = 1u << (e.x & 31);
+    if (__ldcg(p) & m) continue;  // warp-uniform: one address
+    const uint32_t end = csc_off[e.x + 1];
+    int u[kXChunk / 32];
+    bool f = false;
+#pragma unroll
+    for (int k = 0; k < kXChunk / 32; ++k) {
+      const uint32_t q = (uint32_t)e.y + 32 * k + lane;
+      u[k] = q < end ? __ldg(csc_src + q) : -1;
+    }
+#pragma unroll
+    for (int k = 0; k < kXChunk / 32; ++k)
+      f |= u[k] >= 0 && ((changed[u[k] >> 5] >> (u[k] & 31)) & 1u);
+    if (!__any_sync(FULL, f))
+      vain += kXChunk / 32;
+    else if (lane == 0)
+      atomicOr(p, m);
+  }
+  vain = __reduce_add_sync(FULL, vain);
+  if (lane == 0 && vain) atomicAdd(missed, vain);
+}
+
+// The in-edges after the first kXLight of each row, in chunks: at most
+// E / kXLight entries.
+__global__ void __launch_bounds__(kNT)
+    k_expand_list(const int32_t *csc_off, int nV, int2 *list, int32_t *n) {
+  for (int v = blockIdx.x * kNT + threadIdx.x; v < nV; v += gridDim.x * kNT) {
+    const int off = csc_off[v], rest = csc_off[v + 1] - off - kXLight;
+    if (rest <= 0) continue;
+    const int nc = (rest + kXChunk - 1) / kXChunk;
+    const int at = atomicAdd(n, nc);
+    for (int k = 0; k < nc; ++k) list[at + k] = make_int2(v, off + kXLight + k * kXChunk);
+  }
+}
+
+// Sets the next-frontier bit of every out-neighbour of a marked vertex: by
+// push, or by pull where the marked vertices have more than 1 / kXPullDiv of
+// the edges: a push is bound by the reductions on words that several SMs fill
+// at once, a pull has one per word and reads a few in-edges per vertex.  A
+// pull that looked at more than 1 / kXMissDiv of the in-edges in vain makes
+// the next kXWait iterations push.  us per run, push only (rows and chunks in
+// a kernel each) / with 1/2, 1/4, 1/8, 1/16: the reference's PageRank on
+// R-MAT 200 K, 3 M edges 3712 / 3010, 2933, 2901, 2900; 20 K 1797 / 1478,
+// 1431, 1420, 1448; Erdos-Renyi 200 K 1785 / 1371, 1349, 1331, 1369; run()
+// on R-MAT 2^18, CC 418 / 391, 374, 373, -, BFS 217 / 193, 173, 171, -; SSSP on
+// R-MAT 2^21 4309 / 4088, 4078, 4091, 4166.  CC on R-MAT 2^14 with 200 grid
+// islands, whose pulls would miss: 2147 / 2252, 2271, 2293, and 2200 with the
+// rule on misses.
+constexpr int kXPullDiv = 8;
+constexpr int kXMissDiv = 4;
+constexpr int kXWait = 16;
+__global__ void __launch_bounds__(kNT)
+    k_expand(const int32_t *act, const gas_counters *cnt, const uint8_t *ret,
+             const int32_t *csr_off, const int32_t *csr_dst, const int32_t *csc_off,
+             const int32_t *csc_src, int nV, int nE, const uint32_t *changed, const int2 *chunks,
+             ExpandCtl *ctl, const int2 *list, const int32_t *n_list, uint32_t *bits) {
+  __shared__ int s_start[kNT / 32][32], s_excl[kNT / 32][32];
+  const bool marked = expand_may_pull(cnt, ctl, list, nE);
+  if (marked && (long long)ctl->n_edges * kXPullDiv > nE) {
+    expand_pull(csc_off, csc_src, changed, nV, list, *n_list, bits, &ctl->missed);
+    return;
+  }
+  if (marked) {  // the light rows are still to be pushed
+    const int n = cnt->n_active, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
+    for (long long base = 32LL * ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); base < n;
+         base += 32LL * nwarps) {
+      const long long i = base + lane;
+      int off = 0, deg = 0;
+      if (i < n && ret[i]) {
+        const int v = act[i];
+        off = csr_off[v];
+        deg = csr_off[v + 1] - off;
+      }
+      expand_light(off, deg, csr_dst, bits, s_start[warp], s_excl[warp]);
+    }
+  }
+  expand_chunks(chunks, ctl->n_chunks, csr_dst, bits);
 }
 
 // Compaction of the next-frontier bitmap into the ascending active list with
@@ -380,14 +531,15 @@ __device__ __forceinline__ void c_round_load(uint32_t myword, const int32_t *csc
 }
 
 // Members and in-edges per block (part) and per warp (wpart); also takes
-// the expansion's out-edge count and clears its control word.
+// the expansion's out-edge count and clears its control word and marks.
 __global__ void __launch_bounds__(kNT)
-    k_compact_count(const uint32_t *bits, const int32_t *csc_off, int nW, int2 *part,
-                    int2 *wpart, ExpandCtl *ctl, gas_counters *cnt) {
+    k_compact_count(const uint32_t *bits, uint32_t *changed, const int32_t *csc_off, int nW, int nE,
+                    int2 *part, int2 *wpart, ExpandCtl *ctl, gas_counters *cnt) {
   __shared__ int2 s_t[kCWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int w0 = (blockIdx.x * kCWarps + warp) * kCWords;
   const uint32_t myword = lane < kCWords && w0 + lane < nW ? bits[w0 + lane] : 0u;
+  if (lane < kCWords && w0 + lane < nW) changed[w0 + lane] = 0u;
   const unsigned nz = __ballot_sync(0xffffffffu, myword != 0u);
   int c = __popc(myword), d = 0;
 #pragma unroll 1
@@ -419,6 +571,8 @@ __global__ void __launch_bounds__(kNT)
       cnt->n_scatter_edges = ctl->n_edges;
       ctl->n_edges = 0;
       ctl->n_chunks = 0;
+      ctl->wait = (long long)ctl->missed * kXMissDiv > nE ? kXWait : max(ctl->wait - 1, 0);
+      ctl->missed = 0;
     }
   }
 }
@@ -790,17 +944,21 @@ gas_status_t scatter_common(gas_engine *e, void *stream, const LoopEnd &end) {
   e->slots_pending = false;
   ExpandCtl *ctl = static_cast<ExpandCtl *>(e->xctl);
   int2 *chunks = static_cast<int2 *>(e->xchunks);
+  const int2 *list = static_cast<const int2 *>(e->xlist);
   // the active and chunk counts are only known on the device: fixed grids
-  k_expand_rows<<<grid_for(e->nV, kNT, 8 * e->num_sms), kNT, 0, S(stream)>>>(
-      e->act, e->cnt, e->ret, e->csr_off, e->csr_dst, e->bits, slot, (uint8_t *)e->vd,
-      (int)e->vbytes, chunks, ctl);
-  k_expand_chunks<<<grid_for(e->nE / kXLight, kNT / 32, 8 * e->num_sms), kNT, 0, S(stream)>>>(
-      chunks, ctl, e->csr_dst, e->bits);
+  k_expand_mark<<<grid_for(e->nV, kNT, 8 * e->num_sms), kNT, 0, S(stream)>>>(
+      e->act, e->cnt, e->ret, e->csr_off, e->csr_dst, e->changed, e->bits, slot,
+      (uint8_t *)e->vd, (int)e->vbytes, chunks, list, e->nE, ctl);
+  k_expand<<<grid_for(std::max<int64_t>(e->nV, e->nE / 2), kNT, 8 * e->num_sms), kNT, 0,
+             S(stream)>>>(e->act, e->cnt, e->ret, e->csr_off, e->csr_dst, e->csc_off, e->csc_src,
+                          e->nV, e->nE, e->changed, chunks, ctl,
+                          list, e->xlist_n, e->bits);
   CUDA_TRY(cudaGetLastError());
   const int nW = (e->nV + 31) / 32, nb = e->n_cblocks;
   int2 *part = static_cast<int2 *>(e->cpart), *wpart = part + nb;
   const int tile = e->prog == GAS_PROG_USER ? 0 : kBuiltinTile;  // users partition themselves
-  k_compact_count<<<nb, kNT, 0, S(stream)>>>(e->bits, e->csc_off, nW, part, wpart, ctl, e->cnt);
+  k_compact_count<<<nb, kNT, 0, S(stream)>>>(e->bits, e->changed, e->csc_off, nW, e->nE, part, wpart,
+                                             ctl, e->cnt);
   if (nb > kCSumBlocks) k_compact_spine<<<1, kNT, 0, S(stream)>>>(part, nb);
   k_compact_write<<<nb, kNT, 0, S(stream)>>>(e->bits, e->csc_off, nW, part, wpart,
                                              nb > kCSumBlocks ? 1 : 0, e->act, e->scan,
@@ -997,6 +1155,7 @@ gas_status_t gas_engine_set_graph(gas_engine *e, int32_t nV, void *vertex_data,
   plan.add((uint8_t **)&e->slot, V * e->vbytes);
   plan.add((uint8_t **)&e->gres, V * std::max<size_t>(e->gbytes, 4));
   plan.add(&e->bits, nW);
+  plan.add(&e->changed, nW);
   // smallest tile is kNT * 2 items (gather values larger than 16 bytes)
   const int64_t min_tile = kNT * 2;
   e->tile_cap = (int32_t)(((int64_t)V + (int64_t)E + min_tile - 1) / min_tile + 1);
@@ -1008,6 +1167,11 @@ gas_status_t gas_engine_set_graph(gas_engine *e, int32_t nV, void *vertex_data,
   // a row of d > kXLight out-edges lists ceil(d / kXChunk) <= d / kXLight chunks
   plan.add((int2 **)&e->xchunks, E / kXLight + 1);
   plan.add((ExpandCtl **)&e->xctl, 1);
+  e->xlist = nullptr;  // in-edges in host memory are not looked through
+  if (!e->edges_on_host && !e->graph_only) {
+    plan.add((int2 **)&e->xlist, E / kXLight + 1);
+    plan.add(&e->xlist_n, 1);
+  }
   e->n_cblocks = (int32_t)std::max<size_t>(1, (nW + kCBlockWords - 1) / kCBlockWords);
   // block totals, then the blocks' per-warp totals
   plan.add((int2 **)&e->cpart, (size_t)e->n_cblocks * (1 + kCWarps));
@@ -1080,6 +1244,12 @@ gas_status_t gas_engine_set_graph(gas_engine *e, int32_t nV, void *vertex_data,
   if (V)
     CUDA_TRY(cudaMemcpyAsync(e->vd, vertex_data, V * e->vbytes, cudaMemcpyHostToDevice, st));
   CUDA_TRY(cudaMemsetAsync(e->bits, 0, nW * 4, st));
+  CUDA_TRY(cudaMemsetAsync(e->changed, 0, nW * 4, st));
+  if (e->xlist) {
+    CUDA_TRY(cudaMemsetAsync(e->xlist_n, 0, sizeof(int32_t), st));
+    k_expand_list<<<grid_for(nV, kNT, 8 * e->num_sms), kNT, 0, st>>>(
+        e->csc_off, nV, static_cast<int2 *>(e->xlist), e->xlist_n);
+  }
   CUDA_TRY(cudaMemsetAsync(e->xctl, 0, sizeof(ExpandCtl), st));
   CUDA_TRY(cudaMemsetAsync(e->slab_fix_n, 0, sizeof(int32_t), st));
   CUDA_TRY(cudaMemsetAsync(e->hist, 0, 8 * sizeof(int32_t), st));
@@ -1119,7 +1289,7 @@ gas_status_t gas_engine_set_active(gas_engine *e, int32_t start, int32_t end,
   }
   const int n = end - start;
   k_set_range<<<grid_for((int64_t)n + 1, kNT, 8 * e->num_sms), kNT, 0, S(stream)>>>(
-      start, n, e->csc_off, e->act, e->scan, e->cnt);
+      start, n, e->csc_off, e->act, e->scan, e->cnt, &static_cast<ExpandCtl *>(e->xctl)->wait);
   CUDA_TRY(cudaGetLastError());
   e->tpart_valid = false;
   e->n_active = n;

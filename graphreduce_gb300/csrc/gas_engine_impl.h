@@ -112,6 +112,9 @@ struct gas_engine {
   uint8_t *ret = nullptr;
   void *slot = nullptr, *gres = nullptr;
   uint32_t *bits = nullptr;
+  void *xlist = nullptr;       // in-edges past the first of each row, in chunks
+  int32_t *xlist_n = nullptr;
+  uint32_t *changed = nullptr;  // expansion: vertices whose apply returned true
   void *tile_first = nullptr, *tile_carry = nullptr;
   int32_t *tile_a0 = nullptr;
   int32_t tile_cap = 0;
