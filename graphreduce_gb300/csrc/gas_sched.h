@@ -40,6 +40,14 @@ constexpr size_t kSmallWithGraph = (size_t)16 << 20;
 SmallBytes bfs_small_bytes(int64_t nV, int64_t nE);
 SmallBytes min_small_bytes(int64_t nV, int64_t nE);
 
+// Launches such a kernel as a cooperative grid with a CTA per kCtaEdges
+// vertices and edges; where that is at most cluster_upto CTAs, as one cluster
+// of up to kClusterMost.
+constexpr int kCtaEdges = 2048;  // 8192 and more: 1.3x and more slower below 100 K edges
+constexpr int kClusterMost = 16;
+cudaError_t launch_small(void *grid_fn, void *cluster_fn, int cluster_upto, const gas_engine *e,
+                         void **args, cudaStream_t s);
+
 // BFS on a graph of at most kBfsSmallMaxV vertices as one cooperative
 // kernel (gas_small.cu): same depths and iteration count as run_fast.
 // reserve: the kernel's buffers, kept with the graph; false if there is no

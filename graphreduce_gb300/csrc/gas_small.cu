@@ -65,10 +65,11 @@ constexpr int kSbAlone = 29;        // in-edges a thread looks at alone
 // on while the frontier grows or holds more than V/beta vertices.
 constexpr int kSbAlpha = 14;
 constexpr int kSbBeta = 24;
+constexpr int kSbCluster = 128;     // CTAs asked for up to which a cluster is enough (R-MAT
+                                    // 16 K, 110 CTAs: 60 us against 68; 65 K, 450: 82 and 82)
 constexpr int kSbDense = 2;         // out-edges per thread of the grid from which a
                                     // top-down level's finds are not queued (1 to 4
                                     // within 2 % of one another)
-constexpr int kSbCtaEdges = 2048;   // vertices and edges per CTA, as in gas_small_min.cu
 
 using gasgrid::warp_add;
 
@@ -226,7 +227,7 @@ __device__ __forceinline__ void sb_pull(const Bfs &g, const uint32_t *F, uint32_
   }
 }
 
-template <bool kCount>
+template <bool kCount, bool kCluster>
 __global__ void __launch_bounds__(kSbNT, 1)
     k_bfs_small(Bfs g, const int32_t *__restrict__ act, int n_act, uint32_t *bits, Queue qa,
                 Queue qb, int nW, long long nE, int forced, int max_iter, SmallCtl *c,
@@ -236,9 +237,10 @@ __global__ void __launch_bounds__(kSbNT, 1)
   // does not run)
 #define SB_SYNC(out, from)                                                       \
   do {                                                                           \
-    if (!gasgrid::barrier_with(&c->bar, bar, &(out), [&] {                       \
-          return __ldcg(reinterpret_cast<const int4 *>(from));                   \
-        })) {                                                                    \
+    const auto load = [&] { return __ldcg(reinterpret_cast<const int4 *>(from)); }; \
+    if constexpr (kCluster) {                                                    \
+      gasgrid::cluster_barrier_with(&(out), load);                               \
+    } else if (!gasgrid::barrier_with(&c->bar, bar, &(out), load)) {             \
       if (threadIdx.x == 0) atomicExch(&cnt->error, (int)GAS_ERR_DEVICE);        \
       return;                                                                    \
     }                                                                            \
@@ -369,6 +371,32 @@ __global__ void __launch_bounds__(kSbNT, 1)
 
 namespace gas {
 
+cudaError_t launch_small(void *grid_fn, void *cluster_fn, int cluster_upto, const gas_engine *e,
+                         void **args, cudaStream_t s) {
+  const int64_t want = std::max<int64_t>(1, ((int64_t)e->nV + e->nE) / kCtaEdges);
+  if (want <= cluster_upto) {
+    const int n = (int)std::min<int64_t>(want, kClusterMost);
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = n;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(n);
+    cfg.blockDim = dim3(kNT);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaError_t ce = n > 8 ? cudaFuncSetAttribute(
+                                 cluster_fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)
+                           : cudaSuccess;
+    if (ce == cudaSuccess) ce = cudaLaunchKernelExC(&cfg, cluster_fn, args);
+    if (ce == cudaSuccess) return ce;
+    cudaGetLastError();  // no room for such a cluster: a cooperative grid
+  }
+  return cudaLaunchCooperativeKernel(grid_fn, dim3((int)std::min<int64_t>(want, e->num_sms)),
+                                     dim3(kNT), args, 0, s);
+}
+
 bool bfs_small_eligible(const gas_engine *e, gas_schedule_t schedule) {
   const char *v = getenv("GAS_BFS_SMALL");
   if (v && v[0] == '0') return false;
@@ -403,9 +431,6 @@ gas_status_t run_bfs_small(gas_engine *e, gas_schedule_t schedule, int32_t max_i
   const size_t V = (size_t)e->nV, H = heavy_cap(e->nE);
   SmallCtl *ctl = static_cast<SmallCtl *>(e->sb_ctl);
   const bool count = e->profiling;
-  void *fn = count ? (void *)k_bfs_small<true> : (void *)k_bfs_small<false>;
-  const int grid = (int)std::max<int64_t>(
-      1, std::min<int64_t>(e->num_sms, ((int64_t)e->nV + e->nE) / kSbCtaEdges));
   // the kernel leaves its bitmaps and control word clear; they are cleared
   // here after allocation, after a run that failed, and when bytes count
   if (!e->sb_clean || count) {
@@ -425,7 +450,9 @@ gas_status_t run_bfs_small(gas_engine *e, gas_schedule_t schedule, int32_t max_i
   int max_iter = max_iterations;
   void *args[] = {&g, &act, &n_act, &bits, &qa, &qb, &nw, &nE, &forced, &max_iter, &ctl, &cnt};
   if (count) prof_begin(e, s, kProfPush, 0);
-  CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kSbNT), args, 0, s));
+  CUDA_TRY(launch_small(count ? (void *)k_bfs_small<true, false> : (void *)k_bfs_small<false, false>,
+                        count ? (void *)k_bfs_small<true, true> : (void *)k_bfs_small<false, true>,
+                        kSbCluster, e, args, s));
   prof_end(e, s);
   if (count) {
     SmallCtl h;

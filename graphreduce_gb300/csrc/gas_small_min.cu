@@ -58,7 +58,8 @@ namespace {
 
 using namespace gasstage;
 
-constexpr int kCtaEdges = 2048;   // 8192 and more: 1.3x and more slower below 100 K edges
+constexpr int kMinCluster = 32;   // CTAs asked for up to which a cluster is enough (R-MAT
+                                  // 4 K, 60 CTAs: 117 us against 113)
 constexpr int kDense = 8;         // 2: 4 % slower on Erdos-Renyi 65 K, even on R-MAT
 
 struct MinCtl {
@@ -133,7 +134,7 @@ __device__ __forceinline__ void walk(const int4 *Q, int nq, int most, int w0,
   }
 }
 
-template <bool kWeighted>
+template <bool kWeighted, bool kCluster>
 __global__ void __launch_bounds__(kNT, 1)
     k_min_small(const int32_t *__restrict__ csr_off, const int32_t *__restrict__ csr_dst,
                 const int32_t *__restrict__ csr_w, int32_t *vd, int32_t *vd2, Queue qa, Queue qb,
@@ -142,9 +143,12 @@ __global__ void __launch_bounds__(kNT, 1)
   // leaves
 #define MIN_SYNC(next)                                                            \
   do {                                                                            \
-    if (!gasgrid::barrier_with(&c->bar, bar, &head, [&] {                         \
-          return __ldcg(reinterpret_cast<const int4 *>(&c->q[(next) % 3]));       \
-        })) {                                                                     \
+    const auto load = [&] {                                                       \
+      return __ldcg(reinterpret_cast<const int4 *>(&c->q[(next) % 3]));           \
+    };                                                                            \
+    if constexpr (kCluster) {                                                     \
+      gasgrid::cluster_barrier_with(&head, load);                                 \
+    } else if (!gasgrid::barrier_with(&c->bar, bar, &head, load)) {               \
       if (threadIdx.x == 0) atomicExch(&cnt->error, (int)GAS_ERR_DEVICE);         \
       return;                                                                     \
     }                                                                             \
@@ -285,10 +289,9 @@ gas_status_t run_min_small(gas_engine *e, int32_t max_iterations, gas_run_stats 
   gas_counters *cnt = e->cnt;
   void *args[] = {&csr_off, &csr_dst, &csr_w, &vd, &vd2, &qa, &qb, &nV, &zero_cap,
                   &max_iterations, &ctl, &cnt};
-  void *fn = weighted ? (void *)k_min_small<true> : (void *)k_min_small<false>;
-  const int grid = (int)std::max<int64_t>(
-      1, std::min<int64_t>(e->num_sms, ((int64_t)e->nV + e->nE) / kCtaEdges));
-  CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kNT), args, 0, s));
+  CUDA_TRY(launch_small(weighted ? (void *)k_min_small<true, false> : (void *)k_min_small<false, false>,
+                        weighted ? (void *)k_min_small<true, true> : (void *)k_min_small<false, true>,
+                        kMinCluster, e, args, s));
   GAS_TRY(engine_sync_counts(e, stream));
   const gas_counters c = *e->h_cnt;
   e->sm_clean = c.error == 0 || c.error == GAS_ERR_ITER_CAP;
