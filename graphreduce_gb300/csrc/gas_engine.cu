@@ -791,9 +791,8 @@ void free_graph(gas_engine *e) {
   for (void **p : e->arena_ptrs) *p = nullptr;
   e->arena_ptrs.clear();
   dfree(e->arena);
-  for (int i = 0; i < 2; ++i) { dfree(e->pr_rank[i]); dfree(e->pr_contrib[i]); }
-  dfree(e->pr_seed); dfree(e->pr_inv_deg); dfree(e->pr_l1); dfree(e->csr_to_csc);
-  e->pr_tiles.free();
+  dfree(e->csr_to_csc);
+  e->pr_mem.free();
   e->pr_hot_mem.free();
   e->pr_hot_n = 0;
   e->pr_hot_known = false;

@@ -132,12 +132,11 @@ struct gas_engine {
   int32_t *pr_seed = nullptr;  // personalization seed of the run (-1: none)
   float *pr_inv_deg = nullptr;  // [V] RN(1 / out-degree) (0: none)
   double *pr_l1 = nullptr;
-  int32_t pr_l1_cap = 0;
   // tiles of the in-edges: rows ended before each, head and tail carry records
   int32_t *pr_tile_row = nullptr;
   void *pr_head = nullptr, *pr_tail = nullptr;
   uint32_t *pr_end_bits = nullptr;  // the last in-edges of the rows
-  DeviceGroup pr_tiles;
+  DeviceGroup pr_mem;
   // hot sources of the graph (gas_runs.cu): their numbers, the iteration's
   // contributions, the in-edges with their slots
   void *pr_hot_ctl = nullptr;

@@ -401,6 +401,8 @@ __device__ __forceinline__ void block_sum_store(double v, double *out) {
 // 47.3.
 constexpr int kPrK = 8;
 constexpr int kPrCtas = 4;
+constexpr int kPrCtasMost = 8;     // gather CTAs per SM, and with the join's, which
+constexpr int kPrPartsPerSm = 24;  // each leave a part of the residual
 constexpr int kPrW = 32 * kPrK;
 // s_val is padded by one word per kPrK: a lane reads about kPrK words past
 // its neighbour, which without the pad puts 32 / kPrK lanes on one bank
@@ -935,20 +937,17 @@ gas_status_t pagerank_run(gas_engine *e, double damping, double tol, int32_t max
   const int nV = e->nV;
   if (nV == 0) return GAS_OK;
   if (seed >= nV) return gas::fail(GAS_ERR_INVALID, "seed %d outside [0, %d)", seed, nV);
-  for (int i = 0; i < 2; ++i) {
-    if (!e->pr_rank[i]) CUDA_TRY(cudaMalloc(&e->pr_rank[i], (size_t)nV * 4));
-    if (!e->pr_contrib[i]) CUDA_TRY(cudaMalloc(&e->pr_contrib[i], (size_t)nV * 4));
-  }
-  if (!e->pr_seed) CUDA_TRY(cudaMalloc(&e->pr_seed, sizeof(int32_t)));
-  if (!e->pr_inv_deg) CUDA_TRY(cudaMalloc(&e->pr_inv_deg, (size_t)nV * 4));
   PrCtx c;
   c.n_tiles = (int)(((long long)e->nE + kPrW - 1) / kPrW);
   if (!e->pr_tile_row) {  // once per graph
-    const size_t words = (size_t)c.n_tiles * (kPrW / 32);
-    CUDA_TRY(e->pr_tiles.alloc({GROUP_PART(e->pr_tile_row, (size_t)c.n_tiles * 4),
-                                GROUP_PART(e->pr_head, (size_t)c.n_tiles * sizeof(PrCarry)),
-                                GROUP_PART(e->pr_tail, (size_t)c.n_tiles * sizeof(PrCarry)),
-                                GROUP_PART(e->pr_end_bits, words * 4)}));
+    const size_t T = (size_t)c.n_tiles, words = T * (kPrW / 32), v = (size_t)nV * 4;
+    CUDA_TRY(e->pr_mem.alloc(
+        {GROUP_PART(e->pr_rank[0], v), GROUP_PART(e->pr_rank[1], v),
+         GROUP_PART(e->pr_contrib[0], v), GROUP_PART(e->pr_contrib[1], v),
+         GROUP_PART(e->pr_inv_deg, v), GROUP_PART(e->pr_seed, sizeof(int32_t)),
+         GROUP_PART(e->pr_l1, sizeof(double) * (kPrPartsPerSm * (size_t)e->num_sms + 2)),
+         GROUP_PART(e->pr_tile_row, T * 4), GROUP_PART(e->pr_head, T * sizeof(PrCarry)),
+         GROUP_PART(e->pr_tail, T * sizeof(PrCarry)), GROUP_PART(e->pr_end_bits, words * 4)}));
     CUDA_TRY(cudaMemsetAsync(e->pr_end_bits, 0, words * 4, S(stream)));
     k_pr_tiles<<<gas::engine_grid(std::max({c.n_tiles, e->n_ne, 1}), kNT, 8 * e->num_sms), kNT, 0,
                  S(stream)>>>(e->ne_end, e->n_ne, c.n_tiles, e->pr_tile_row, e->pr_end_bits);
@@ -964,20 +963,15 @@ gas_status_t pagerank_run(gas_engine *e, double damping, double tol, int32_t max
   else
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pr_gather<false>, kNT,
                                                            kNT / 32 * sizeof(PrStage)));
-  c.merge_grid = e->num_sms * (per_sm > 0 ? per_sm : 1);  // resident CTAs only
+  // resident CTAs only, and none without a tile
+  const int warps = c.n_hot ? kHotWarps : kNT / 32;
+  c.merge_grid = std::max(1, std::min(e->num_sms * std::min(std::max(per_sm, 1), kPrCtasMost),
+                                      (c.n_tiles + warps - 1) / warps));
   // a thread per tile record, at most 16 CTAs per SM: the records' loads
   // are dependent chains, so they want many threads in flight
-  c.fix_grid = (int)std::min<long long>(16LL * e->num_sms,
+  c.fix_grid = (int)std::min<long long>((long long)(kPrPartsPerSm - kPrCtasMost) * e->num_sms,
                                         std::max(1, std::max(c.n_tiles, nV / 4) / kNT + 1));
   const int nparts = c.merge_grid + c.fix_grid;
-  if (!e->pr_l1 || e->pr_l1_cap < nparts + 2) {
-    if (e->pr_l1) cudaFree(e->pr_l1);
-    e->pr_l1 = nullptr;
-    if (e->graphs[kGraphPagerank]) cudaGraphExecDestroy(e->graphs[kGraphPagerank]);
-    e->graphs[kGraphPagerank] = nullptr;
-    e->pr_l1_cap = nparts + 2;
-    CUDA_TRY(cudaMalloc(&e->pr_l1, sizeof(double) * (size_t)e->pr_l1_cap));
-  }
   c.residual = e->pr_l1 + nparts;
   c.pol.csc_src = c.n_hot ? e->pr_hot_src : e->csc_src;
   c.pol.inv_deg = e->pr_inv_deg;
