@@ -72,13 +72,14 @@ constexpr int kBfsSmallMaxV = 1 << 24;
 // records per iteration, only up to this many.
 constexpr int kBfsSmallRecordsMaxV = 1 << 18;
 // SSSP and CC from the full active set likewise (figures in
-// gas_small_min.cu): under AUTO up to 2^21 vertices; the kernel still halves
-// the fixed heuristic's time at 2^22, but from there on LEARNED's
-// multi-kernel push is the faster schedule and the heuristic stays what it
-// is compared with.  Under LEARNED up to 2^20: at 2^21 the multi-kernel push
-// wins on R-MAT CC (731 against 824 us).
-constexpr int kMinSmallMaxV = 1 << 21;
-constexpr int kMinSmallLearnedMaxV = 1 << 20;
+// gas_small_min.cu): under AUTO below 2^22 vertices; the kernel still halves
+// the fixed heuristic's time there, but from there on LEARNED's multi-kernel
+// push is the faster schedule and the heuristic stays what it is compared
+// with.  Under LEARNED up to 2^21 for SSSP (901 against 978 us on R-MAT,
+// Erdos-Renyi 2092 against 2367), to 2^20 for CC (at 2^21 824 against 731).
+constexpr int kMinSmallMaxV = (1 << 22) - 1;
+constexpr int kSsspSmallLearnedMaxV = 1 << 21;
+constexpr int kCcSmallLearnedMaxV = 1 << 20;
 
 // Instantiated CUDA graphs cached per engine (valid until the next
 // set_graph, since their kernels capture the engine's buffers).

@@ -1056,8 +1056,8 @@ void reserve_fast_buffers(gas_engine *e) {
     return;
   }
   const bool sized = (e->prog == GAS_PROG_BFS && e->nV > kBfsSmallRecordsMaxV) ||
-                     ((e->prog == GAS_PROG_SSSP || e->prog == GAS_PROG_CC) &&
-                      e->nV > kMinSmallLearnedMaxV);
+                     (e->prog == GAS_PROG_SSSP && e->nV > kSsspSmallLearnedMaxV) ||
+                     (e->prog == GAS_PROG_CC && e->nV > kCcSmallLearnedMaxV);
   if (!sized) return;
   if (ensure_fast_buffers(e) != GAS_OK) {  // tight memory: the first run asks again
     e->fast_mem.free();

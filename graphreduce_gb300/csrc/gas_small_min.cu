@@ -249,8 +249,9 @@ bool min_small_eligible(const gas_engine *e, gas_schedule_t schedule) {
   // per-iteration records and kernel times come from the multi-kernel loop
   if (e->trace_on || e->profiling || e->edges_on_host) return false;
   if (!e->active_full || e->counts_dirty || e->n_active != e->nV) return false;
-  return e->nV > 0 &&
-         e->nV <= (schedule == GAS_SCHED_AUTO ? kMinSmallMaxV : kMinSmallLearnedMaxV);
+  const int learned =
+      e->prog == GAS_PROG_SSSP ? kSsspSmallLearnedMaxV : kCcSmallLearnedMaxV;
+  return e->nV > 0 && e->nV <= (schedule == GAS_SCHED_AUTO ? kMinSmallMaxV : learned);
 }
 
 SmallBytes min_small_bytes(int64_t nV, int64_t nE) {

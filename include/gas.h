@@ -247,8 +247,9 @@ typedef enum {
                            /* sequentially in CSC order (parity mode)      */
   GAS_SCHED_LEARNED = 5    /* push or pull per iteration from the engine's */
                            /* schedule model (gas_engine_set_schedule_model) */
-  /* SSSP and CC from the full active set: graphs of up to 2^21 (AUTO) or
-   * 2^20 (LEARNED) vertices run as one cooperative kernel that pushes in
+  /* SSSP and CC from the full active set: graphs of less than 2^22 (AUTO) or
+   * up to 2^21 (SSSP, LEARNED) or 2^20 (CC, LEARNED) vertices run as one
+   * kernel, a cooperative grid or a thread-block cluster, that pushes in
    * every iteration; with tracing or profiling on, and for other active
    * sets, the per-iteration choice is made as stated. */
 } gas_schedule_t;

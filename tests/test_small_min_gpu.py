@@ -95,7 +95,7 @@ def test_one_kernel_equals_the_push_and_the_oracle(program, name):
     eng.close()
 
 
-@pytest.mark.parametrize("schedule,nV,one", [("auto", 1 << 21, True), ("auto", (1 << 21) + 1, False),
+@pytest.mark.parametrize("schedule,nV,one", [("auto", (1 << 22) - 1, True), ("auto", 1 << 22, False),
                                              ("learned", 1 << 20, True),
                                              ("learned", (1 << 20) + 1, False)])
 def test_size_limits(schedule, nV, one):
