@@ -66,8 +66,9 @@ struct DeviceGroup {
 // The engine object.
 // ---------------------------------------------------------------------------
 // BFS runs on graphs up to this many vertices take the one-kernel path
-// (figures in gas_small.cu; measured to 2^24, where it is 15 to 25 % faster).
-constexpr int kBfsSmallMaxV = 1 << 24;
+// (figures in gas_small.cu: on every graph measured to this size the faster
+// one; at 2^24 it wins on R-MAT and loses on some Erdos-Renyi graphs).
+constexpr int kBfsSmallMaxV = 1 << 23;
 // ... but with tracing or profiling on, to which the multi-kernel loop gives
 // records per iteration, only up to this many.
 constexpr int kBfsSmallRecordsMaxV = 1 << 18;

@@ -1,4 +1,4 @@
-// gas_small.cu -- BFS on graphs of up to 2^24 vertices as one persistent
+// gas_small.cu -- BFS on graphs of up to 2^23 vertices as one persistent
 // kernel.
 //
 // A BFS level is a few microseconds to some tens of them, and the fast
@@ -32,17 +32,19 @@
 // level (-1) only repeats a claim that fails.  The barrier's wait is bounded:
 // past the limit every CTA leaves the kernel with an error.
 //
-// Up to about 2^20 vertices bound by the latency of a level's chain (5 to
-// 10 us), beyond by L2 lookups (a depth per edge of a top-down level, a depth
-// and a frontier bit per vertex of a bottom-up one).  Measured, us per run
-// (one kernel with a warp per bitmap word and two barriers a top-down level
-// up to 2^18 vertices, the multi-kernel loop above them / here): R-MAT, 8 edges per vertex, 1 K 90 / 65, 16 K 108 / 69, 65 K 128 /
-// 79, 250 K 178 / 89, 600 K 175 / 98, 1 M 203 / 104, 16 per vertex 4 M 317 /
-// 194; Erdos-Renyi 100 K 138 / 83, 600 K 242 / 113, 2 M 257 / 160.  Above the
-// old line over three sources, multi-kernel / here: R-MAT 4 M 283-335 /
-// 186-200, directed 280-300 / 186-210, 8 M 421-455 / 313-360, 16.8 M 687-813 /
-// 537-692; Erdos-Renyi 4 M 424-458 / 255-270, 8 M 605-919 / 471-618; so the
-// line is the largest size measured.
+// Bound by latency at every size: on R-MAT 65 K the warps wait at barriers (45
+// cycles an issue; a level's chain is 5 to 10 us), on R-MAT 4 M for loads (12)
+// and at barriers (11), with L1 at 17 % and L2 at 11 % of their peaks.
+// Measured, us per run (before / here; before: one kernel with a warp per
+// bitmap word and two barriers a top-down level up to 2^18 vertices, the
+// multi-kernel loop above): R-MAT, 8 edges per vertex, 1 K 90 / 65, 16 K 108 /
+// 69, 65 K 128 / 79, 250 K 178 / 89, 600 K 175 / 98, 1 M 203 / 104, 16 per
+// vertex 4 M 317 / 194; Erdos-Renyi 100 K 138 / 83, 600 K 242 / 113, 2 M 257 /
+// 160.  Above the old line over three or four graphs each, multi-kernel / here:
+// R-MAT 4 M 283-335 / 186-200, directed 280-300 / 186-210, 8 M 421-455 /
+// 313-360; Erdos-Renyi 4 M 424-473 / 252-271, 8 M 605-919 / 471-618.  Past the
+// line, at 2^24: R-MAT 692-814 / 492-692, Erdos-Renyi 8 edges per vertex
+// 1364-1448 / 1010-1059, but 16 per vertex 1040-1056 / 1242-1391.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -235,7 +235,7 @@ gas_status_t gas_engine_download_vertex_data_async(gas_engine *e, void *dst,
  * previous level), and AUTO and LEARNED both take Beamer, Asanovic and
  * Patterson's direction rule (SC'12; bottom-up once the frontier's out-edges
  * exceed 1/14 of the edges not yet explored, top-down again once it shrinks
- * below V/24 vertices).  Graphs of up to 2^24 vertices run as one cooperative
+ * below V/24 vertices).  Graphs of up to 2^23 vertices run as one cooperative
  * kernel under every schedule but PUSH (of up to 2^18 with tracing or
  * profiling on). */
 typedef enum {

@@ -130,7 +130,7 @@ def test_vertices_visited_before_the_run_stay():
         assert (vd[visited] == 7).all() and st.iterations == wst.iterations
 
 
-@pytest.mark.parametrize("nV,one_kernel", [(1 << 24, True), ((1 << 24) + 1, False)])
+@pytest.mark.parametrize("nV,one_kernel", [(1 << 23, True), ((1 << 23) + 1, False)])
 def test_largest_graph(nV, one_kernel):
     rng = np.random.default_rng(4)
     hops = np.sort(rng.choice(nV, 60, replace=False))
