@@ -84,12 +84,6 @@ DRAM_PER_LAUNCH = {
     ("mss_push", "rmat-s22"): 814.0e6,
     # CC push, mean over the 63 launches of the same step (same profile)
     ("push", "rmat-s22-cc"): 103.2e6,
-    # k_pr_merge + k_pr_merge_fix, one iteration at scale 24
-    # (profiles/k_pr_merge_pagerank_rmat-s24.md)
-    ("pr_gather", "rmat-s24"): 1.647e9,
-    # k_ppr_pieces + k_ppr_fix, one PPR iteration of the 64-graph batch
-    # (profiles/k_ppr_pieces_batched-8graphs.md)
-    ("ppr_iteration", "batched-64"): 10.30e9,
 }
 
 
@@ -169,12 +163,12 @@ LIMITER = {
                 "algorithmic bytes are L2 hits (profiles/k_mss_push_sssp8-batched_rmat-s20.md)",
     "push": "latency of dependent loads per light row with 93 % of warp slots occupied; "
             "L2 tags 36 %, DRAM 25 % (profiles/k_push_cc-islands_rmat-s20.md)",
-    "pr_gather": "L1 data pipe (70 %): one wavefront per random contribution gather; DRAM "
-                 "18 % (profiles/k_pr_merge_pagerank_rmat-s24.md)",
-    "ppr_iteration": "latency of the 64-byte contribution-row gathers, 62 % of warp slots "
-                     "occupied (profiles/k_ppr_pieces_batched-8graphs.md)",
-    "bfs_small": "latency: one cooperative kernel, a few microseconds per level, the graph in "
-                 "L2 (profiles/k_bfs_small_bfs_rmat-s16.md)",
+    "pr_gather": "L1 data pipe (68 %): a wavefront per random contribution that is not a hot "
+                 "source's (profiles/k_pr_gather_pagerank_rmat-s22.md)",
+    "ppr_iteration": "L1 data pipe (70 %) of the 64-byte contribution-row gathers, most of them "
+                     "L2 hits (profiles/captures_small-and-batched.md)",
+    "bfs_small": "latency: one kernel, a few microseconds per level, the graph in L2 "
+                 "(profiles/captures_small-and-batched.md)",
 }
 
 
@@ -818,7 +812,7 @@ def run_c1(args, model):
             "identical_to_builtin": bool(np.array_equal(up["bfs_depth"], depth))
             and up["bfs_levels"] == last["learned"].iterations}
     if p.pull_launches == 0 and p.push_launches == 1:  # graphs of up to 2^18 vertices
-        roof = roofline("k_bfs_small (every level in one cooperative kernel)", "bfs_small",
+        roof = roofline("k_bfs_small (every level in one kernel)", "bfs_small",
                         p.push_bytes, p.push_ms, 1, "rmat-s16",
                         {"timed_with_byte_counting": True})
     elif p.push_ms >= p.pull_ms:
@@ -834,7 +828,7 @@ def run_c1(args, model):
         "workload": f"BFS rmat-s{C1_SCALE}-ef{EDGE_FACTOR}-sym seed {C1_SEED}, source = first "
                     f"vertex of maximum out-degree ({src}, degree {deg})",
         "V": el.nV, "E": el.nE, "levels": last["learned"].iterations,
-        "schedule": "learned (direction rule: bottom-up while the frontier's out-edges > E/16)",
+        "schedule": "learned (Beamer's direction rule)",
         "ms": round(times["learned"], 4), "gteps": gteps(units, times["learned"]),
         "e2e": {"ms": round(ms_e2e, 4), "gteps": gteps(units, ms_e2e),
                 "h2d_bytes": el.nV * 4, "d2h_bytes": el.nV * 4},
@@ -917,7 +911,7 @@ def run_pagerank(args, check=True):
     e.set_profiling(False)
     e.close()
     units = el.nE * st_u.iterations
-    roof = roofline("k_pr_merge + k_pr_merge_fix (one PageRank iteration's gather)",
+    roof = roofline("k_pr_gather + k_pr_join (one PageRank iteration's gather)",
                     "pr_gather", prof.pagerank_bytes, prof.pagerank_ms,
                     prof.pagerank_launches, f"rmat-s{scale}")
     res = {
@@ -1195,12 +1189,12 @@ def run_batched(args, check=True):
 
     units = bfs_units + ppr_units
     value = units / (ms * 1e-3) / 1e9
-    # roofline of the PPR iteration (pieces + fix + residual kernels), timed by
+    # roofline of the PPR iteration (units + fix + rows kernels), timed by
     # the autotuner with CUDA events: per edge its source index and the L
     # lanes of the source's contribution; per vertex offsets (8 B), seed mask
     # (4 B), old rank, new rank and new contribution (3 x 4L B)
     ppr_bytes = E * (4 + 4 * L) + V * (12 + 12 * L)
-    roof = roofline("PPR iteration (k_ppr_pieces + k_ppr_fix + k_ppr_finish)",
+    roof = roofline("PPR iteration (k_ppr_units + k_ppr_fix + k_ppr_rows)",
                     "ppr_iteration", ppr_bytes, ms_iter, 1,
                     "batched-64" if G == BATCH_GRAPHS else f"batched-{G}",
                     {"traffic_note": "DRAM bytes per iteration; the [V][16] contribution "
@@ -1425,8 +1419,8 @@ def run_lanes24(args):
                   "plain_iterations": plain_iters[0],
                   "speedup_vs_plain": round(ms_plain_p / ms_p, 3),
                   "residual": st.ppr_residual,
-                  "roofline": roofline("PPR iteration (k_ppr_pieces + k_ppr_fix + "
-                                       "k_ppr_finish)", "ppr_iteration", ppr_bytes, ms_iter, 1,
+                  "roofline": roofline("PPR iteration (k_ppr_units + k_ppr_fix + "
+                                       "k_ppr_rows)", "ppr_iteration", ppr_bytes, ms_iter, 1,
                                        f"rmat-s{scale}-16-seeds", {"piece_edges": piece})}
     total_units = bfs_units + ppr_units
     out["value"] = gteps(total_units, ms_b + ms_p)
