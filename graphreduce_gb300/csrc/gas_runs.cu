@@ -895,11 +895,15 @@ gas_status_t pr_hot_plan(gas_engine *e, int32_t *scratch, cudaStream_t s, int *n
     return GAS_OK;
   }
   e->pr_hot_mem.free();
-  if (e->pr_hot_mem.alloc({GROUP_PART(e->pr_hot_ctl, sizeof(PrHot)),
+  // the copy is a quarter of the free memory at most: other objects may need it
+  size_t free_bytes = 0, total = 0;
+  CUDA_TRY(cudaMemGetInfo(&free_bytes, &total));
+  if ((size_t)e->nE * sizeof(int32_t) > free_bytes / 4 ||
+      e->pr_hot_mem.alloc({GROUP_PART(e->pr_hot_ctl, sizeof(PrHot)),
                            GROUP_PART(e->pr_hot_id, kHotSlots * sizeof(int32_t)),
                            GROUP_PART(e->pr_hot_val, kHotSlots * sizeof(float)),
                            GROUP_PART(e->pr_hot_src, (size_t)e->nE * sizeof(int32_t))}) !=
-      cudaSuccess) {
+          cudaSuccess) {
     cudaGetLastError();
     e->pr_hot_known = true;
     e->pr_hot_n = 0;
