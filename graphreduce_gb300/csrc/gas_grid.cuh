@@ -27,8 +27,9 @@ struct Barrier {
 constexpr unsigned int kGaveUp = 1u << 30;
 
 // Every CTA of a cooperative launch calls it; index (0..2, thread 0's copy
-// counts) starts at next and goes back there at the end.  Returns false in all threads when a wait gave up (here or
-// in another CTA), and the caller leaves the kernel.  with(): run by thread
+// counts) starts at next and goes back there at the end.  Returns false in all
+// threads when a wait gave up (here or in another CTA), and the caller leaves
+// the kernel.  with(): run by thread
 // 0 after the wait, its result returned in *out to every thread of the CTA
 // (one load for the CTA instead of one per thread).
 template <class T, class F>

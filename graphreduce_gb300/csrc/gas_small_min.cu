@@ -74,8 +74,8 @@ struct MinCtl {
 // lowering offers its target.
 template <bool kWeighted, bool kLowerOnly>
 __device__ __forceinline__ void walk(const int4 *Q, int nq, int most, int w0,
-                                     const int32_t *R, int32_t *W, const int32_t *csr_off, const int32_t *csr_dst,
-                                     const int32_t *csr_w, int32_t zero_cap, int (*s_row)[3],
+                                     const int32_t *R, int32_t *W, const int32_t *csr_off,
+                                     const int32_t *csr_dst, const int32_t *csr_w, int32_t zero_cap, int (*s_row)[3],
                                      Stage &st, const Queue &N, Count *ctr) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int kRounds = 4;
