@@ -78,7 +78,7 @@ using gasgrid::warp_add;
 struct SmallCtl {
   gasgrid::Barrier bar;
   Count q[3];       // of the level being read, filled and cleared (rotating)
-  Count made;       // of a queue made from a bitmap
+  Count made[2];    // of queues made from a bitmap (in turn)
   long long bytes;  // algorithmic bytes (profiling)
 };
 
@@ -275,6 +275,7 @@ __global__ void __launch_bounds__(kSbNT, 1)
   bool capped = false;
   bool pulled = false;    // the frontier was found bottom-up
   bool unqueued = false;  // it is in the bitmap only
+  int mk = 0;             // made[mk] is the next made queue's count, and is clear
   long long seen = 0;                   // out-edges of the levels expanded
   int prev = 0;                         // members of the level before
   for (int k = 0;; ++k) {
@@ -300,16 +301,22 @@ __global__ void __launch_bounds__(kSbNT, 1)
     for (int w = tid; w < nW; w += nthr) O[w] = 0u;
     if (tid == 0) *reinterpret_cast<int4 *>(&c->q[old]) = make_int4(0, 0, 0, 0);
     const Queue Q = k & 1 ? qb : qa, next = k & 1 ? qa : qb;
-    const bool made = !pull && unqueued;
-    if (made) {  // the queue of a frontier that is in the bitmap only
+    if (!pull && unqueued) {  // the queue of a frontier that is in the bitmap only
+      Count *made = &c->made[mk];
       for (int w0 = dealt_warp(); w0 < nW; w0 += nthr >> 5) {
         const uint32_t word = F[w0];
         if (!word) continue;  // warp-uniform
         const int v[1] = {(word >> lane) & 1u ? (w0 << 5) + lane : -1};
-        offer(st, v, g.csr_off, Q, &c->made);
+        offer(st, v, g.csr_off, Q, made);
       }
-      flush(st, g.csr_off, Q, &c->made);
-      SB_SYNC(head, &c->made);
+      flush(st, g.csr_off, Q, made);
+      SB_SYNC(head, made);
+      // the other count was last read before the barrier that ended its own
+      // level, and the one that ends this level comes before it is added to
+      // again.  (One count, cleared after the level's end, is being added to
+      // by then where the next level makes its queue as well.)
+      mk ^= 1;
+      if (tid == 0) *reinterpret_cast<int4 *>(&c->made[mk]) = make_int4(0, 0, 0, 0);
     }
     unqueued = pull || edges >= kSbDense * nthr;
     int e = 0, m = 0;  // this level's finds, when they are not queued
@@ -349,7 +356,6 @@ __global__ void __launch_bounds__(kSbNT, 1)
     else
       ++n_push;
     SB_SYNC(head, &c->q[nxt]);
-    if (made && tid == 0) c->made = Count{0, 0, 0, 0};  // every CTA has read it
   }
   if (kCount) warp_add(bytes, &c->bytes);
   // the next run finds the bitmaps clear (nothing reads them any more)
@@ -365,6 +371,7 @@ __global__ void __launch_bounds__(kSbNT, 1)
     // and the control word clear for the next run (a CTA still to read a
     // count finds no edges and leaves as well)
     c->q[0] = c->q[1] = c->q[2] = Count{0, 0, 0, 0};
+    c->made[0] = c->made[1] = Count{0, 0, 0, 0};
   }
 #undef SB_SYNC
 }

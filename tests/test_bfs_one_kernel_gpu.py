@@ -168,3 +168,29 @@ def test_records_on_larger_graphs():
                 p = eng.profile()
                 assert p.push_launches + p.pull_launches > 1
             switch(False)
+
+
+def test_wide_levels_in_a_row():
+    """26 top-down levels one after the other whose finds are only marked
+    (320 K out-edges each, more than two per thread of the grid), so that each
+    level makes its queue from the bitmap right after one that did: the makes'
+    counts must not be cleared while the next one adds to them.  Run often, as
+    a lost count shows by timing only."""
+    rng = np.random.default_rng(11)
+    layers, n = 40, 20_000
+    u = np.arange(n * (layers - 1))
+    src = np.repeat(u, 16)
+    dst = (src // n + 1) * n + rng.integers(0, n, len(src))
+    dst[::16] = u + n             # every vertex of the next layer is found
+    dst[1::16 * n] = dst[::16 * n]
+    hubs = np.arange(0, len(src), 16 * n)  # vertex 0 of a layer: rows of several entries
+    for h in hubs:
+        src[h + 16:h + 16 * 20] = src[h]
+    order = np.argsort(src, kind="stable")
+    el = EdgeList(n * layers, src[order].astype(np.int32), dst[order].astype(np.int32))
+    want = np.repeat(np.arange(layers, dtype=np.int32), n)
+    got = runs(el, "auto", [(0, n)] * 40, True)
+    for vd, st in got:
+        np.testing.assert_array_equal(vd, want)
+        assert (st.iterations, st.push_iters, st.pull_iters) == (layers, 26, 13)
+        assert st.kernel_launches == 1
