@@ -416,7 +416,9 @@ __device__ __forceinline__ void expand_pull(const int32_t *csc_off, const int32_
     const int2 e = list[c];  // vertex, first in-edge
     uint32_t *p = bits + (e.x >> 5);
     const uint32_t m = 1u << (e.x & 31);
-    if (__ldcg(p) & m) continue;  // warp-uniform: one address
+    // the votes below need the whole warp, and other warps set bits of the
+    // word meanwhile: the lanes agree on what they have read
+    if (__any_sync(FULL, (__ldcg(p) & m) != 0u)) continue;
     const uint32_t end = csc_off[e.x + 1];
     int u[kXChunk / 32];
     bool f = false;

@@ -84,3 +84,34 @@ def test_generic_runs(program, name):
                 eng.getResults()
                 np.testing.assert_array_equal(vd, ref)
                 assert st.iterations == it
+
+
+def test_neighbouring_hubs_of_many_chunks():
+    """64 hubs that share two words of the next frontier, with 60 chunks of
+    in-edges each, every third full of changed in-neighbours: warps set a word's
+    bits while others test them to skip their chunk."""
+    hubs, chunks, m = 64, 60, 3000
+    rng = np.random.default_rng(8)
+    s = hubs                     # the source, then m vertices it leads to, then m unreached
+    reached, rest = s + 1 + np.arange(m), s + 1 + m + np.arange(m)
+    row = [rng.choice(rest, 70)]
+    for c in range(chunks):
+        row.append(rng.choice(reached if c % 3 == 1 else rest, 256))
+    row = np.concatenate(row)
+    nV = s + 1 + 2 * m + 20
+    path = np.concatenate([[5], np.arange(nV - 20, nV)])
+    el = weighted(nV, np.concatenate([np.full(m, s), np.tile(row, hubs), path[:-1]]),
+                  np.concatenate([reached, np.repeat(np.arange(hubs), len(row)), path[1:]]))
+    ref, it = oracle.sssp(el.nV, el.src, el.dst, el.weights, s)
+    assert (ref[:hubs] < 200).all()
+    with closing(GASEngineGPU("sssp")) as eng:
+        vd = initial_vertex_data("sssp", el.nV, s)
+        fresh = vd.copy()
+        eng.setGraph(el.nV, vd, el.nE, el.weights, el.src, el.dst)
+        for _ in range(20):
+            eng.upload_vertex_data(fresh)
+            eng.setActive(0, el.nV)
+            st = eng.run_schedule("generic", max_iterations=el.nV + 2)
+            eng.getResults()
+            np.testing.assert_array_equal(vd, ref)
+            assert st.iterations == it
