@@ -1637,7 +1637,9 @@ gas_status_t ensure_sssp(gas_batch *b, int lanes, int n_sources) {
   return GAS_OK;
 }
 
-gas_status_t ensure_bfs(gas_batch *b, int lanes, int n_sources) {
+// s: the run's stream, which the initial values are ordered by (they are in
+// place at return: the state outlives a run that fails, and its stream).
+gas_status_t ensure_bfs(gas_batch *b, int lanes, int n_sources, cudaStream_t s) {
   gas_engine *e = b->eng;
   const size_t nV = std::max(1, e->nV);
   GAS_TRY(ensure_frontier(b));
@@ -1646,8 +1648,10 @@ gas_status_t ensure_bfs(gas_batch *b, int lanes, int n_sources) {
     CUDA_TRY(b->bfs_mem.alloc({GROUP_PART(b->vn, nV * 8), GROUP_PART(b->fr, nV * 4),
                                GROUP_PART(b->alive, ng * 4), GROUP_PART(b->g_off, ng * 4),
                                GROUP_PART(b->dir, sizeof(MsDir))}));
-    CUDA_TRY(cudaMemcpy(b->g_off, b->v_off.data(), b->v_off.size() * 4, cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemset(b->dir, 0, sizeof(MsDir)));
+    CUDA_TRY(cudaMemcpyAsync(b->g_off, b->v_off.data(), b->v_off.size() * 4,
+                             cudaMemcpyHostToDevice, s));
+    CUDA_TRY(cudaMemsetAsync(b->dir, 0, sizeof(MsDir), s));
+    CUDA_TRY(cudaStreamSynchronize(s));
   }
   if (b->depth_lanes != lanes) {
     drop_graph(b);
@@ -2315,7 +2319,8 @@ gas_status_t gas_batch_build(gas_batch *b, void *stream) {
                                b->dst.data(), stream));
   if (!b->cnt) {
     CUDA_TRY(cudaMalloc(&b->cnt, 3 * sizeof(gas_counters)));
-    CUDA_TRY(cudaMemset(b->cnt, 0, 3 * sizeof(gas_counters)));
+    CUDA_TRY(cudaMemsetAsync(b->cnt, 0, 3 * sizeof(gas_counters), (cudaStream_t)stream));
+    CUDA_TRY(cudaStreamSynchronize((cudaStream_t)stream));  // runs take other streams
     CUDA_TRY(cudaMallocHost(&b->h_cnt, 3 * sizeof(gas_counters)));
     CUDA_TRY(cudaMalloc(&b->prm, sizeof(BatchParams)));
     CUDA_TRY(cudaMalloc(&b->edges, sizeof(unsigned long long)));
@@ -2376,7 +2381,7 @@ gas_status_t gas_batch_run(gas_batch *b, const gas_batch_job *job, int32_t *dept
   prm.n_seeds = G * LP;
   std::vector<int32_t> sg, ss;
   if (LB) {
-    GAS_TRY(ensure_bfs(b, LB, G * LB));
+    GAS_TRY(ensure_bfs(b, LB, G * LB, s));
     sg.resize((size_t)G * LB);
     for (int g = 0; g < G; ++g)
       for (int l = 0; l < LB; ++l) {
@@ -2470,17 +2475,20 @@ gas_status_t gas_batch_run(gas_batch *b, const gas_batch_job *job, int32_t *dept
     for (int l = 0; l < LP; ++l) stats->ppr_lane_residual[l] = resid[1 + l];
   }
   if (LS && cs.error) {
-    CUDA_TRY(cudaMemset(&b->cnt[2].error, 0, sizeof(int32_t)));
+    CUDA_TRY(cudaMemsetAsync(&b->cnt[2].error, 0, sizeof(int32_t), s));
+    CUDA_TRY(cudaStreamSynchronize(s));
     return fail(cs.error == GAS_ERR_ITER_CAP ? GAS_ERR_ITER_CAP : GAS_ERR_DEVICE,
                 "batch sssp: device error %d after %d iterations", cs.error, cs.iteration);
   }
   if (LB && cb.error) {
-    CUDA_TRY(cudaMemset(&b->cnt[0].error, 0, sizeof(int32_t)));
+    CUDA_TRY(cudaMemsetAsync(&b->cnt[0].error, 0, sizeof(int32_t), s));
+    CUDA_TRY(cudaStreamSynchronize(s));
     return fail(cb.error == GAS_ERR_ITER_CAP ? GAS_ERR_ITER_CAP : GAS_ERR_DEVICE,
                 "batch bfs: device error %d after %d levels", cb.error, cb.iteration);
   }
   if (LP && cp.error) {
-    CUDA_TRY(cudaMemset(&b->cnt[1].error, 0, sizeof(int32_t)));
+    CUDA_TRY(cudaMemsetAsync(&b->cnt[1].error, 0, sizeof(int32_t), s));
+    CUDA_TRY(cudaStreamSynchronize(s));
     return fail(cp.error == GAS_ERR_ITER_CAP ? GAS_ERR_ITER_CAP : GAS_ERR_DEVICE,
                 "batch ppr: residual %.3e after %d iterations", resid[0], cp.iteration);
   }

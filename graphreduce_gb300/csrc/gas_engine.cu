@@ -1264,7 +1264,7 @@ gas_status_t gas_engine_set_graph(gas_engine *e, int32_t nV, void *vertex_data,
   // the host vectors are released at return: wait for the copies
   CUDA_TRY(cudaStreamSynchronize(st));
   e->n_ne = *h_ne;
-  gas::reserve_fast_buffers(e);
+  gas::reserve_fast_buffers(e, stream);
   e->n_active = 0;
   e->n_edges = 0;
   e->counts_dirty = false;

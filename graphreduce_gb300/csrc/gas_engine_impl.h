@@ -234,7 +234,7 @@ gas_status_t engine_sync_counts(gas_engine *e, void *stream);
 int engine_grid(int64_t work_items, int per_block, int cap);
 // the fast schedule's buffers, with the graph's arrays where a run will want
 // them (large BFS, SSSP and CC graphs), so that the first run finds them
-void reserve_fast_buffers(gas_engine *e);
+void reserve_fast_buffers(gas_engine *e, void *stream);
 // CSR/CSC on the device (gas_build.cu): fills csc_off/csc_src/csr_off/
 // csr_dst (+ csc_ed/csr_ed), which must be allocated; the permutations
 // (edge-list index per CSC / CSR position) when asked for.

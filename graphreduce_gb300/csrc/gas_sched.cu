@@ -1032,7 +1032,7 @@ gas_status_t body(gas_engine *e, cudaStream_t cs, cudaGraphConditionalHandle h,
   return compaction(e, cs, c, h, 1);
 }
 
-gas_status_t ensure_fast_buffers(gas_engine *e) {
+gas_status_t ensure_fast_buffers(gas_engine *e, cudaStream_t s) {
   if (e->q_ids) return GAS_OK;
   const size_t V = (size_t)e->nV, nW = (V + 31) / 32;
   const size_t nqb = (nW + kQWordsPerBlock - 1) / kQWordsPerBlock;
@@ -1041,7 +1041,7 @@ gas_status_t ensure_fast_buffers(gas_engine *e) {
       {GROUP_PART(e->q_ids, V * 4), GROUP_PART(e->q_vals, V * 4), GROUP_PART(e->q_end, V * 4),
        GROUP_PART(e->q_delta, V * 4), GROUP_PART(e->snap, V * 4), GROUP_PART(e->cbits, nW * 4),
        GROUP_PART(e->qpart, nqb * (1 + kQWarpsPerBlock) * sizeof(int4))}));
-  CUDA_TRY(cudaMemset(e->cbits, 0, (nW ? nW : 1) * 4));
+  CUDA_TRY(cudaMemsetAsync(e->cbits, 0, (nW ? nW : 1) * 4, s));
   return GAS_OK;
 }
 
@@ -1049,7 +1049,7 @@ gas_status_t ensure_fast_buffers(gas_engine *e) {
 
 namespace gas {
 
-void reserve_fast_buffers(gas_engine *e) {
+void reserve_fast_buffers(gas_engine *e, void *stream) {
   if (e->graph_only) return;
   if (e->prog == GAS_PROG_BFS && e->nV <= kBfsSmallMaxV && !e->edges_on_host) {
     if (e->nV > kBfsSmallRecordsMaxV) bfs_small_reserve(e);
@@ -1059,7 +1059,8 @@ void reserve_fast_buffers(gas_engine *e) {
                      (e->prog == GAS_PROG_SSSP && e->nV > kSsspSmallLearnedMaxV) ||
                      (e->prog == GAS_PROG_CC && e->nV > kCcSmallLearnedMaxV);
   if (!sized) return;
-  if (ensure_fast_buffers(e) != GAS_OK) {  // tight memory: the first run asks again
+  if (ensure_fast_buffers(e, S(stream)) != GAS_OK ||
+      cudaStreamSynchronize(S(stream)) != cudaSuccess) {  // tight memory: the first run asks again
     e->fast_mem.free();
     cudaGetLastError();
     clear_error();
@@ -1154,7 +1155,7 @@ gas_status_t run_fast(gas_engine *e, gas_schedule_t schedule,
     return run_bfs_small(e, schedule, max_iterations, stats, stream);
   if (min_small_eligible(e, schedule) && min_small_reserve(e))
     return run_min_small(e, max_iterations, stats, stream);
-  GAS_TRY(ensure_fast_buffers(e));
+  GAS_TRY(ensure_fast_buffers(e, S(stream)));
   FastCtx ctx;
   ctx.nW = (e->nV + 31) / 32;
   ctx.n_qblocks = (ctx.nW + kQWordsPerBlock - 1) / kQWordsPerBlock;
