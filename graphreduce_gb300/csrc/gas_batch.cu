@@ -1544,6 +1544,20 @@ void bfree(T *&p) {
   p = nullptr;
 }
 
+// Another allocation in place of p's.  On failure p is null (the caller's size
+// of it has to say so) and the runtime's last error is cleared, or the next
+// launch would report it.
+template <class T>
+cudaError_t renew(T *&p, size_t bytes) {
+  bfree(p);
+  const cudaError_t ce = cudaMalloc((void **)&p, bytes);
+  if (ce != cudaSuccess) {
+    p = nullptr;
+    cudaGetLastError();
+  }
+  return ce;
+}
+
 void drop_graph(gas_batch *b) {
   if (b->graph) cudaGraphExecDestroy(b->graph);
   b->graph = nullptr;
@@ -1624,14 +1638,12 @@ gas_status_t ensure_sssp(gas_batch *b, int lanes, int n_sources) {
         {GROUP_PART(b->dist, nV * LS * 4), GROUP_PART(b->q_vals, nV * LS * 4)}));
     b->dist_ls = LS;
   }
-  if (!b->lane_rounds) {
-    CUDA_TRY(cudaMalloc(&b->lane_rounds, kMaxLanes * 4));
-    CUDA_TRY(cudaMalloc(&b->lanes_active, 4));
-  }
+  if (!b->lane_rounds) CUDA_TRY(renew(b->lane_rounds, kMaxLanes * 4));
+  if (!b->lanes_active) CUDA_TRY(renew(b->lanes_active, 4));
   if (b->sssp_srcs_cap < n_sources) {
     drop_graph(b);
-    bfree(b->sssp_srcs);
-    CUDA_TRY(cudaMalloc(&b->sssp_srcs, (size_t)std::max(1, n_sources) * 4));
+    b->sssp_srcs_cap = 0;
+    CUDA_TRY(renew(b->sssp_srcs, (size_t)std::max(1, n_sources) * 4));
     b->sssp_srcs_cap = n_sources;
   }
   return GAS_OK;
@@ -1655,14 +1667,14 @@ gas_status_t ensure_bfs(gas_batch *b, int lanes, int n_sources, cudaStream_t s) 
   }
   if (b->depth_lanes != lanes) {
     drop_graph(b);
-    bfree(b->depth);
-    CUDA_TRY(cudaMalloc(&b->depth, nV * lanes * 4));
+    b->depth_lanes = 0;
+    CUDA_TRY(renew(b->depth, nV * lanes * 4));
     b->depth_lanes = lanes;
   }
   if (b->srcs_cap < n_sources) {
     drop_graph(b);
-    bfree(b->srcs);
-    CUDA_TRY(cudaMalloc(&b->srcs, (size_t)std::max(1, n_sources) * 4));
+    b->srcs_cap = 0;
+    CUDA_TRY(renew(b->srcs, (size_t)std::max(1, n_sources) * 4));
     b->srcs_cap = n_sources;
   }
   return GAS_OK;
@@ -1771,24 +1783,22 @@ gas_status_t ensure_ppr(gas_batch *b, int lanes, int P, int n_seeds, int grid_ro
     b->ppr_lanes = lanes;
     b->piece_edges = 0;
   }
-  if (!b->seed_mask) CUDA_TRY(cudaMalloc(&b->seed_mask, nV * 4));
+  if (!b->seed_mask) CUDA_TRY(renew(b->seed_mask, nV * 4));
   if (!b->ticket) {
-    CUDA_TRY(cudaMalloc(&b->ticket, 4));
+    CUDA_TRY(renew(b->ticket, 4));
     CUDA_TRY(cudaMemsetAsync(b->ticket, 0, 4, s));
   }
   if (b->seeds_cap < n_seeds) {
     drop_graph(b);
-    bfree(b->seeds);
     b->seeds_cap = 0;
-    CUDA_TRY(cudaMalloc(&b->seeds, (size_t)n_seeds * 4));
+    CUDA_TRY(renew(b->seeds, (size_t)n_seeds * 4));
     b->seeds_cap = n_seeds;
   }
   const int need_l1 = grid_rows * G;
   if (b->l1_cap < need_l1) {
     drop_graph(b);
-    bfree(b->l1);
     b->l1_cap = 0;
-    CUDA_TRY(cudaMalloc(&b->l1, (size_t)need_l1 * sizeof(double)));
+    CUDA_TRY(renew(b->l1, (size_t)need_l1 * sizeof(double)));
     b->l1_cap = need_l1;
   }
   if (b->piece_edges == P) return GAS_OK;

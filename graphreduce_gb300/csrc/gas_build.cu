@@ -410,6 +410,7 @@ gas_status_t build_graph_device(gas_engine *e, const int32_t *srcs, const int32_
     const cudaError_t ce = cudaMalloc((void **)&w.base, w.used);
     if (ce != cudaSuccess) {
       w.base = nullptr;
+      cudaGetLastError();
       return fail(GAS_ERR_NOMEM, "device graph build: %s", cudaGetErrorString(ce));
     }
   }

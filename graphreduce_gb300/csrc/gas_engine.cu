@@ -776,6 +776,7 @@ struct ArenaPlan {
     if (ce != cudaSuccess) {
       e->arena = nullptr;
       e->arena_ptrs.clear();
+      cudaGetLastError();
       return gas::fail(GAS_ERR_NOMEM, "cudaMalloc of %zu bytes: %s", bytes,
                        cudaGetErrorString(ce));
     }

@@ -41,6 +41,7 @@ struct DeviceGroup {
     const cudaError_t ce = cudaMalloc(&base, total);
     if (ce != cudaSuccess) {
       base = nullptr;
+      cudaGetLastError();  // the caller has it: not for the next launch to report
       return ce;
     }
     size_t at = 0;

@@ -70,3 +70,48 @@ def test_first_loop_run_on_a_stream_of_its_own(program, busy_default_stream):
         np.testing.assert_array_equal(vd, ref)
         assert st.iterations == it
         torch.cuda.synchronize()
+
+
+class Filled:
+    """All of the device's memory taken but for about `leave` bytes."""
+
+    def __init__(self, leave):
+        import torch
+        torch.cuda.empty_cache()
+        self.taken = []
+        for step in (1 << 33, 1 << 30, 1 << 26, 1 << 23):
+            while torch.cuda.mem_get_info()[0] > leave + step:
+                self.taken.append(torch.empty(step, dtype=torch.uint8, device="cuda"))
+
+    def release(self):
+        import torch
+        self.taken.clear()
+        torch.cuda.empty_cache()
+
+
+def test_batch_runs_after_one_that_found_no_memory():
+    """The lanes' rows do not fit: the run fails, and a later run of the lanes
+    that ran before makes its rows anew."""
+    n = 1 << 21
+    i = np.arange(n - 1, dtype=np.int32)
+    i = i[i % 1000 != 999]
+    with closing(Batch()) as b:
+        b.add_graph(n, i, i + 1, np.ones(len(i), np.int32))
+        b.build()
+        depth = np.arange(n) % 1000
+        depth[1000:] = -1
+        one = np.zeros((1, 1), np.int32)
+        many = np.zeros((1, 32), np.int32)
+        for kind in ("bfs", "sssp"):
+            b.run(**{f"{kind}_sources": one})
+            full = Filled(128 << 20)  # 32 lanes' rows take 256 MB
+            with pytest.raises(GasError):
+                b.run(**{f"{kind}_sources": many})
+            full.release()
+            r = b.run(**{f"{kind}_sources": one})
+            got = r.depth if kind == "bfs" else r.dist
+            reached = depth >= 0
+            np.testing.assert_array_equal(got[reached, 0], depth[reached])
+            r = b.run(**{f"{kind}_sources": many})
+            got = r.depth if kind == "bfs" else r.dist
+            np.testing.assert_array_equal(got[reached], np.repeat(depth[reached][:, None], 32, 1))
