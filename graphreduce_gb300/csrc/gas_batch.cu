@@ -2340,13 +2340,12 @@ gas_status_t gas_batch_build(gas_batch *b, void *stream) {
   std::vector<int32_t>().swap(b->src);
   std::vector<int32_t>().swap(b->dst);
   std::vector<int32_t>().swap(b->w);
-  // the traversals' frontier, so that the first run finds it (tight memory:
-  // that run asks again)
-  if (ensure_frontier(b) != GAS_OK) {
-    b->frontier_mem.free();
-    cudaGetLastError();
+  // the traversals' frontier (four words per vertex, and a word per 64 edges),
+  // so that the first run finds it; that run asks again where it is more than
+  // a quarter of the free memory, as a batch may only ever run PPR
+  if (gas::within_quarter_of_free((size_t)nV * 17 + (size_t)b->n_edges / 16) &&
+      ensure_frontier(b) != GAS_OK)
     gas::clear_error();
-  }
   b->built = true;
   return GAS_OK;
 }
@@ -2410,7 +2409,16 @@ gas_status_t gas_batch_run(gas_batch *b, const gas_batch_job *job, int32_t *dept
   }
   std::vector<int32_t> pg;
   if (LP) {
-    GAS_TRY(ensure_ppr(b, LP, P, G * LP, c.grid_rows, s));
+    gas_status_t st = ensure_ppr(b, LP, P, G * LP, c.grid_rows, s);
+    if (st != GAS_OK && !LB && !LS && b->next) {
+      // the traversals' frontier, which this run does not use, may have the
+      // memory that it needs
+      drop_graph(b);
+      b->frontier_mem.free();
+      gas::clear_error();
+      st = ensure_ppr(b, LP, P, G * LP, c.grid_rows, s);
+    }
+    GAS_TRY(st);
     pg.resize((size_t)G * LP);
     for (int g = 0; g < G; ++g)
       for (int l = 0; l < LP; ++l) {

@@ -234,8 +234,11 @@ gas_status_t engine_commit(gas_engine *e, void *stream);
 gas_status_t engine_sync_counts(gas_engine *e, void *stream);
 int engine_grid(int64_t work_items, int per_block, int cap);
 // the fast schedule's buffers, with the graph's arrays where a run will want
-// them (large BFS, SSSP and CC graphs), so that the first run finds them
+// them (large BFS, SSSP and CC graphs), so that the first run finds them; not
+// where they are more than a quarter of the free memory, as nobody has asked
+// for such a run yet
 void reserve_fast_buffers(gas_engine *e, void *stream);
+bool within_quarter_of_free(size_t bytes);
 // CSR/CSC on the device (gas_build.cu): fills csc_off/csc_src/csr_off/
 // csr_dst (+ csc_ed/csr_ed), which must be allocated; the permutations
 // (edge-list index per CSC / CSR position) when asked for.

@@ -1049,16 +1049,26 @@ gas_status_t ensure_fast_buffers(gas_engine *e, cudaStream_t s) {
 
 namespace gas {
 
+bool within_quarter_of_free(size_t bytes) {
+  if (bytes <= kSmallWithGraph) return true;  // not worth the question
+  size_t free_bytes = 0, total = 0;
+  if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) return false;
+  return bytes <= free_bytes / 4;
+}
+
 void reserve_fast_buffers(gas_engine *e, void *stream) {
   if (e->graph_only) return;
   if (e->prog == GAS_PROG_BFS && e->nV <= kBfsSmallMaxV && !e->edges_on_host) {
-    if (e->nV > kBfsSmallRecordsMaxV) bfs_small_reserve(e);
+    if (e->nV > kBfsSmallRecordsMaxV &&
+        within_quarter_of_free(bfs_small_bytes(e->nV, e->nE).all()))
+      bfs_small_reserve(e);
     return;
   }
   const bool sized = (e->prog == GAS_PROG_BFS && e->nV > kBfsSmallRecordsMaxV) ||
                      (e->prog == GAS_PROG_SSSP && e->nV > kSsspSmallLearnedMaxV) ||
                      (e->prog == GAS_PROG_CC && e->nV > kCcSmallLearnedMaxV);
-  if (!sized) return;
+  // (five words per vertex, and a little)
+  if (!sized || !within_quarter_of_free((size_t)e->nV * 21)) return;
   if (ensure_fast_buffers(e, S(stream)) != GAS_OK ||
       cudaStreamSynchronize(S(stream)) != cudaSuccess) {  // tight memory: the first run asks again
     e->fast_mem.free();
@@ -1155,7 +1165,14 @@ gas_status_t run_fast(gas_engine *e, gas_schedule_t schedule,
     return run_bfs_small(e, schedule, max_iterations, stats, stream);
   if (min_small_eligible(e, schedule) && min_small_reserve(e))
     return run_min_small(e, max_iterations, stats, stream);
-  GAS_TRY(ensure_fast_buffers(e, S(stream)));
+  if (ensure_fast_buffers(e, S(stream)) != GAS_OK) {
+    // the one-kernel paths' buffers, which this run does not use, may have the
+    // memory that it needs
+    e->sb_mem.free();
+    e->sm_mem.free();
+    clear_error();
+    GAS_TRY(ensure_fast_buffers(e, S(stream)));
+  }
   FastCtx ctx;
   ctx.nW = (e->nV + 31) / 32;
   ctx.n_qblocks = (ctx.nW + kQWordsPerBlock - 1) / kQWordsPerBlock;
