@@ -904,12 +904,17 @@ struct __align__(8) CVal {
   float s, c;
 };
 
-// Knuth two-sum: a.s + b.s = s + err exactly; compensations add up in c.
+// Knuth two-sum: a + b = s + c exactly.
+__device__ __forceinline__ CVal two_sum(float a, float b) {
+  const float s = __fadd_rn(a, b);
+  const float bp = __fsub_rn(s, a);
+  return CVal{s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, bp)), __fsub_rn(b, bp))};
+}
+
+// Compensations add up in c.
 __device__ __forceinline__ CVal two_sum_add(CVal a, CVal b) {
-  const float s = __fadd_rn(a.s, b.s);
-  const float bp = __fsub_rn(s, a.s);
-  const float err = __fadd_rn(__fsub_rn(a.s, __fsub_rn(s, bp)), __fsub_rn(b.s, bp));
-  return CVal{s, __fadd_rn(__fadd_rn(a.c, b.c), err)};
+  const CVal t = two_sum(a.s, b.s);
+  return CVal{t.s, __fadd_rn(__fadd_rn(a.c, b.c), t.c)};
 }
 
 struct PprArgs {
@@ -1195,20 +1200,38 @@ __device__ __forceinline__ void ppr_row_load(const PprArgs &a, int l, PprRow<VL>
   }
 }
 
-// The L1 step is kept without FP64 (two conversions and two additions per
-// rank took three quarters of this kernel's time at GB300's FP64 rate):
-// new - old = s + c exactly (two-sum), and |new - old| joins the thread's
-// sum by two-sum, so its error is of second order in 2^-24.
+// A thread's sum of L1 steps, in no fewer bits than FP64 sums have but (nearly)
+// without FP64 (two conversions and two additions per rank took three quarters
+// of k_ppr_rows' time at GB300's FP64 rate).  A step |new - old| = s + c exactly
+// (two-sum); s goes into a, what that addition rounds off and c into b, what
+// those round off into t.  N steps are off by at most N^3 2^-73 of their sum,
+// FP64 by up to N 2^-53, so every kL1Flush rows go into an FP64 sum.  (34 M
+// ranks, 2.1 M vertices of 16 lanes: 528 us per iteration of all kernels, with
+// FP64 throughout 649; with a and b alone, whose additions round at 2^-49, 524.)
+constexpr int kL1Flush = 64;
+struct L1Sum {
+  float a = 0.f, b = 0.f, t = 0.f;
+  __device__ __forceinline__ void add(CVal step) {
+    if (step.s < 0.f) step = CVal{-step.s, -step.c};
+    const CVal x = two_sum(a, step.s), y = two_sum(b, step.c), z = two_sum(y.s, x.c);
+    a = x.s;
+    b = z.s;
+    t = __fadd_rn(t, __fadd_rn(y.c, z.c));
+  }
+  __device__ __forceinline__ double value() const {
+    return __dadd_rn((double)a, __dadd_rn((double)b, (double)t));
+  }
+};
+
 template <int VL>
 __device__ __forceinline__ void ppr_row_finish(const PprArgs &a, int l, const PprRow<VL> &w,
-                                               float d, float base, CVal (&l1)[VL]) {
+                                               float d, float base, L1Sum (&l1)[VL]) {
   Lanes<VL> rank, contrib;
 #pragma unroll
   for (int q = 0; q < VL; ++q) {
     const float b = ((w.seed >> (l + q)) & 1u) ? base : 0.f;
     const float r = __fadd_rn(b, __fmul_rn(d, w.sum.f[q]));
-    const CVal step = two_sum_add(CVal{r, 0.f}, CVal{-w.old.f[q], 0.f});
-    l1[q] = two_sum_add(l1[q], step.s < 0.f ? CVal{-step.s, -step.c} : step);
+    l1[q].add(two_sum(r, -w.old.f[q]));
     rank.f[q] = r;
     contrib.f[q] = w.deg ? __fdiv_rn(r, (float)w.deg) : 0.f;
   }
@@ -1229,9 +1252,21 @@ __global__ void __launch_bounds__(kNT)
   const int l = threadIdx.x % T * VL, grp = threadIdx.x / T, per_block = kNT / T;
   const float d = (float)a.prm->damping, base = (float)(1.0 - a.prm->damping);
   const bool first = a.cnt->iteration == 0;
-  CVal l1[VL];
+  L1Sum l1[VL];
+  double done[VL];  // of the rows already flushed
 #pragma unroll
-  for (int q = 0; q < VL; ++q) l1[q] = CVal{0.f, 0.f};
+  for (int q = 0; q < VL; ++q) done[q] = 0.0;
+  int rows = 0;
+  const auto flush = [&](int n) {
+    rows += n;
+    if (rows < kL1Flush) return;
+    rows = 0;
+#pragma unroll
+    for (int q = 0; q < VL; ++q) {
+      done[q] = __dadd_rn(done[q], l1[q].value());
+      l1[q] = L1Sum();
+    }
+  };
   if (l < a.L) {
     const int stride = gridDim.x * per_block;
     int i = blockIdx.x * per_block + grp;
@@ -1246,6 +1281,7 @@ __global__ void __launch_bounds__(kNT)
       for (int k = 0; k < 2; ++k) ppr_row_load<VL>(a, l, w[k]);
 #pragma unroll
       for (int k = 0; k < 2; ++k) ppr_row_finish<VL>(a, l, w[k], d, base, l1);
+      flush(2);
     }
     if (i < a.n_ne) {
       PprRow<VL> w;
@@ -1263,12 +1299,13 @@ __global__ void __launch_bounds__(kNT)
           for (int q = 0; q < VL; ++q) w.sum.f[q] = 0.f;
           ppr_row_load<VL>(a, l, w);
           ppr_row_finish<VL>(a, l, w, d, base, l1);
+          flush(1);
         }
   }
   // per-lane block sums in a fixed order
   __shared__ double s[kNT * VL];
 #pragma unroll
-  for (int q = 0; q < VL; ++q) s[grp * a.G + l + q] = (double)l1[q].s + (double)l1[q].c;
+  for (int q = 0; q < VL; ++q) s[grp * a.G + l + q] = __dadd_rn(done[q], l1[q].value());
   __syncthreads();
   if (threadIdx.x < a.G) {
     double t = 0.0;

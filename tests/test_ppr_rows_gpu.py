@@ -2,11 +2,13 @@
 than one group folds (16) and than a CTA has groups, rows ending exactly at a
 unit's (128 in-edges) or a step's (8) end, an edge count that is no multiple of 8,
 every vector width of the lanes, a graph without edges."""
+import math
+
 import numpy as np
 import pytest
 
 import oracle
-from graphreduce_gb300 import Batch
+from graphreduce_gb300 import Batch, GasError
 from graphreduce_gb300.graph import EdgeList
 from test_batch_gpu import PPR_L1, PPR_TOL
 
@@ -55,4 +57,51 @@ def test_lanes_against_the_fp64_oracle(graphs, lanes, piece):
                 continue
             ref, _, _ = oracle.ppr_fp64(el.nV, el.src, el.dst, int(seeds[g, l]), 0.85, 1e-13)
             assert np.abs(got[:, l].astype(np.float64) - ref).sum() <= PPR_L1, (g, l)
+    b.close()
+
+
+def test_residual_has_the_bits_of_an_fp64_sum():
+    """Steps of 2^-4, 2^-29 and 2^-54 in the rows of one thread: every partial
+    sum fits 53 bits, so an FP64 sum of them is exact in any order, and 48 bits
+    lose the smallest."""
+    n = 100_000
+
+    def fan(*degs):
+        """A seed and a chain of vertices with degs[i] out-edges, all but one to
+        a last vertex; the chain's end leads to n others as well."""
+        k = len(degs)
+        src, dst, sink = [], [], k + n
+        for i, d in enumerate(degs):
+            to = np.full(d, sink)
+            if i < k - 1:
+                to[0] = i + 1
+            else:
+                to[:n] = k + np.arange(n)
+            src.append(np.full(d, i))
+            dst.append(to)
+        return EdgeList(sink + 1, np.concatenate(src).astype(np.int32),
+                        np.concatenate(dst).astype(np.int32))
+    i = np.arange(4, dtype=np.int32)
+    graphs = [EdgeList(5, i, i + 1), fan(1, 1 << 4, 1 << 4, 1 << 17),
+              fan(1, 1 << 16, 1 << 17, 1 << 17)]
+    seeds = np.zeros((3, 32), np.int32)
+    b = Batch()
+    for el in graphs:
+        b.add_graph(el.nV, el.src, el.dst)
+    b.build()
+    ranks = []
+    for cap in (3, 4):
+        r = np.empty((b.num_vertices, 32), np.float32)
+        with pytest.raises(GasError):
+            b.run(ppr_seeds=seeds, damping=0.5, tol=1e-30, max_ppr_iterations=cap, rank_out=r)
+        assert (r == r[:, :1]).all()
+        ranks.append(r[:, 0].astype(np.float64))
+    step = np.abs(ranks[1] - ranks[0])
+    assert {2.0 ** -4, 2.0 ** -29, 2.0 ** -54} <= set(step)
+    want = math.fsum(step)
+    assert want < 0.5 and (np.remainder(step * 2.0 ** 54, 1) == 0).all()
+    assert math.fsum(step[step > 2.0 ** -54]) != want
+    r = b.run(ppr_seeds=seeds, damping=0.5, tol=want)
+    assert r.stats.ppr_iterations == 4
+    assert list(r.stats.ppr_lane_residual[:32]) == [want] * 32
     b.close()
