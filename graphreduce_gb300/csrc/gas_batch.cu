@@ -936,17 +936,18 @@ struct PprArgs {
   unsigned int *ticket;   // blocks of k_ppr_rows done (left at 0)
 };
 
-// The gather's plan.  A row's in-edges are cut into units of at most 128
-// edges; the units of a window of 2,048 are sorted by their number of steps
-// (8 edges each), and S units that follow one another in that order, S the
-// groups of a warp, form a slice: the warp walks them side by side, and since
-// they are (nearly) equally long their rows end at the same step.  The
-// sources are stored step by step, S x 8 to a step, short rows padded with
-// the index of a contribution row of zeros: a warp's reads of them are whole
-// lines and need no bounds.  (A walk of consecutive rows by 8 groups finds a
-// row end in three of four steps, in one group, and all wait for it: 630 us
-// per iteration at 64 M edges and 16 lanes, issue slots half busy with 16
-// warps per SM, against 367.)
+// The gather's plan.  A row's in-edges are cut into units of at most 128 edges;
+// the units of a window of 2,048 are sorted by their number of steps (8 edges
+// each), and S units that follow one another in that order, S the groups of a
+// warp, form a slice: the warp walks them side by side, and since they are
+// (nearly) equally long their rows end at the same step.  The sources are
+// stored step by step, S x 8 to a step, short units padded with the index of a
+// contribution row of zeros: a warp's reads of them are whole lines and need no
+// bounds.  Whole steps of padding come first, so that all units of a slice end
+// in its last step, the one summed term by term.  (A walk of consecutive rows
+// by 8 groups finds a row end in three of four steps, in one group, and all
+// wait for it: 630 us per iteration at 64 M edges and 16 lanes, issue slots
+// half busy with 16 warps per SM, against 367.)
 constexpr int kPprU = 8;          // in-edges of a step of the gather
 constexpr int kPprUnit = 128;     // in-edges of a unit
 constexpr int kPprWindow = 2048;  // units sorted together
@@ -1456,8 +1457,9 @@ __global__ void __launch_bounds__(kNT)
       int v = nV;
       if (s * S + g < U) {
         const int2 p = place[s * S + g];
-        const int e = step * kPprU + j;
-        if (e < p.y) v = csc_src[p.x + e];
+        const int lead = t1 - t0 - (p.y + kPprU - 1) / kPprU;
+        const int e = (step - lead) * kPprU + j;
+        if (e >= 0 && e < p.y) v = csc_src[p.x + e];
       }
       idx[(size_t)t0 * S * kPprU + i] = v;
     }

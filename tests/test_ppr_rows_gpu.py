@@ -105,3 +105,22 @@ def test_residual_has_the_bits_of_an_fp64_sum():
     assert r.stats.ppr_iterations == 4
     assert list(r.stats.ppr_lane_residual[:32]) == [want] * 32
     b.close()
+
+
+@pytest.mark.parametrize("lanes", [1, 2, 6, 16, 32])
+def test_a_short_row_next_to_long_ones_is_summed_term_by_term(lanes):
+    """A row with contributions c, c 2^-24 and c 2^-24, whose sum is a float but
+    whose pairwise sum loses it; the hub's units are longer and share its walk."""
+    p1, q1, p2, q2, v, sink, d = 1, 2, 3, 4, 5, 6, 1 << 12
+    pairs = ([(0, p1), (0, q1), (p1, p2), (p2, v), (q1, q2)] + [(q1, sink)] * (d - 1)
+             + [(q2, v)] * 2 + [(q2, sink)] * (d - 2))
+    src, dst = np.array(pairs, np.int32).T
+    b = Batch()
+    b.add_graph(7, src.copy(), dst.copy())
+    b.build()
+    rank = np.empty((7, lanes), np.float32)
+    with pytest.raises(GasError):
+        b.run(ppr_seeds=np.zeros((1, lanes), np.int32), damping=0.5, tol=1e-30,
+              max_ppr_iterations=3, rank_out=rank)
+    assert (rank[v] == np.float32(2.0 ** -4 + 2.0 ** -27)).all()
+    b.close()
