@@ -114,3 +114,27 @@ def test_size_limits(schedule, nV, one):
     np.testing.assert_array_equal(vd, ref)
     assert st.iterations == rit and (st.kernel_launches == 1) == one
     eng.close()
+
+
+@pytest.mark.parametrize("schedule,nV,one", [("auto", (1 << 22) - 1, True), ("auto", 1 << 22, False),
+                                             ("learned", 1 << 21, True),
+                                             ("learned", (1 << 21) + 1, False),
+                                             ("learned", 5000, True)])
+def test_sssp_size_limits(schedule, nV, one):
+    """SSSP has a limit of its own under LEARNED."""
+    from graphreduce_gb300.learn import DATA, MLP
+    rng = np.random.default_rng(6)
+    src, dst = rng.integers(0, nV, (2, 2 * nV)).astype(np.int32)
+    w = rng.integers(1, 65, 2 * nV).astype(np.int32)
+    s = int(src[0])
+    ref, rit = oracle.sssp(nV, src, dst, w, s)
+    eng = GASEngineGPU("sssp")
+    vd = initial_vertex_data("sssp", nV, s)
+    eng.setGraph(nV, vd, 2 * nV, w, src, dst)
+    eng.set_schedule_model(MLP.load(DATA / "schedule_head.npz"))
+    eng.setActive(0, nV)
+    st = eng.run_schedule(schedule)
+    eng.getResults()
+    np.testing.assert_array_equal(vd, ref)
+    assert st.iterations == rit and (st.kernel_launches == 1) == one
+    eng.close()
