@@ -412,9 +412,9 @@ __device__ __forceinline__ void ms_store_depths(int32_t *depth, int L, int G, in
 template <int WW>
 __global__ void __launch_bounds__(kNT, 5)
     k_ms_write(uint32_t *tbits, uint32_t *vn, const int32_t *csr_off,
-               int nW, const int32_t *part, const int2 *wpart, int L, int G, const gas_counters *cnt,
-               int32_t *depth, int32_t *q_mask, int32_t *q_end, int32_t *q_delta,
-               int32_t *chunk_row, uint32_t *fr, uint32_t *alive, const int32_t *g_off,
+               int nW, const int32_t *part, const int2 *wpart, int L, int G,
+               const gas_counters *cnt, int32_t *depth, int32_t *q_mask, int32_t *q_end,
+               int32_t *q_delta, int32_t *chunk_row, uint32_t *fr, uint32_t *alive, const int32_t *g_off,
                int n_graphs, int nV) {
   // rows spanning many chunks (hubs), written by the whole warp at the end
   constexpr int kBig = 64;
@@ -1816,7 +1816,8 @@ gas_status_t ensure_ppr(gas_batch *b, int lanes, int P, int n_seeds, int grid_ro
     drop_graph(b);
     b->ppr_lanes = 0;
     const size_t row = (size_t)lanes * 4;
-    CUDA_TRY(b->ppr_mem.alloc({GROUP_PART(b->rank, nV * row), GROUP_PART(b->contrib, (nV + 1) * row),
+    CUDA_TRY(b->ppr_mem.alloc({GROUP_PART(b->rank, nV * row),
+                               GROUP_PART(b->contrib, (nV + 1) * row),
                                GROUP_PART(b->sum, n_ne * row),
                                GROUP_PART(b->partial, (size_t)b->n_slots * lanes * sizeof(CVal))}));
     b->ppr_lanes = lanes;

@@ -901,9 +901,12 @@ gas_status_t launch_generic_gather(gas_engine *e, bool fuse, bool ordered,
 gas_status_t builtin_gather(gas_engine *e, bool fuse, bool ordered,
                             bool partitioned, void *stream) {
   switch (e->prog) {
-    case GAS_PROG_SSSP: return launch_generic_gather<progs::Sssp>(e, fuse, ordered, partitioned, stream);
-    case GAS_PROG_CC: return launch_generic_gather<progs::Cc>(e, fuse, ordered, partitioned, stream);
-    case GAS_PROG_PAGERANK: return launch_generic_gather<progs::PageRank>(e, fuse, ordered, partitioned, stream);
+    case GAS_PROG_SSSP:
+      return launch_generic_gather<progs::Sssp>(e, fuse, ordered, partitioned, stream);
+    case GAS_PROG_CC:
+      return launch_generic_gather<progs::Cc>(e, fuse, ordered, partitioned, stream);
+    case GAS_PROG_PAGERANK:
+      return launch_generic_gather<progs::PageRank>(e, fuse, ordered, partitioned, stream);
     default: return GAS_OK;  // BFS: gatherMap/gatherReduce are no-ops
   }
 }
@@ -959,8 +962,8 @@ gas_status_t scatter_common(gas_engine *e, void *stream, const LoopEnd &end) {
   const int nW = (e->nV + 31) / 32, nb = e->n_cblocks;
   int2 *part = static_cast<int2 *>(e->cpart), *wpart = part + nb;
   const int tile = e->prog == GAS_PROG_USER ? 0 : kBuiltinTile;  // users partition themselves
-  k_compact_count<<<nb, kNT, 0, S(stream)>>>(e->bits, e->changed, e->csc_off, nW, e->nE, part, wpart,
-                                             ctl, e->cnt);
+  k_compact_count<<<nb, kNT, 0, S(stream)>>>(e->bits, e->changed, e->csc_off, nW, e->nE, part,
+                                             wpart, ctl, e->cnt);
   if (nb > kCSumBlocks) k_compact_spine<<<1, kNT, 0, S(stream)>>>(part, nb);
   k_compact_write<<<nb, kNT, 0, S(stream)>>>(e->bits, e->csc_off, nW, part, wpart,
                                              nb > kCSumBlocks ? 1 : 0, e->act, e->scan,

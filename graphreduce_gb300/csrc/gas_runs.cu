@@ -793,8 +793,8 @@ __global__ void __launch_bounds__(kNT)
 // Deterministic sum of the per-CTA residuals; sets the loop condition.
 __global__ void __launch_bounds__(kNT)
     k_pr_finish(const double *l1_part, int n, const double *tol_p,
-                gas_counters *cnt, double *residual, int32_t *fix_n,
-                cudaGraphConditionalHandle h, int in_graph) {
+                gas_counters *cnt, double *residual, cudaGraphConditionalHandle h,
+                int in_graph) {
   __shared__ double s[kNT];
   double v = 0.0;
   for (int i = threadIdx.x; i < n; i += kNT) v += l1_part[i];
@@ -807,7 +807,6 @@ __global__ void __launch_bounds__(kNT)
   if (threadIdx.x == 0) {
     const double l1 = s[0];
     const double tol = *tol_p;
-    if (fix_n) *fix_n = 0;  // the fixup of this iteration has run
     const int max_iter = cnt->max_iter;
     *residual = l1;
     const int it = ++cnt->iteration;
@@ -868,7 +867,7 @@ gas_status_t pr_body(gas_engine *e, cudaStream_t cs,
                                          e->csc_off, e->nV, e->cnt, e->pr_l1 + c->merge_grid);
   gas::prof_end(e, cs);
   k_pr_finish<<<1, kNT, 0, cs>>>(e->pr_l1, c->merge_grid + c->fix_grid, c->residual + 1,
-                                 e->cnt, c->residual, nullptr, h, e->in_graph ? 1 : 0);
+                                 e->cnt, c->residual, h, e->in_graph ? 1 : 0);
   CUDA_TRY(cudaGetLastError());
   return GAS_OK;
 }

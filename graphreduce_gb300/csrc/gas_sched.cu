@@ -236,7 +236,6 @@ __global__ void __launch_bounds__(kNT, 8)
 }
 
 constexpr int kSpineNT = 1024;  // k_q_spine (with the loop control, below)
-constexpr int kBfsPullDiv = 16;  // BFS pull_div of the counters (unused by its AUTO rule)
 // BFS AUTO: the direction rule of Beamer, Asanovic & Patterson ("Direction-
 // Optimizing Breadth-First Search", SC'12) with the paper's constants.  A
 // top-down level is followed by a bottom-up one when the queue's out-edges
@@ -1204,9 +1203,7 @@ gas_status_t run_fast(gas_engine *e, gas_schedule_t schedule,
   if (!host_loop && !e->graphs[slot]) GAS_TRY(build_fast_graph(e, &ctx, &e->graphs[slot]));
   const int forced = schedule == GAS_SCHED_PUSH ? 1 : schedule == GAS_SCHED_PULL ? 2
                      : schedule == GAS_SCHED_LEARNED ? 3 : 0;
-  // BFS pulls while the frontier's out-edges exceed 1/16 of the edges
-  const int pull_div = e->prog == GAS_PROG_BFS ? kBfsPullDiv : e->pull_div;
-  k_fast_reset<<<1, 1, 0, S(stream)>>>(e->cnt, max_iterations, forced, pull_div);
+  k_fast_reset<<<1, 1, 0, S(stream)>>>(e->cnt, max_iterations, forced, e->pull_div);
   cudaError_t ce = cudaGetLastError();
   if (host_loop) {
     if (ce == cudaSuccess) {

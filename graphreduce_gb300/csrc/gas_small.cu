@@ -459,9 +459,9 @@ gas_status_t run_bfs_small(gas_engine *e, gas_schedule_t schedule, int32_t max_i
   int max_iter = max_iterations;
   void *args[] = {&g, &act, &n_act, &bits, &qa, &qb, &nw, &nE, &forced, &max_iter, &ctl, &cnt};
   if (count) prof_begin(e, s, kProfPush, 0);
-  CUDA_TRY(launch_small(count ? (void *)k_bfs_small<true, false> : (void *)k_bfs_small<false, false>,
-                        count ? (void *)k_bfs_small<true, true> : (void *)k_bfs_small<false, true>,
-                        kSbCluster, e, args, s));
+  void *grid_fn = count ? (void *)k_bfs_small<true, false> : (void *)k_bfs_small<false, false>;
+  void *cluster_fn = count ? (void *)k_bfs_small<true, true> : (void *)k_bfs_small<false, true>;
+  CUDA_TRY(launch_small(grid_fn, cluster_fn, kSbCluster, e, args, s));
   prof_end(e, s);
   if (count) {
     SmallCtl h;

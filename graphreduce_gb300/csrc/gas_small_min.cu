@@ -75,8 +75,9 @@ struct MinCtl {
 template <bool kWeighted, bool kLowerOnly>
 __device__ __forceinline__ void walk(const int4 *Q, int nq, int most, int w0,
                                      const int32_t *R, int32_t *W, const int32_t *csr_off,
-                                     const int32_t *csr_dst, const int32_t *csr_w, int32_t zero_cap, int (*s_row)[3],
-                                     Stage &st, const Queue &N, Count *ctr) {
+                                     const int32_t *csr_dst, const int32_t *csr_w,
+                                     int32_t zero_cap, int (*s_row)[3], Stage &st,
+                                     const Queue &N, Count *ctr) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int kRounds = 4;
   const int lane = threadIdx.x & 31;
@@ -193,8 +194,8 @@ __global__ void __launch_bounds__(kNT, 1)
       *reinterpret_cast<int4 *>(&c->q[(k + 2) % 3]) = make_int4(0, 0, 0, 0);
     const int w0 = head.y % (nthr / 32);  // light rows begin where the heavy ones end
     if (edges < kDense * nthr) {
-      walk<kWeighted, false>(Q.heavy, head.y, kHeavyMost, 0, R, W, csr_off, csr_dst, csr_w, zero_cap,
-                             s_row[warp], st, N, ctr);
+      walk<kWeighted, false>(Q.heavy, head.y, kHeavyMost, 0, R, W, csr_off, csr_dst, csr_w,
+                             zero_cap, s_row[warp], st, N, ctr);
       walk<kWeighted, false>(Q.light, head.x, 32, w0, R, W, csr_off, csr_dst, csr_w, zero_cap,
                              s_row[warp], st, N, ctr);
       flush(st, csr_off, N, ctr);
@@ -290,9 +291,11 @@ gas_status_t run_min_small(gas_engine *e, int32_t max_iterations, gas_run_stats 
   gas_counters *cnt = e->cnt;
   void *args[] = {&csr_off, &csr_dst, &csr_w, &vd, &vd2, &qa, &qb, &nV, &zero_cap,
                   &max_iterations, &ctl, &cnt};
-  CUDA_TRY(launch_small(weighted ? (void *)k_min_small<true, false> : (void *)k_min_small<false, false>,
-                        weighted ? (void *)k_min_small<true, true> : (void *)k_min_small<false, true>,
-                        kMinCluster, e, args, s));
+  void *grid_fn =
+      weighted ? (void *)k_min_small<true, false> : (void *)k_min_small<false, false>;
+  void *cluster_fn =
+      weighted ? (void *)k_min_small<true, true> : (void *)k_min_small<false, true>;
+  CUDA_TRY(launch_small(grid_fn, cluster_fn, kMinCluster, e, args, s));
   GAS_TRY(engine_sync_counts(e, stream));
   const gas_counters c = *e->h_cnt;
   e->sm_clean = c.error == 0 || c.error == GAS_ERR_ITER_CAP;
